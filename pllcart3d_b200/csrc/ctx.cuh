@@ -70,6 +70,7 @@ struct pllgpu_ctx {
     // cos / sin of 2 pi m / N and of pi k / (2N)
     bool fft_on = false;
     bool xt_on = false;         // FP64 form: TMA-staged marching explicit operator
+    int xt_cap[4] = {};         // its blocks resident at once, per variable
     double2 *fft_tw[2] = {nullptr, nullptr}, *fft_wq[2] = {nullptr, nullptr};
     UmmaPlan um;                // precision form's tensor-core DCT (when shapes allow)
     double* scal = nullptr;     // device scalars (S_*)

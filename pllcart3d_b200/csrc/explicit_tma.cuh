@@ -3,8 +3,8 @@
 // ymom / zmom, L573-590, L970-989, L1127-1146, L1280-1298) as a
 // plane-marching kernel with TMA-staged shared-memory tiles.
 //
-// A block owns a tile of XT_TJ rows (j) x XT_TK cells (k) and walks XT_NI
-// planes along x.  Every plane's tiles arrive by cp.async.bulk.tensor (one
+// A block owns a tile of XT_TJ rows (j) x XT_TK cells (k) and walks ni planes
+// along x (chosen per launch, launch_explicit_tma).  Every plane's tiles arrive by cp.async.bulk.tensor (one
 // thread issues them; an mbarrier per ring slot counts the bytes): q with a
 // +-3 halo in j and k (the WENO5 stencils along y and z), and, with a +-1
 // halo, each field the variable reads at a j or k offset (velocities,
@@ -35,7 +35,6 @@ namespace {
 constexpr int XT_TK = 32;   // k cells per tile (one warp across)
 constexpr int XT_TJ = 8;    // j rows per tile (one warp each)
 constexpr int XT_NS = 4;    // plane slots of the ring
-constexpr int XT_NI = 32;   // planes per block
 constexpr int XT_THREADS = XT_TK * XT_TJ;
 constexpr long long XT_WAIT_CYCLES = 2000000000LL;   // ~1 s of SM clock
 
@@ -152,7 +151,7 @@ __device__ __forceinline__ real xt_upwind(const real* v, const real* __restrict_
 
 template <int VAR, typename real>
 __global__ void __launch_bounds__(XT_THREADS) k_explicit_tma(const __grid_constant__ XtMaps maps, Geo G, Rng R,
-                                                             Consts K, ExplicitArgs<real> A, int* status)
+                                                             Consts K, ExplicitArgs<real> A, int ni, int* status)
 {
     using GM = XtGeom<real>;
     using SM = XtSmem<real, VAR>;
@@ -164,8 +163,8 @@ __global__ void __launch_bounds__(XT_THREADS) k_explicit_tma(const __grid_consta
     const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
     const int k0 = 1 + blockIdx.x * XT_TK;
     const int j0 = R.js + blockIdx.y * XT_TJ;
-    const int i0 = R.is + blockIdx.z * XT_NI;
-    const int i1 = min(i0 + XT_NI - 1, R.ie);
+    const int i0 = R.is + blockIdx.z * ni;
+    const int i1 = min(i0 + ni - 1, R.ie);
     const int k = k0 + tx, j = j0 + ty;
     const bool live = k >= R.ks && k <= R.ke && j <= R.je;
     const long sx = G.sx, sy = G.sy;

@@ -49,6 +49,26 @@ bool field_map(CUtensorMap* m, const real* base, const Geo& G, int box_k, int bo
               CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// planes a block of the marching explicit operator walks: the length that
+// minimises waves x (planes + 2), a wave being the `cap` blocks the GPU holds
+// at once and 2 planes' time what a block spends filling its ring and windows.
+// A fixed 32 planes left a 64x32x32 run on 8 blocks of 148 SMs' worth (73 us
+// per launch) and 256x128x128 on 1.7 waves.
+inline int xt_planes(long tiles, int planes, int cap)
+{
+    int best = 1;
+    long cost = -1;
+    for (int n = 1; n <= 64 && n <= planes; ++n) {
+        const long blocks = tiles * ((planes + n - 1) / n);
+        const long c = (blocks + cap - 1) / cap * (n + 2);
+        if (cost < 0 || c <= cost) {
+            cost = c;
+            best = n;
+        }
+    }
+    return best;
+}
+
 // the TMA-staged plane-marching explicit operator (explicit_tma.cuh); false
 // when a tensor map cannot be made (the caller then runs k_explicit)
 template <typename real, int VAR>
@@ -71,9 +91,11 @@ bool launch_explicit_tma(pllgpu_ctx* ctx, const ExplicitArgs<real>& A)
     if (!field_map<real>(&M.q, A.q, ctx->G, GM::KB3, GM::JB3)) return false;
     for (int a = 0; a < XtSet<VAR>::NA; ++a)
         if (!field_map<real>(&M.a[a], staged[a], ctx->G, GM::KB1, GM::JB1)) return false;
-    const dim3 grid((ctx->G.nz + XT_TK - 1) / XT_TK, (nj(R) + XT_TJ - 1) / XT_TJ, (ni(R) + XT_NI - 1) / XT_NI);
-    go<NoBatch>(ctx, k_explicit_tma<VAR, real>, grid, XT_THREADS, XtSmem<real, VAR>::DYN, M, ctx->G, R, ctx->K, A,
-                                                                                     ctx->status);
+    const dim3 tiles((ctx->G.nz + XT_TK - 1) / XT_TK, (nj(R) + XT_TJ - 1) / XT_TJ);
+    const int np = xt_planes((long)tiles.x * tiles.y, ni(R), ctx->xt_cap[VAR]);
+    const dim3 grid(tiles.x, tiles.y, (ni(R) + np - 1) / np);
+    go<NoBatch>(ctx, k_explicit_tma<VAR, real>, grid, XT_THREADS, XtSmem<real, VAR>::DYN, M, ctx->G, R, ctx->K, A, np,
+                ctx->status);
     return true;
 }
 
@@ -935,6 +957,19 @@ bool setup_fft(pllgpu_ctx* c)
 }
 #endif
 
+// shared-memory opt-in of the marching explicit operator and the blocks of
+// it that the device holds at once
+template <int VAR, typename real>
+void xt_setup(pllgpu_ctx* c)
+{
+    int sms = 148, per = 1;
+    cudaFuncSetAttribute(k_explicit_tma<VAR, real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         XtSmem<real, VAR>::DYN);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_explicit_tma<VAR, real>, XT_THREADS, XtSmem<real, VAR>::DYN);
+    c->xt_cap[VAR] = sms * std::max(per, 1);
+}
+
 template <typename real>
 bool alloc_state(pllgpu_ctx* c)
 {
@@ -991,14 +1026,10 @@ bool alloc_state(pllgpu_ctx* c)
                          (int)adi_z_smem_bytes<VW, real>());
     if constexpr (std::is_same<real, float>::value) {
         if (p->explicit_kernel == 2) {
-            cudaFuncSetAttribute(k_explicit_tma<VC, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<float, VC>::DYN);
-            cudaFuncSetAttribute(k_explicit_tma<VU, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<float, VU>::DYN);
-            cudaFuncSetAttribute(k_explicit_tma<VV, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<float, VV>::DYN);
-            cudaFuncSetAttribute(k_explicit_tma<VW, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<float, VW>::DYN);
+            xt_setup<VC, float>(c);
+            xt_setup<VU, float>(c);
+            xt_setup<VV, float>(c);
+            xt_setup<VW, float>(c);
         }
         const bool shape_ok = (p->ny == 128 || p->ny == 256) && (p->nz == 128 || p->nz == 256);
         if (shape_ok && !p->exact_dct && p->dct_kernel != 1 && !setup_umma(c)) return false;
@@ -1006,14 +1037,10 @@ bool alloc_state(pllgpu_ctx* c)
 #if !PLL_FP64_EXACT
         if (!p->exact_dct && fft_len_ok(p->ny) && fft_len_ok(p->nz) && !setup_fft(c)) return false;
         if (!p->exact_dct && c->nelem < (1L << 31) && encode_tiled()) {
-            cudaFuncSetAttribute(k_explicit_tma<VC, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<double, VC>::DYN);
-            cudaFuncSetAttribute(k_explicit_tma<VU, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<double, VU>::DYN);
-            cudaFuncSetAttribute(k_explicit_tma<VV, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<double, VV>::DYN);
-            cudaFuncSetAttribute(k_explicit_tma<VW, double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 XtSmem<double, VW>::DYN);
+            xt_setup<VC, double>(c);
+            xt_setup<VU, double>(c);
+            xt_setup<VV, double>(c);
+            xt_setup<VW, double>(c);
             c->xt_on = true;
         }
 #endif
