@@ -16,6 +16,7 @@
 #include "fft_dct.cuh"
 #include "forms.h"
 #include "host_common.cuh"
+#include "line_part.cuh"
 #include "umma_dct.cuh"
 
 namespace pll {
@@ -141,71 +142,83 @@ void launch_explicit(pllgpu_ctx* ctx, const real* un, const real* vn, const real
     mark(ctx, lab[VAR]);
 }
 
-// the precision form's segmented solve along x (AXIS 0) or y (AXIS 1):
-// lines of P * RS rows or one fewer, P = 16 segments of RS rows, RS in
-// {4, 8, 16, 32} ({4, 8, 16} for an FP64 instantiation: a thread holds its
-// segment's rows in registers); false: not applicable.  (32 segments of
-// 16 rows for 512-row lines measured slower in FP32: at 1024 threads a block
-// spills its 16-row registers.)
-template <int VAR, int AXIS, int P, int RS, typename real>
-void line_seg(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X, int n)
+// the partitioned solves (line_part.cuh): lines of up to 256 rows in 8 rows a
+// lane, 4 to 32 lanes by the line's length, up to 512 in 16 rows a lane; the
+// exact form and longer lines take the sequential sweeps
+constexpr int LINE_PART_MAX = 512, Z_PART_MAX = 256;
+
+template <int VAR, int AXIS, typename real, int E, int L, int TL>
+void line_part(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X)
 {
-    const dim3 grid((nk(R) + 31) / 32, AXIS == 0 ? nj(R) : ni(R)), blk(32 * P);
-    constexpr size_t smem = line_seg_smem<VAR, AXIS, P, RS, real>();
-    if (n == P * RS)
-        go<k_line_seg_b<VAR, AXIS, P, RS, true, real>>(ctx, k_line_seg<VAR, AXIS, P, RS, true, real>, grid, blk, smem,
-                                                       ctx->G, R, ctx->K, X);
-    else
-        go<k_line_seg_b<VAR, AXIS, P, RS, false, real>>(ctx, k_line_seg<VAR, AXIS, P, RS, false, real>, grid, blk, smem,
-                                                        ctx->G, R, ctx->K, X);
+    using LP = LinePart<VAR, AXIS, real, E, L, TL>;
+    if (LP::SMEM > 48 * 1024)
+        cudaFuncSetAttribute(k_line_seg<VAR, AXIS, real, E, L, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)LP::SMEM);
+    const dim3 grid(R.ke / TL + 1, AXIS == 0 ? nj(R) : ni(R));   // tiles from k = 0: aligned row pieces
+    go<k_line_seg_b<VAR, AXIS, real, E, L, TL>>(ctx, k_line_seg<VAR, AXIS, real, E, L, TL>, grid, LP::T, LP::SMEM,
+                                                ctx->G, R, ctx->K, X);
 }
 
 template <int VAR, int AXIS, typename real>
-bool launch_line_seg(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X)
+bool launch_line_part(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X)
 {
-    if (ctx->P.exact_dct || ctx->nelem >= (1L << 31)) return false;
     const int n = AXIS == 0 ? ni(R) : nj(R);
-    constexpr int p = 16;
-    const int rs = (n + p - 1) / p;   // rows per segment
-    constexpr bool f32 = std::is_same<real, float>::value;
-    if (rs != 4 && rs != 8 && rs != 16 && !(f32 && rs == 32)) return false;
-    if (n != p * rs) {
-        // one row short: the kernel loads the row past the line (and the
-        // viscosity family one beyond it), which must lie in the padded box
-        const int start = AXIS == 0 ? R.is : R.js, top = AXIS == 0 ? ctx->G.NX - 1 : ctx->G.NY - 1;
-        if (n != p * rs - 1 || start + p * rs + LineCoef<VAR, AXIS>::off > top) return false;
-    }
-    if (rs == 4) line_seg<VAR, AXIS, p, 4, real>(ctx, R, X, n);
-    else if (rs == 8) line_seg<VAR, AXIS, p, 8, real>(ctx, R, X, n);
-    else if (rs == 16) line_seg<VAR, AXIS, p, 16, real>(ctx, R, X, n);
-    else if constexpr (f32) line_seg<VAR, AXIS, p, 32, real>(ctx, R, X, n);
+    if (ctx->P.exact_dct || n > LINE_PART_MAX) return false;
+    constexpr int TL = sizeof(real) == 8 ? 8 : 16;   // 64-byte row pieces
+    if (n <= 32) line_part<VAR, AXIS, real, 8, 4, TL>(ctx, R, X);
+    else if (n <= 64) line_part<VAR, AXIS, real, 8, 8, TL>(ctx, R, X);
+    else if (n <= 128) line_part<VAR, AXIS, real, 8, 16, TL>(ctx, R, X);
+    else if (n <= 256) line_part<VAR, AXIS, real, 8, 32, TL>(ctx, R, X);
+    else line_part<VAR, AXIS, real, 16, 32, 8>(ctx, R, X);
     return true;
 }
 
-// shared-memory opt-in of the segmented solves (static separator arrays and
-// dynamic row tiles together pass the 48 KB default: FP32 from 16 rows per
-// segment, FP64 from 4)
-template <int VAR, int AXIS, int P, int RS, typename real>
-void line_seg_attr()
+template <int VAR, typename real, int L>
+void z_part(pllgpu_ctx* ctx, const Rng& R, const MuPtrs<real>& mu, double alpha)
 {
-    const int b = (int)line_seg_smem<VAR, AXIS, P, RS, real>();
-    cudaFuncSetAttribute(k_line_seg<VAR, AXIS, P, RS, true, real>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
-    cudaFuncSetAttribute(k_line_seg<VAR, AXIS, P, RS, false, real>, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
+    constexpr int LINES = 4 * (32 / L);   // per block
+    go<k_adi_z_part_b<VAR, real, 8, L>>(ctx, k_adi_z_part<VAR, real, 8, L>, dim3((nj(R) + LINES - 1) / LINES, ni(R)),
+                                        128, 0, ctx->G, R, ctx->K, mu, bufs<real>(ctx).S, ctx->scal, alpha);
 }
 
 template <int VAR, typename real>
-void line_seg_attrs()
+bool launch_z_part(pllgpu_ctx* ctx, const Rng& R, const MuPtrs<real>& mu, double alpha)
 {
-    line_seg_attr<VAR, 0, 16, 4, real>();
-    line_seg_attr<VAR, 1, 16, 4, real>();
-    line_seg_attr<VAR, 0, 16, 8, real>();
-    line_seg_attr<VAR, 0, 16, 16, real>();
-    line_seg_attr<VAR, 1, 16, 8, real>();
-    line_seg_attr<VAR, 1, 16, 16, real>();
-    if constexpr (std::is_same<real, float>::value) {
-        line_seg_attr<VAR, 0, 16, 32, real>();
-        line_seg_attr<VAR, 1, 16, 32, real>();
-    }
+    const int n = nk(R);
+    if (ctx->P.exact_dct || n > Z_PART_MAX) return false;
+    if (n <= 32) z_part<VAR, real, 4>(ctx, R, mu, alpha);
+    else if (n <= 64) z_part<VAR, real, 8>(ctx, R, mu, alpha);
+    else if (n <= 128) z_part<VAR, real, 16>(ctx, R, mu, alpha);
+    else z_part<VAR, real, 32>(ctx, R, mu, alpha);
+    return true;
+}
+
+template <typename T, int E, int L, int TL>
+void poisson_part(pllgpu_ctx* ctx, T* hat, int kz_major)
+{
+    using PP = PoissonPart<T, E, L, TL>;
+    const int N = ctx->G.ny * ctx->G.nz;
+    if (PP::SMEM > 48 * 1024)
+        cudaFuncSetAttribute(k_poisson_part<T, E, L, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PP::SMEM);
+    go<k_poisson_part_b<T, E, L, TL>>(ctx, k_poisson_part<T, E, L, TL>, (N + TL - 1) / TL, PP::TH, PP::SMEM, ctx->G.nx,
+                                      ctx->G.ny, ctx->G.nz, ctx->K, ctx->lam_y, ctx->lam_z, hat, kz_major);
+}
+
+// the x-tridiagonal of every Poisson mode, in place
+template <typename T>
+void launch_modes(pllgpu_ctx* ctx, T* hat, int kz_major)
+{
+    const int nx = ctx->G.nx, N = ctx->G.ny * ctx->G.nz;
+    constexpr int TL = 8;
+    if (ctx->P.exact_dct || nx > LINE_PART_MAX)
+        go<k_poisson_x_b<T>>(ctx, k_poisson_x<T>, (N + 127) / 128, 128, 0, nx, ctx->G.ny, ctx->G.nz, ctx->K, ctx->lam_y,
+                             ctx->lam_z, hat, ctx->mode_cc, ctx->mode_rr, kz_major);
+    else if (nx <= 32) poisson_part<T, 8, 4, TL>(ctx, hat, kz_major);
+    else if (nx <= 64) poisson_part<T, 8, 8, TL>(ctx, hat, kz_major);
+    else if (nx <= 128) poisson_part<T, 8, 16, TL>(ctx, hat, kz_major);
+    else if (nx <= 256) poisson_part<T, 8, 32, TL>(ctx, hat, kz_major);
+    else poisson_part<T, 16, 32, TL>(ctx, hat, kz_major);
+    mark(ctx, "poisson_x");
 }
 
 template <typename real, int VAR>
@@ -230,46 +243,25 @@ void launch_implicit(pllgpu_ctx* ctx, double g, double r)
     X.r = r;
     X.alpha = alpha;
     const int lb = tune_line_block(ctx->tune_line);
-    bool ydone = false;
-    if constexpr (!std::is_same<real, float>::value && !PLL_FP64_EXACT && VAR == VC) {
-        // FP64 forms: the segmented y solve for concentration (0.65 against
-        // 0.95 ms per step at 512x256x256).  For momentum, whose segments
-        // also stage viscosity rows, one 512-thread block per SM measured
-        // slower than the prefetching sweep (1.12 against 1.00 ms).
-        ydone = launch_line_seg<VAR, 1, real>(ctx, R, X);
-    }
-    if constexpr (std::is_same<real, float>::value) {
-        // the precision form's partitioned solves: segmented when the line
-        // length allows, else for concentration the warp solve of short
-        // lines
-        ydone = launch_line_seg<VAR, 1, real>(ctx, R, X);
-        if (!ydone && VAR == VC && nj(R) <= ZP_MAX && nj(R) >= 2 * (ZP_MAX / 32) && !ctx->P.exact_dct) {
-            go<k_adi_y_part_b<VAR, float>>(ctx, k_adi_y_part<VAR, float>, dim3((nk(R) + 31) / 32, ni(R)), 256,
-                                           adi_y_part_smem<float>(), ctx->G, R, ctx->K, X.mu, B.S, ctx->scal, alpha);
-            ydone = true;
-        }
-    }
+#if PLL_FP64_EXACT
+    constexpr bool part = sizeof(real) == 4;   // the exact form keeps the reference's sweeps
+#else
+    constexpr bool part = true;
+#endif
+    bool ydone = false, zdone = false, xdone = false;
+    if constexpr (part) ydone = launch_line_part<VAR, 1, real>(ctx, R, X);
     if (!ydone)
         go<k_line_pf_b<VAR, 1, real>>(ctx, k_line_pf<VAR, 1, real>, dim3((nk(R) + lb - 1) / lb, ni(R)), lb, 0, ctx->G,
                                       R, ctx->K, X);
     mark(ctx, ly[VAR]);
-    bool zdone = false;
-    if constexpr (std::is_same<real, float>::value || !PLL_FP64_EXACT) {
-        if (nk(R) <= ZP_MAX && nk(R) >= 2 * (ZP_MAX / 32) && !ctx->P.exact_dct) {
-            // the partitioned warp solve (precision form and FP64 form)
-            go<k_adi_z_part_b<VAR, real>>(ctx, k_adi_z_part<VAR, real>, dim3((nj(R) + 3) / 4, ni(R)), 128, 0, ctx->G, R,
-                                          ctx->K, X.mu, B.S, ctx->scal, alpha);
-            zdone = true;
-        }
-    }
+    if constexpr (part) zdone = launch_z_part<VAR, real>(ctx, R, X.mu, alpha);
     if (!zdone) {
         constexpr size_t smem = adi_z_smem_bytes<VAR, real>();
         go<k_adi_z_tiled_b<VAR, real>>(ctx, k_adi_z_tiled<VAR, real>, dim3((nj(R) + 127) / 128, ni(R)), 128, smem,
                                        ctx->G, R, ctx->K, X.mu, B.S, B.cc, ctx->scal, alpha);
     }
     mark(ctx, lz[VAR]);
-    bool xdone = false;
-    if constexpr (std::is_same<real, float>::value) xdone = launch_line_seg<VAR, 0, real>(ctx, R, X);
+    if constexpr (part) xdone = launch_line_part<VAR, 0, real>(ctx, R, X);
     if (!xdone)
         go<k_line_pf_b<VAR, 0, real>>(ctx, k_line_pf<VAR, 0, real>, dim3((nk(R) + lb - 1) / lb, nj(R)), lb, 0, ctx->G,
                                       R, ctx->K, X);
@@ -357,9 +349,7 @@ void launch_poisson_umma(pllgpu_ctx* ctx)
     launch_umma(ctx, 0, (long)nx * ny, nz, UmmaEpi{ny, N, 1, ny, 1.f, 0, 1}, B.dct2);
     // forward y: dct1[x][kz][ky] = sum_y dct2[x][kz][y] Ty[ky][y]
     launch_umma(ctx, 1, (long)nx * nz, ny, UmmaEpi{nz, N, ny, 1, 1.f, 0, 0}, B.dct1);
-    go<k_poisson_x2_b>(ctx, k_poisson_x2, (int)((N + 127) / 128), 128, 0, nx, ny, nz, ctx->K, ctx->lam_y, ctx->lam_z,
-                       B.dct1, (float*)ctx->mode_rr, ctx->mode_cc, 1);
-    mark(ctx, "poisson_x");
+    launch_modes<float>(ctx, B.dct1, 1);
     // inverse y: dct2[x][y][kz] = sum_ky dct1[x][kz][ky] Tiy[y][ky] (stored transposed)
     launch_umma(ctx, 2, (long)nx * nz, ny, UmmaEpi{nz, N, 1, nz, 1.f, 0, 1}, B.dct2);
     // inverse z into phi's interior, divided by 4*ny*nz
@@ -406,9 +396,7 @@ void launch_poisson_fft(pllgpu_ctx* ctx)
     const FftLines zlines{nx * ny, ny, N, nz, 1, N, nz, 1, 1.0};
     fft_pass<0, false>(ctx, ny, ylines, 0, B.dct1, B.dct2);
     fft_pass<0, true>(ctx, nz, zlines, 1, B.dct2, B.dct1);
-    go<k_poisson_x_b<double>>(ctx, k_poisson_x<double>, (int)((N + 127) / 128), 128, 0, nx, ny, nz, ctx->K,
-                              ctx->lam_y, ctx->lam_z, B.dct1, ctx->mode_cc, ctx->mode_rr, 0);
-    mark(ctx, "poisson_x");
+    launch_modes<double>(ctx, B.dct1, 0);
     fft_pass<1, false>(ctx, ny, ylines, 0, B.dct1, B.dct2);
     // into phi's interior, times 1/(4 ny nz) (exact: a power of two)
     FftLines out = zlines;
@@ -448,9 +436,7 @@ void launch_poisson(pllgpu_ctx* ctx)
     d = GemmDesc{ny, nz, nz, nx, N, nz, 1, 0, 1, nz, N, nz, 1, 0.0, 0};
     launch_gemm(ctx, d, B.dct2, B.Tz, B.dct1);
     // x-tridiagonal per mode, in place in dct1, FP64 arithmetic
-    go<k_poisson_x_b<real>>(ctx, k_poisson_x<real>, (int)((N + 127) / 128), 128, 0, nx, ny, nz, ctx->K,
-                            ctx->lam_y, ctx->lam_z, B.dct1, ctx->mode_cc, ctx->mode_rr, 0);
-    mark(ctx, "poisson_x");
+    launch_modes<real>(ctx, B.dct1, 0);
     // inverse, y pass: dct2[x][y][kz] = sum_ky Tiy[y][ky] dct1[x][ky][kz]
     d = GemmDesc{ny, nz, ny, nx, 0, ny, 1, N, nz, 1, N, nz, 1, 0.0, 0};
     launch_gemm(ctx, d, B.Tiy, B.dct1, B.dct2);
@@ -999,23 +985,6 @@ bool alloc_state(pllgpu_ctx* c)
     dct_matrix<real>(1, p->nz, T.data());
     cudaMemcpy(B.Tiz, T.data(), sizeof(real) * p->nz * p->nz, cudaMemcpyHostToDevice);
     // kernels above the 48 KB default of dynamic shared memory
-    if constexpr (std::is_same<real, float>::value) {
-        cudaFuncSetAttribute(k_adi_y_part<VC, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)adi_y_part_smem<float>());
-        cudaFuncSetAttribute(k_adi_y_part<VU, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)adi_y_part_smem<float>());
-        cudaFuncSetAttribute(k_adi_y_part<VV, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)adi_y_part_smem<float>());
-        cudaFuncSetAttribute(k_adi_y_part<VW, float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)adi_y_part_smem<float>());
-    }
-    if constexpr (!std::is_same<real, float>::value && !PLL_FP64_EXACT) line_seg_attrs<VC, real>();
-    if constexpr (std::is_same<real, float>::value) {
-        line_seg_attrs<VC, real>();
-        line_seg_attrs<VU, real>();
-        line_seg_attrs<VV, real>();
-        line_seg_attrs<VW, real>();
-    }
     cudaFuncSetAttribute(k_adi_z_tiled<VC, real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)adi_z_smem_bytes<VC, real>());
     cudaFuncSetAttribute(k_adi_z_tiled<VU, real>, cudaFuncAttributeMaxDynamicSharedMemorySize,

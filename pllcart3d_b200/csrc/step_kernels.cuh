@@ -1003,206 +1003,6 @@ struct k_adi_z_tiled_b {
 
 
 // ---------------------------------------------------------------------------
-// The precision form's z line solve: one warp per line, the line held in
-// registers (8 rows per lane) and solved by a partition method instead of
-// the sequential Thomas chain.  Row 8l of each lane is a separator; the lane
-// eliminates its 7 interior rows in terms of its own separator and the next
-// lane's (x_e = g_e - v_e S_l - w_e S_{l+1}), the 32 separator equations
-// form a tridiagonal system solved by parallel cyclic reduction over warp
-// shuffles, and the interior rows follow.  S is read once and the solution
-// written once (the Thomas form also writes and re-reads c' and the
-// eliminated right-hand side).  Same coefficients and closures as
-// k_adi_z_tiled; FP32-level agreement, not bitwise.  Lines of up to 256.
-// Rows move between global memory (coalesced, row m by lane m % 32) and the
-// lane that owns them (8l .. 8l+7) through a skewed shared buffer.
-// ---------------------------------------------------------------------------
-constexpr int ZP_MAX = 256;
-__device__ __forceinline__ int zp_skew(int m) { return m + (m >> 3); }
-
-// 1/x of the partitioned solves: FP32 approximate (<= 2 ulp; the pivots of
-// these diagonally dominant systems are >= 1 in magnitude), FP64 IEEE
-template <typename real>
-__device__ __forceinline__ real rcp_(real x) { return (real)1 / x; }
-template <>
-__device__ __forceinline__ float rcp_<float>(float x) { return __fdividef(1.0f, x); }
-
-// Partitioned solve of one line of 32 E rows held E per lane (rows
-// E l .. E l + E - 1 on lane l; a of the first row and c of the last are 0;
-// rows past the line are identity rows): row E l of each lane is a
-// separator, the lane eliminates its E-1 interior rows in terms of its own
-// separator and the next lane's (x_e = g_e - v_e S_l - w_e S_{l+1}), the 32
-// separator equations are solved by parallel cyclic reduction over warp
-// shuffles, then the interior rows.  FP32, diagonally dominant systems.
-template <typename real, int E>
-__device__ __forceinline__ void zp_solve(const real* A, const real* B, const real* C, const real* Rr, real* x,
-                                         int lane)
-{
-    // interior rows e = 1..E-1: forward in terms of the own separator S_l
-    real ch[E], rh[E], ah[E];
-    {
-        const real ib = rcp_<real>(B[1]);
-        ch[1] = C[1] * ib;
-        rh[1] = Rr[1] * ib;
-        ah[1] = A[1] * ib;
-    }
-#pragma unroll
-    for (int e = 2; e < E; ++e) {
-        const real id = rcp_<real>(B[e] - A[e] * ch[e - 1]);
-        ch[e] = C[e] * id;
-        rh[e] = (Rr[e] - A[e] * rh[e - 1]) * id;
-        ah[e] = -A[e] * ah[e - 1] * id;
-    }
-    // backward: x_e = g_e - v_e S_l - w_e S_{l+1}
-    real g[E], v[E], w[E];
-    g[E - 1] = rh[E - 1];
-    v[E - 1] = ah[E - 1];
-    w[E - 1] = ch[E - 1];
-#pragma unroll
-    for (int e = E - 2; e >= 1; --e) {
-        g[e] = rh[e] - ch[e] * g[e + 1];
-        v[e] = ah[e] - ch[e] * v[e + 1];
-        w[e] = -ch[e] * w[e + 1];
-    }
-    // separator row 8l: A0 x_{8l-1} + B0 S_l + C0 x_{8l+1} = R0
-    real gp = __shfl_up_sync(0xffffffffu, g[E - 1], 1);
-    real vp = __shfl_up_sync(0xffffffffu, v[E - 1], 1);
-    real wp = __shfl_up_sync(0xffffffffu, w[E - 1], 1);
-    if (lane == 0) gp = vp = wp = (real)0;
-    real al = -A[0] * vp;
-    real be = B[0] - A[0] * wp - C[0] * v[1];
-    real ga = -C[0] * w[1];
-    real rho = Rr[0] - A[0] * gp - C[0] * g[1];
-    // parallel cyclic reduction of the 32 separator equations
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        real al_m = __shfl_up_sync(0xffffffffu, al, d), be_m = __shfl_up_sync(0xffffffffu, be, d);
-        real ga_m = __shfl_up_sync(0xffffffffu, ga, d), rho_m = __shfl_up_sync(0xffffffffu, rho, d);
-        real al_p = __shfl_down_sync(0xffffffffu, al, d), be_p = __shfl_down_sync(0xffffffffu, be, d);
-        real ga_p = __shfl_down_sync(0xffffffffu, ga, d), rho_p = __shfl_down_sync(0xffffffffu, rho, d);
-        if (lane < d) {
-            al_m = (real)0;
-            be_m = (real)1;
-            ga_m = (real)0;
-            rho_m = (real)0;
-        }
-        if (lane + d > 31) {
-            al_p = (real)0;
-            be_p = (real)1;
-            ga_p = (real)0;
-            rho_p = (real)0;
-        }
-        const real k1 = al * rcp_<real>(be_m), k2 = ga * rcp_<real>(be_p);
-        const real nal = -k1 * al_m, nga = -k2 * ga_p;
-        be = be - k1 * ga_m - k2 * al_p;
-        rho = rho - k1 * rho_m - k2 * rho_p;
-        al = nal;
-        ga = nga;
-    }
-    const real Sl = rho * rcp_<real>(be);
-    real Sn = __shfl_down_sync(0xffffffffu, Sl, 1);
-    if (lane == 31) Sn = (real)0;
-    x[0] = Sl;
-#pragma unroll
-    for (int e = 1; e < E; ++e) x[e] = g[e] - v[e] * Sl - w[e] * Sn;
-}
-
-template <int VAR, typename real>
-__device__ __forceinline__ void k_adi_z_part_run(const uint3 blockIdx, const dim3 gridDim,
-    Geo G, Rng R, Consts K, MuPtrs<real> mu,
-                                                    real* __restrict__ S, const double* __restrict__ scal,
-                                                    double alpha)
-{
-    constexpr int E = ZP_MAX / 32;   // rows per lane
-    constexpr int BUF = ZP_MAX + ZP_MAX / 8 + 8;
-    __shared__ real bS[4][BUF];
-    __shared__ real bM[4][BUF];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int j = R.js + blockIdx.x * 4 + warp;
-    const int i = R.is + blockIdx.y;
-    if (j > R.je) return;   // warp-uniform
-    const int n = R.ke - R.ks + 1;
-    const real fac = (real)(0.5 * scal[S_DT] * alpha);
-    constexpr int LO = Closure<VAR, 2>::lo, HI = Closure<VAR, 2>::hi;
-    const real* __restrict__ mz = VAR == VU ? mu.xz : VAR == VV ? mu.yz : mu.cell;
-    const int moff = VAR == VW ? -1 : 0;
-    const real dzc = (real)(VAR == VW ? K.d2z : K.d1z);
-    const real ihz = (real)K.ihz, cdz = (real)K.cdz;
-    const long base = (long)i * G.sx + (long)j * G.sy + R.ks;
-    real* sS = bS[warp];
-    real* sM = bM[warp];
-#pragma unroll
-    for (int t = 0; t < E; ++t) {
-        const int m = t * 32 + lane;
-        if (m < n) sS[zp_skew(m)] = S[base + m];
-        if (VAR != VC && m <= n) sM[zp_skew(m)] = mz[base + moff + m];
-    }
-    if (VAR != VC && lane == 0 && n == ZP_MAX) sM[zp_skew(ZP_MAX)] = mz[base + moff + ZP_MAX];
-    __syncwarp();
-
-    // this lane's rows m = 8 lane + e: a x_{m-1} + b x_m + c x_{m+1} = r
-    real A[E], B[E], C[E], Rr[E];
-#pragma unroll
-    for (int e = 0; e < E; ++e) {
-        const int m = E * lane + e;
-        if (m < n) {
-            real a, c;
-            if (VAR == VC) {
-                a = cdz;
-                c = cdz;
-            } else {
-                a = dzc * sM[zp_skew(m)] * ihz;
-                c = dzc * sM[zp_skew(m + 1)] * ihz;
-            }
-            const real b = -(a + c);
-            real la = -fac * a, lb = (real)1.0 - fac * b, lc = -fac * c, lr = sS[zp_skew(m)];
-            if (m == 0) {
-                if (LO == 1) lb += la;
-                else if (LO == 2) lb -= la;
-                la = (real)0;
-            }
-            if (m == n - 1) {
-                if (HI == 1) lb += lc;
-                else if (HI == 2) lb -= lc;
-                lc = (real)0;
-            }
-            A[e] = la;
-            B[e] = lb;
-            C[e] = lc;
-            Rr[e] = lr;
-        } else {   // identity rows past the line
-            A[e] = (real)0;
-            B[e] = (real)1;
-            C[e] = (real)0;
-            Rr[e] = (real)0;
-        }
-    }
-    real x[E];
-    zp_solve<real, E>(A, B, C, Rr, x, lane);
-    __syncwarp();
-#pragma unroll
-    for (int e = 0; e < E; ++e) sS[zp_skew(E * lane + e)] = x[e];
-    __syncwarp();
-#pragma unroll
-    for (int t = 0; t < E; ++t) {
-        const int m = t * 32 + lane;
-        if (m < n) S[base + m] = sS[zp_skew(m)];
-    }
-}
-template <int VAR, typename real>
-__global__ void __launch_bounds__(128) k_adi_z_part(Geo G, Rng R, Consts K, MuPtrs<real> mu,
-                                                    real* __restrict__ S, const double* __restrict__ scal,
-                                                    double alpha)
-{
-    k_adi_z_part_run<VAR, real>(blockIdx, gridDim, G, R, K, mu, S, scal, alpha);
-}
-template <int VAR, typename real>
-struct k_adi_z_part_b {
-    static constexpr auto run = &k_adi_z_part_run<VAR, real>;
-    static constexpr int maxt = 128, minb = 0;
-};
-
-
-// ---------------------------------------------------------------------------
 // Viscosity family and offset that the implicit coefficients of VAR along
 // AXIS read (A_umom/A_vmom/A_wmom, pllcart3d.c:1443-1536): a at line
 // position m uses family[m + OFF], c uses family[m + OFF + 1]; the scale is
@@ -1242,119 +1042,6 @@ __device__ __forceinline__ void line_ac(const Consts& K, real m0, real m1, real&
         c = over_h<real>((real)d * m1, h, ih, K.pow2);
     }
 }
-
-// ---------------------------------------------------------------------------
-// The precision form's y line solve with the same partitioned warp solver:
-// a block of 8 warps stages 32 neighbouring lines (consecutive k, coalesced
-// rows of the tile) and their viscosity family through shared memory, each
-// warp solves 4 of them, the block writes the solutions back in place.  Same
-// coefficients and closures as k_line_pf<VAR, 1>; S read once, written once.
-// ---------------------------------------------------------------------------
-constexpr int YP_PITCH = ZP_MAX + ZP_MAX / 8 + 1;   // odd: conflict-free columns
-
-template <typename real>
-constexpr size_t adi_y_part_smem() { return sizeof(real) * 2 * 32 * YP_PITCH; }
-
-template <int VAR, typename real>
-__device__ __forceinline__ void k_adi_y_part_run(const uint3 blockIdx, const dim3 gridDim,
-    Geo G, Rng R, Consts K, MuPtrs<real> mu,
-                                                    real* __restrict__ S, const double* __restrict__ scal,
-                                                    double alpha)
-{
-    constexpr int E = ZP_MAX / 32;
-    extern __shared__ __align__(16) unsigned char ysm_raw[];
-    real* ysm = (real*)ysm_raw;
-    real* tS = ysm;                      // [32 lines][YP_PITCH]
-    real* tM = ysm + 32 * YP_PITCH;
-    const int i = R.is + blockIdx.y;
-    const int k0 = R.ks + blockIdx.x * 32;
-    const int nl = (R.ke - k0 + 1) < 32 ? (R.ke - k0 + 1) : 32;
-    const int n = R.je - R.js + 1;
-    const long sy = G.sy;
-    const long base0 = (long)i * G.sx + (long)R.js * sy + k0;
-    constexpr int OFF = LineCoef<VAR, 1>::off;
-    const real* __restrict__ fam = VAR == VC ? nullptr : line_family<VAR, 1, real>(mu);
-    const real dy = (real)(LineCoef<VAR, 1>::twice ? K.d2y : K.d1y);
-    const real ihy = (real)K.ihy, cdy = (real)K.cdy;
-    const real fac = (real)(0.5 * scal[S_DT] * alpha);
-    constexpr int LO = Closure<VAR, 1>::lo, HI = Closure<VAR, 1>::hi;
-    // tile loads: thread (kl, row group m0) moves rows m0, m0 + 8, ...;
-    // unrolled so that many rows' loads are in flight at once
-    const int tkl = threadIdx.x & 31, tm0 = threadIdx.x >> 5;
-#pragma unroll 11
-    for (int t = 0; t < ZP_MAX / 8 + 1; ++t) {
-        const int m = tm0 + 8 * t;
-        if (tkl < nl && m <= n) {
-            if (m < n) tS[tkl * YP_PITCH + zp_skew(m)] = S[base0 + (long)m * sy + tkl];
-            if (VAR != VC) tM[tkl * YP_PITCH + zp_skew(m)] = fam[base0 + (long)(m + OFF) * sy + tkl];
-        }
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int kl = warp; kl < nl; kl += 8) {
-        const real* ls = tS + kl * YP_PITCH;
-        const real* lm = tM + kl * YP_PITCH;
-        real A[E], B[E], C[E], Rr[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) {
-            const int m = E * lane + e;
-            if (m < n) {
-                real a, c;
-                if (VAR == VC) {
-                    a = cdy;
-                    c = cdy;
-                } else {
-                    a = dy * lm[zp_skew(m)] * ihy;
-                    c = dy * lm[zp_skew(m + 1)] * ihy;
-                }
-                const real b = -(a + c);
-                real la = -fac * a, lb = (real)1.0 - fac * b, lc = -fac * c;
-                if (m == 0) {
-                    if (LO == 1) lb += la;
-                    else if (LO == 2) lb -= la;
-                    la = (real)0;
-                }
-                if (m == n - 1) {
-                    if (HI == 1) lb += lc;
-                    else if (HI == 2) lb -= lc;
-                    lc = (real)0;
-                }
-                A[e] = la;
-                B[e] = lb;
-                C[e] = lc;
-                Rr[e] = ls[zp_skew(m)];
-            } else {
-                A[e] = (real)0;
-                B[e] = (real)1;
-                C[e] = (real)0;
-                Rr[e] = (real)0;
-            }
-        }
-        real x[E];
-        zp_solve<real, E>(A, B, C, Rr, x, lane);
-        __syncwarp();
-#pragma unroll
-        for (int e = 0; e < E; ++e) tS[kl * YP_PITCH + zp_skew(E * lane + e)] = x[e];
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int t = 0; t < ZP_MAX / 8; ++t) {
-        const int m = tm0 + 8 * t;
-        if (tkl < nl && m < n) S[base0 + (long)m * sy + tkl] = tS[tkl * YP_PITCH + zp_skew(m)];
-    }
-}
-template <int VAR, typename real>
-__global__ void __launch_bounds__(256) k_adi_y_part(Geo G, Rng R, Consts K, MuPtrs<real> mu,
-                                                    real* __restrict__ S, const double* __restrict__ scal,
-                                                    double alpha)
-{
-    k_adi_y_part_run<VAR, real>(blockIdx, gridDim, G, R, K, mu, S, scal, alpha);
-}
-template <int VAR, typename real>
-struct k_adi_y_part_b {
-    static constexpr auto run = &k_adi_y_part_run<VAR, real>;
-    static constexpr int maxt = 256, minb = 0;
-};
 
 // ---------------------------------------------------------------------------
 // Line solves along a strided axis (AXIS 0: x, lines (j,k); AXIS 1: y,
@@ -1548,324 +1235,6 @@ template <int VAR, int AXIS, typename real>
 struct k_line_pf_b {
     static constexpr auto run = &k_line_pf_run<VAR, AXIS, real>;
     static constexpr int maxt = 128, minb = 0;
-};
-
-// ---------------------------------------------------------------------------
-// The precision form's line solve along a strided axis (x or y) by a
-// partition method: a block owns 32 neighbouring lines (lane = line, adjacent
-// k, so every row access is one coalesced 128-byte transaction) and cuts each
-// line into P segments of RS rows, one warp per segment.  A thread keeps
-// its segment's right-hand side in registers; its viscosity rows (momentum)
-// and, for the x sweep, its q_old rows are copied into shared memory by
-// cp.async, each thread copying and later reading only its own rows.  The
-// thread eliminates the interior rows in terms of the segment's first row
-// (its separator) and the next segment's, the P separator equations of
-// every line are solved by one thread per line through shared memory, and
-// each thread finishes its rows with the separators known.  Every input is
-// read once from HBM and every output written once (the sequential sweep
-// also writes and re-reads c' and the eliminated rhs).  Same coefficients
-// and closures as k_line_pf (x: convective outflow, q_new = q_old + delta,
-// concentration's Neumann ghosts; y: in place into S); FP32-level agreement
-// with the sequential sweep, not bitwise.
-// ---------------------------------------------------------------------------
-
-// dynamic shared memory of k_line_seg: the viscosity family's rows (RS + 1
-// per thread, momentum) then the x sweep's q_old rows (RS per thread)
-template <int VAR, int AXIS, int P, int RS, typename real = float>
-constexpr size_t line_seg_smem()
-{
-    return sizeof(real) * 32 * P * ((VAR != VC ? RS + 1 : 0) + (AXIS == 0 ? RS : 0));
-}
-
-// one element global -> shared by cp.async (4 or 8 bytes)
-template <typename real>
-__device__ __forceinline__ void ls_cp_async(real* dst, const real* src)
-{
-    if (sizeof(real) == 8)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                     "l"(src)
-                     : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
-                     "l"(src)
-                     : "memory");
-}
-
-// an optimisation barrier on x: later reads cannot reuse values computed
-// from it before (keeps each sweep recomputing its row coefficients instead
-// of holding four per row in registers; a "memory" clobber does the same
-// for the shared-memory rows)
-__device__ __forceinline__ void ls_fresh(float& x) { asm volatile("" : "+f"(x)); }
-__device__ __forceinline__ void ls_fresh(double& x) { asm volatile("" : "+d"(x)); }
-
-// FULL: the line has P * RS rows; else P * RS - 1 and the last
-// segment's last row is an identity row (its loads read the row past the
-// line, which the host checks lies inside the padded box)
-template <int VAR, int AXIS, int P, int RS, bool FULL, typename real = float>
-__device__ __forceinline__ void k_line_seg_run(const uint3 blockIdx, const dim3 gridDim,
-    Geo G, Rng R, Consts K, XsweepArgs<real> A)
-{
-    __shared__ real eq[4][P][32];       // separator equations
-    __shared__ real tail[3][P][32];     // last interior row of each segment
-    __shared__ real sep[P + 1][32];     // separator values
-    extern __shared__ __align__(16) unsigned char ls_raw[];
-    real* ls_dyn = (real*)ls_raw;       // [row][thread] tiles: viscosity, then q_old (x)
-    constexpr int LO = Closure<VAR, AXIS>::lo, HI = Closure<VAR, AXIS>::hi;
-    constexpr int OFF = LineCoef<VAR, AXIS>::off;
-    constexpr int TS = 32 * P;
-    const int lane = threadIdx.x & 31, l = threadIdx.x >> 5;
-    const int k = R.ks + blockIdx.x * 32 + lane;
-    const int o = blockIdx.y;   // j (AXIS 0) or i (AXIS 1) offset
-    const bool live = k <= R.ke;
-    const bool last_seg = l == P - 1;
-    constexpr int n = FULL ? P * RS : P * RS - 1;
-    // offsets fit in 32 bits (the host checks the field size)
-    const int st = AXIS == 0 ? (int)G.sx : (int)G.sy;
-    const long base = AXIS == 0 ? (long)R.is * G.sx + (long)(R.js + o) * G.sy + k
-                                : (long)(R.is + o) * G.sx + (long)R.js * G.sy + k;
-    const long seg = base + (long)(l * RS) * st;
-    const real dt = (real)A.scal[S_DT];
-    const real fac = (real)(0.5 * A.scal[S_DT] * A.alpha);
-    const real* __restrict__ fam = VAR == VC ? nullptr : line_family<VAR, AXIS, real>(A.mu);
-    real* __restrict__ S = A.S;
-    // this thread's row e of the tiles: mym[e * TS], myq[e * TS]
-    real* mym = ls_dyn + threadIdx.x;
-    real* myq = ls_dyn + (VAR != VC ? (RS + 1) * TS : 0) + threadIdx.x;
-
-    if (VAR != VC) {
-        if (live) {
-            const real* mp = fam + seg + OFF * st;
-#pragma unroll
-            for (int e = 0; e <= RS; ++e) ls_cp_async<real>(mym + e * TS, mp + e * st);
-        } else {
-#pragma unroll
-            for (int e = 0; e <= RS; ++e) mym[e * TS] = (real)0;
-        }
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    if (AXIS == 0 && live) {
-#pragma unroll
-        for (int e = 0; e < RS; ++e) ls_cp_async<real>(myq + e * TS, A.q + seg + e * st);
-        asm volatile("cp.async.commit_group;\n" ::: "memory");
-    }
-    real rS[RS];
-    {
-        const real* sp = S + seg;
-#pragma unroll
-        for (int e = 0; e < RS; ++e) rS[e] = live ? sp[e * st] : (real)0;
-    }
-
-    // convective outflow value (x): the thread that owns the line's last row
-    real boun = (real)0;
-    if (AXIS == 0 && live && last_seg) {
-        const long rb = base + (long)n * st;
-        real Hb = -(real)A.scal[S_VBULK] * (A.q[rb] - A.q[rb - st]);
-        Hb = over_h<real>(Hb, K.hx, K.ihx, K.pow2);
-        A.H[rb] = Hb;
-        boun = rk_step<real>(dt, (real)A.g, Hb, (real)A.r, A.Hm[rb]);
-        A.qn[rb] = A.q[rb] + boun;
-    }
-    if (VAR != VC) {
-        // the viscosity rows have landed (the q rows may still be in flight)
-        if (AXIS == 0 && live) asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-        else asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    }
-
-    // row e of this segment: (la, lb, lc, lr) with the line's closures; la of
-    // the line's first row and lc of its last are dropped (the sequential
-    // sweep multiplies them by zero)
-    auto row = [&](int e, real& la, real& lb, real& lc, real& lr) {
-        if (!FULL && last_seg && e == RS - 1) {
-            la = (real)0;
-            lb = (real)1;
-            lc = (real)0;
-            lr = (real)0;
-            return;
-        }
-        real a, c;
-        line_ac<VAR, AXIS, real>(K, VAR == VC ? (real)0 : mym[e * TS], VAR == VC ? (real)0 : mym[(e + 1) * TS], a, c);
-        const real b = -(a + c);
-        la = -fac * a;
-        lb = (real)1 - fac * b;
-        lc = -fac * c;
-        lr = rS[e];
-        if (e == 0 && l == 0) {
-            if (LO == 1) lb += la;
-            else if (LO == 2) lb -= la;
-            la = (real)0;
-        }
-        if (last_seg && e == (FULL ? RS - 1 : RS - 2)) {
-            if (AXIS == 0) lr -= lc * boun;
-            else if (HI == 1) lb += lc;
-            else if (HI == 2) lb -= lc;
-            lc = (real)0;
-        }
-    };
-    auto fresh = [&]() {
-#pragma unroll
-        for (int e = 0; e < RS; ++e) ls_fresh(rS[e]);
-        asm volatile("" ::: "memory");
-    };
-
-    // interior rows top-down: x_e = rh - ah S_l - ch x_{e+1}; at the last
-    // interior row x_{e+1} is the next separator
-    real gL, vL, wL;
-    {
-        real la, lb, lc, lr;
-        row(1, la, lb, lc, lr);
-        real ib = rcp_<real>(lb);
-        real ch = lc * ib, rh = lr * ib, ah = la * ib;
-#pragma unroll
-        for (int e = 2; e < RS; ++e) {
-            row(e, la, lb, lc, lr);
-            ib = rcp_<real>(lb - la * ch);
-            rh = (lr - la * rh) * ib;
-            ah = -la * ah * ib;
-            ch = lc * ib;
-        }
-        gL = rh;
-        vL = ah;
-        wL = ch;
-    }
-    fresh();
-    // bottom-up: x_e = rb - ab S_l - cb S_{l+1} down to the first interior row
-    real g1, v1, w1;
-    {
-        real la, lb, lc, lr;
-        row(RS - 1, la, lb, lc, lr);
-        real ib = rcp_<real>(lb);
-        real rb = lr * ib, cb = lc * ib, ab = la * ib;
-#pragma unroll
-        for (int e = RS - 2; e >= 1; --e) {
-            row(e, la, lb, lc, lr);
-            ib = rcp_<real>(lb - lc * ab);
-            rb = (lr - lc * rb) * ib;
-            cb = -lc * cb * ib;
-            ab = la * ib;
-        }
-        g1 = rb;
-        v1 = ab;
-        w1 = cb;
-    }
-    fresh();
-    tail[0][l][lane] = gL;
-    tail[1][l][lane] = vL;
-    tail[2][l][lane] = wL;
-    __syncthreads();
-    {
-        // separator row: a0 x_{-1} + b0 S_l + c0 x_1 = r0 with x_{-1} the
-        // previous segment's last interior row
-        real a0, b0, c0, r0;
-        row(0, a0, b0, c0, r0);
-        real gp = (real)0, vp = (real)0, wp = (real)0;
-        if (l > 0) {
-            gp = tail[0][l - 1][lane];
-            vp = tail[1][l - 1][lane];
-            wp = tail[2][l - 1][lane];
-        }
-        eq[0][l][lane] = -a0 * vp;
-        eq[1][l][lane] = b0 - a0 * wp - c0 * v1;
-        eq[2][l][lane] = -c0 * w1;
-        eq[3][l][lane] = r0 - a0 * gp - c0 * g1;
-    }
-    __syncthreads();
-    if (l == 0) {
-        // the P separator equations of this lane's line (Thomas); c' and
-        // the eliminated rhs replace gamma and rho in place
-        real ib = rcp_<real>(eq[1][0][lane]);
-        real cp = eq[2][0][lane] * ib, rp = eq[3][0][lane] * ib;
-        eq[2][0][lane] = cp;
-        eq[3][0][lane] = rp;
-#pragma unroll
-        for (int t = 1; t < P; ++t) {
-            const real al = eq[0][t][lane];
-            ib = rcp_<real>(eq[1][t][lane] - al * cp);
-            cp = eq[2][t][lane] * ib;
-            rp = (eq[3][t][lane] - al * rp) * ib;
-            eq[2][t][lane] = cp;
-            eq[3][t][lane] = rp;
-        }
-        real x = rp;
-        sep[P - 1][lane] = x;
-        sep[P][lane] = (real)0;
-#pragma unroll
-        for (int t = P - 2; t >= 0; --t) {
-            x = eq[3][t][lane] - eq[2][t][lane] * x;
-            sep[t][lane] = x;
-        }
-    }
-    __syncthreads();
-    if (!live) return;
-    const real Sl = sep[l][lane], Sn = sep[l + 1][lane];
-    fresh();
-
-    // interior rows with both separators known: Thomas with x_0 = S_l and
-    // x_RS = S_{l+1}; c' in cq, the eliminated rhs replaces rS
-    real cq[RS];
-    {
-        real la, lb, lc, lr;
-        row(1, la, lb, lc, lr);
-        real ib = rcp_<real>(lb);
-        cq[1] = lc * ib;
-        rS[1] = (lr - la * Sl) * ib;
-#pragma unroll
-        for (int e = 2; e < RS; ++e) {
-            row(e, la, lb, lc, lr);
-            ib = rcp_<real>(lb - la * cq[e - 1]);
-            cq[e] = lc * ib;
-            rS[e] = (lr - la * rS[e - 1]) * ib;
-        }
-    }
-    if (AXIS == 0) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-    // q_new (x; for c also its Neumann ghosts in y then z, as k_line_pf) or
-    // the solution in place (y)
-    const int jl = R.js + o;
-    const bool jlo = AXIS == 0 && VAR == VC && jl == R.js, jhi = AXIS == 0 && VAR == VC && jl == R.je;
-    const bool klo = AXIS == 0 && VAR == VC && k == R.ks, khi = AXIS == 0 && VAR == VC && k == R.ke;
-    const bool edge = jlo | jhi | klo | khi;
-    auto put = [&](int e, real x) {
-        if (!FULL && last_seg && e == RS - 1) return;
-        const long id = seg + e * st;
-        if (AXIS != 0) {
-            S[id] = x;
-            return;
-        }
-        const real v = myq[e * TS] + x;
-        A.qn[id] = v;
-        if (edge) {
-            const long sy = G.sy;
-            if (jlo) A.qn[id - sy] = v;
-            if (jhi) A.qn[id + sy] = v;
-            if (klo) {
-                A.qn[id - 1] = v;
-                if (jlo) A.qn[id - sy - 1] = v;
-                if (jhi) A.qn[id + sy - 1] = v;
-            }
-            if (khi) {
-                A.qn[id + 1] = v;
-                if (jlo) A.qn[id - sy + 1] = v;
-                if (jhi) A.qn[id + sy + 1] = v;
-            }
-        }
-    };
-    real x = Sn;
-#pragma unroll
-    for (int e = RS - 1; e >= 1; --e) {
-        x = rS[e] - cq[e] * x;
-        put(e, x);
-    }
-    put(0, Sl);
-}
-template <int VAR, int AXIS, int P, int RS, bool FULL, typename real = float>
-__global__ void __launch_bounds__(32 * P, (RS <= 16 && sizeof(real) == 4) ? 2 : 1)
-    k_line_seg(Geo G, Rng R, Consts K, XsweepArgs<real> A)
-{
-    k_line_seg_run<VAR, AXIS, P, RS, FULL, real>(blockIdx, gridDim, G, R, K, A);
-}
-template <int VAR, int AXIS, int P, int RS, bool FULL, typename real = float>
-struct k_line_seg_b {
-    static constexpr auto run = &k_line_seg_run<VAR, AXIS, P, RS, FULL, real>;
-    static constexpr int maxt = 32 * P, minb = (RS <= 16 && sizeof(real) == 4) ? 2 : 1;
 };
 
 }  // namespace

@@ -42,21 +42,23 @@ KERNEL_WORDS = {
 FAMILY = {
     "explicit_c": "k_explicit_tma", "explicit_u": "k_explicit_tma", "explicit_v": "k_explicit_tma",
     "explicit_w": "k_explicit_tma",
-    "adi_y_c": "k_line_seg (y)", "adi_y_u": "k_line_pf (y)", "adi_y_v": "k_line_pf (y)",
-    "adi_y_w": "k_line_pf (y)",
+    "adi_y_c": "k_line_seg (y)", "adi_y_u": "k_line_seg (y)", "adi_y_v": "k_line_seg (y)",
+    "adi_y_w": "k_line_seg (y)",
     "adi_z_c": "k_adi_z_part", "adi_z_u": "k_adi_z_part", "adi_z_v": "k_adi_z_part",
     "adi_z_w": "k_adi_z_part",
-    "adi_x_c": "k_line_pf (x)", "adi_x_u": "k_line_pf (x)", "adi_x_v": "k_line_pf (x)",
-    "adi_x_w": "k_line_pf (x)",
+    "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
+    "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_fft": "k_dct_fft",
-    "poisson_x": "k_poisson_x", "project": "k_project2", "cfl": "k_cfl",
+    "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl",
 }
 
 # the exact FP64 form's kernels where they differ (bit-reproducible order of
 # operations: no paired-cell kernels, DMMA DCT, tiled z solve)
 FAMILY_EXACT = dict(FAMILY, **{
     "explicit_c": "k_explicit", "explicit_u": "k_explicit", "explicit_v": "k_explicit",
-    "explicit_w": "k_explicit", "adi_y_c": "k_line_pf (y)",
+    "explicit_w": "k_explicit", "adi_y_c": "k_line_pf (y)", "adi_y_u": "k_line_pf (y)", "adi_y_v": "k_line_pf (y)",
+    "adi_y_w": "k_line_pf (y)", "adi_x_c": "k_line_pf (x)", "adi_x_u": "k_line_pf (x)", "adi_x_v": "k_line_pf (x)",
+    "adi_x_w": "k_line_pf (x)", "poisson_x": "k_poisson_x",
     "adi_z_c": "k_adi_z_tiled", "adi_z_u": "k_adi_z_tiled", "adi_z_v": "k_adi_z_tiled",
     "adi_z_w": "k_adi_z_tiled",
     "viscosity": "k_viscosity", "div_rhs": "k_div_rhs", "dct_gemm": "k_gemm_dmma", "project": "k_project"})
@@ -71,7 +73,7 @@ FAMILY_FP32 = {
     "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
     "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_umma": "k_dct_umma_p",
-    "poisson_x": "k_poisson_x2", "project": "k_project2", "cfl": "k_cfl2",
+    "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl2",
 }
 
 
