@@ -48,6 +48,15 @@ struct UmmaPlan {
     float* Tlo[4] = {};
 };
 
+// One axis's DCT passes outside the exact form and the tcgen05 path: by FFT
+// (cos / sin of 2 pi m / N and of pi k / (2N)) or by the folded dense product
+// (its tables of both kinds in fragment order)
+struct DctAxis {
+    enum Mode { NONE, FFT, FOLD } mode = NONE;
+    double2 *tw = nullptr, *wq = nullptr;
+    double* table[2] = {nullptr, nullptr};
+};
+
 }  // namespace pll
 
 using namespace pll;
@@ -66,12 +75,9 @@ struct pllgpu_ctx {
     double *mode_cc = nullptr, *mode_rr = nullptr;  // FP64 Poisson mode scratch
     double* stage64 = nullptr;  // one padded FP64 field (mixed-form transfers)
     double *lam_y = nullptr, *lam_z = nullptr;
-    // FP64 form's FFT DCT passes (power-of-two planes): per axis (0 y, 1 z)
-    // cos / sin of 2 pi m / N and of pi k / (2N)
-    bool fft_on = false;
+    DctAxis dct[2];             // the DCT passes along y and z
     bool xt_on = false;         // FP64 form: TMA-staged marching explicit operator
     int xt_cap[4] = {};         // its blocks resident at once, per variable
-    double2 *fft_tw[2] = {nullptr, nullptr}, *fft_wq[2] = {nullptr, nullptr};
     UmmaPlan um;                // precision form's tensor-core DCT (when shapes allow)
     double* scal = nullptr;     // device scalars (S_*)
     int* status = nullptr;      // device sticky status bits

@@ -132,14 +132,17 @@ template <int N>
 __device__ __forceinline__ int mperm(int j) { return (j & 1) ? N - 1 - (j >> 1) : (j >> 1); }
 
 // KIND 0: DCT-II (REDFT10); KIND 1: DCT-III (REDFT01).  2*FFT_PB
-// consecutive lines per block (inner must be a multiple of 2*FFT_PB).
+// consecutive lines per block; WHOLE: inner is a multiple of 2*FFT_PB, so
+// that a block's lines are all there and evenly spaced.  Stored as T, FP64
+// arithmetic.
 // tw: cos / sin of 2 pi m / N (m < N); wq: cos / sin of pi k / (2N) (k < N)
-template <typename real, int N, int KIND, bool CONTIG>
+template <typename T, int N, int KIND, bool CONTIG, bool WHOLE>
 __device__ __forceinline__ void k_dct_fft_run(const uint3 blockIdx, const dim3 gridDim,
-    FftLines d, const real* __restrict__ in,
-                                                         real* __restrict__ out, const double2* __restrict__ tw,
+    FftLines d, const T* __restrict__ in,
+                                                         T* __restrict__ out, const double2* __restrict__ tw,
                                                          const double2* __restrict__ wq)
 {
+    using real = double;
     constexpr int R1 = FftShape<N>::R1, R2 = FftShape<N>::R2, ROW = FftRow<N>::value;
     constexpr int TL = 2 * FFT_PB;   // real lines per block
     extern __shared__ __align__(16) unsigned char fsm[];
@@ -147,8 +150,18 @@ __device__ __forceinline__ void k_dct_fft_run(const uint3 blockIdx, const dim3 g
     const int tid = threadIdx.x;
     const long L0 = (long)blockIdx.x * TL;
     const long a = L0 / d.inner, b0 = L0 % d.inner;
-    const real* gin = in + a * d.sa_in + b0 * d.sb_in;
-    real* gout = out + a * d.sa_out + b0 * d.sb_out;
+    const T* gin = in + a * d.sa_in + b0 * d.sb_in;
+    T* gout = out + a * d.sa_out + b0 * d.sb_out;
+    __shared__ long off_in[WHOLE ? 1 : TL], off_out[WHOLE ? 1 : TL];   // of a block's lines, from its first
+    const int nl = WHOLE ? TL : min(TL, d.lines - (int)L0);
+    if (!WHOLE) {
+        if (tid < TL) {
+            const long la = (L0 + tid) / d.inner, lb = (L0 + tid) % d.inner;
+            off_in[tid] = (la - a) * d.sa_in + (lb - b0) * d.sb_in;
+            off_out[tid] = (la - a) * d.sa_out + (lb - b0) * d.sb_out;
+        }
+        __syncthreads();
+    }
 
     // ---- load: line l of the tile -> pair l/2, real (even l) or imaginary
     // part; all of a thread's loads are issued before the first store to
@@ -161,7 +174,8 @@ __device__ __forceinline__ void k_dct_fft_run(const uint3 blockIdx, const dim3 g
             const int e = tid + t * FFT_THREADS;
             int l, p;
             if (CONTIG) { l = e / N; p = e % N; } else { p = e / TL; l = e % TL; }
-            v[t] = CONTIG ? gin[(long)l * d.sb_in + p] : gin[l + (long)p * d.se_in];
+            if (WHOLE) v[t] = (real)(CONTIG ? gin[(long)l * d.sb_in + p] : gin[l + (long)p * d.se_in]);
+            else v[t] = l < nl ? (real)gin[off_in[l] + (CONTIG ? (long)p : (long)p * d.se_in)] : (real)0;
         }
 #pragma unroll
         for (int t = 0; t < LPT; ++t) {
@@ -262,20 +276,25 @@ __device__ __forceinline__ void k_dct_fft_run(const uint3 blockIdx, const dim3 g
         const int n = KIND == 0 ? p : mperm<N>(p);
         const real* slot = &C[(l >> 1) * ROW + fslot<N>(n)].re;
         const real v = slot[l & 1] * sc;
-        if (CONTIG) gout[(long)l * d.sb_out + p] = v;
-        else gout[l + (long)p * d.se_out] = v;
+        if (!WHOLE) {
+            if (l < nl) gout[off_out[l] + (CONTIG ? (long)p : (long)p * d.se_out)] = (T)v;
+        } else if (CONTIG) {
+            gout[(long)l * d.sb_out + p] = (T)v;
+        } else {
+            gout[l + (long)p * d.se_out] = (T)v;
+        }
     }
 }
-template <typename real, int N, int KIND, bool CONTIG>
-__global__ void __launch_bounds__(FFT_THREADS) k_dct_fft(FftLines d, const real* __restrict__ in,
-                                                         real* __restrict__ out, const double2* __restrict__ tw,
+template <typename T, int N, int KIND, bool CONTIG, bool WHOLE>
+__global__ void __launch_bounds__(FFT_THREADS) k_dct_fft(FftLines d, const T* __restrict__ in, T* __restrict__ out,
+                                                         const double2* __restrict__ tw,
                                                          const double2* __restrict__ wq)
 {
-    k_dct_fft_run<real, N, KIND, CONTIG>(blockIdx, gridDim, d, in, out, tw, wq);
+    k_dct_fft_run<T, N, KIND, CONTIG, WHOLE>(blockIdx, gridDim, d, in, out, tw, wq);
 }
-template <typename real, int N, int KIND, bool CONTIG>
+template <typename T, int N, int KIND, bool CONTIG, bool WHOLE>
 struct k_dct_fft_b {
-    static constexpr auto run = &k_dct_fft_run<real, N, KIND, CONTIG>;
+    static constexpr auto run = &k_dct_fft_run<T, N, KIND, CONTIG, WHOLE>;
     static constexpr int maxt = FFT_THREADS, minb = 0;
 };
 

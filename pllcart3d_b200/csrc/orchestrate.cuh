@@ -14,6 +14,7 @@
 
 #include "explicit_tma.cuh"
 #include "fft_dct.cuh"
+#include "fold_dct.cuh"
 #include "forms.h"
 #include "host_common.cuh"
 #include "line_part.cuh"
@@ -360,53 +361,69 @@ void launch_poisson_umma(pllgpu_ctx* ctx)
                 UmmaEpi{ny, ctx->G.sx, ctx->G.sy, 1, (float)(p2 ? 1.0 / four_n : four_n), p2 ? 1 : 2, 0}, phi0);
 }
 
-#if !PLL_FP64_EXACT
-// lengths the FFT passes take: powers of two with whole 16-line tiles
+// lengths the FFT passes take
 inline bool fft_len_ok(int n) { return n >= 16 && n <= 256 && (n & (n - 1)) == 0; }
 
-template <int N, int KIND, bool CONTIG>
-void fft_launch(pllgpu_ctx* ctx, const FftLines& d, int axis, const double* in, double* out)
+template <typename T, int N, int KIND, bool CONTIG>
+void fft_launch(pllgpu_ctx* ctx, const FftLines& d, int axis, const T* in, T* out)
 {
-    const unsigned grid = (unsigned)(d.lines / (2 * FFT_PB));
-    go<k_dct_fft_b<double, N, KIND, CONTIG>>(ctx, k_dct_fft<double, N, KIND, CONTIG>, grid, FFT_THREADS,
-                                             fft_smem_bytes<N>(), d, in, out, ctx->fft_tw[axis], ctx->fft_wq[axis]);
-}
-
-template <int KIND, bool CONTIG>
-void fft_pass(pllgpu_ctx* ctx, int N, const FftLines& d, int axis, const double* in, double* out)
-{
-    switch (N) {
-    case 16: fft_launch<16, KIND, CONTIG>(ctx, d, axis, in, out); break;
-    case 32: fft_launch<32, KIND, CONTIG>(ctx, d, axis, in, out); break;
-    case 64: fft_launch<64, KIND, CONTIG>(ctx, d, axis, in, out); break;
-    case 128: fft_launch<128, KIND, CONTIG>(ctx, d, axis, in, out); break;
-    default: fft_launch<256, KIND, CONTIG>(ctx, d, axis, in, out); break;
-    }
+    constexpr int TL = 2 * FFT_PB;
+    const unsigned grid = (unsigned)((d.lines + TL - 1) / TL);
+    const DctAxis& A = ctx->dct[axis];
+    if (d.inner % TL == 0)
+        go<k_dct_fft_b<T, N, KIND, CONTIG, true>>(ctx, k_dct_fft<T, N, KIND, CONTIG, true>, grid, FFT_THREADS,
+                                                  fft_smem_bytes<N>(), d, in, out, A.tw, A.wq);
+    else
+        go<k_dct_fft_b<T, N, KIND, CONTIG, false>>(ctx, k_dct_fft<T, N, KIND, CONTIG, false>, grid, FFT_THREADS,
+                                                   fft_smem_bytes<N>(), d, in, out, A.tw, A.wq);
     mark(ctx, "dct_fft");
 }
 
-// the FP64 form's Poisson solve with FFT DCT passes (compact [x][y][z])
-void launch_poisson_fft(pllgpu_ctx* ctx)
+// one DCT pass along an axis (0 y, 1 z: CONTIG) of length n
+template <typename T, int KIND, bool CONTIG>
+void dct_pass(pllgpu_ctx* ctx, int n, const FftLines& d, const T* in, T* out)
 {
-    Bufs<double>& B = ctx->b64;
+    constexpr int axis = CONTIG ? 1 : 0;
+    if (ctx->dct[axis].mode == DctAxis::FOLD) {
+        const size_t smem = fold_smem<CONTIG>(n);
+        if (smem > 48 * 1024)
+            cudaFuncSetAttribute(k_dct_fold<KIND, CONTIG, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        go<k_dct_fold_b<KIND, CONTIG, T>>(ctx, k_dct_fold<KIND, CONTIG, T>, (d.lines + FOLD_LINES - 1) / FOLD_LINES,
+                                          32 * fold_warps(n), smem, d, n, in, out, ctx->dct[axis].table[KIND]);
+        mark(ctx, "dct_fold");
+        return;
+    }
+    switch (n) {
+    case 16: fft_launch<T, 16, KIND, CONTIG>(ctx, d, axis, in, out); break;
+    case 32: fft_launch<T, 32, KIND, CONTIG>(ctx, d, axis, in, out); break;
+    case 64: fft_launch<T, 64, KIND, CONTIG>(ctx, d, axis, in, out); break;
+    case 128: fft_launch<T, 128, KIND, CONTIG>(ctx, d, axis, in, out); break;
+    default: fft_launch<T, 256, KIND, CONTIG>(ctx, d, axis, in, out); break;
+    }
+}
+
+// the Poisson solve by whole-line DCT passes (compact [x][y][z])
+template <typename T>
+void launch_poisson_lines(pllgpu_ctx* ctx)
+{
+    Bufs<T>& B = bufs<T>(ctx);
     const int nx = ctx->G.nx, ny = ctx->G.ny, nz = ctx->G.nz;
     const long N = (long)ny * nz;
     // y lines: (x, z) -> x*N + z, elements step nz; z lines: (x, y) -> x*N + y*nz
     const FftLines ylines{nx * nz, nz, N, 1, nz, N, 1, nz, 1.0};
     const FftLines zlines{nx * ny, ny, N, nz, 1, N, nz, 1, 1.0};
-    fft_pass<0, false>(ctx, ny, ylines, 0, B.dct1, B.dct2);
-    fft_pass<0, true>(ctx, nz, zlines, 1, B.dct2, B.dct1);
-    launch_modes<double>(ctx, B.dct1, 0);
-    fft_pass<1, false>(ctx, ny, ylines, 0, B.dct1, B.dct2);
-    // into phi's interior, times 1/(4 ny nz) (exact: a power of two)
+    dct_pass<T, 0, false>(ctx, ny, ylines, B.dct1, B.dct2);
+    dct_pass<T, 0, true>(ctx, nz, zlines, B.dct2, B.dct1);
+    launch_modes<T>(ctx, B.dct1, 0);
+    dct_pass<T, 1, false>(ctx, ny, ylines, B.dct1, B.dct2);
+    // into phi's interior, times 1/(4 ny nz)
     FftLines out = zlines;
     out.sa_out = ctx->G.sx;
     out.sb_out = ctx->G.sy;
     out.scale = 1.0 / (4.0 * (double)N);
-    double* phi0 = B.phi + (long)ctx->Rg.is * ctx->G.sx + (long)ctx->Rg.js * ctx->G.sy + ctx->Rg.ks;
-    fft_pass<1, true>(ctx, nz, out, 1, B.dct2, phi0);
+    T* phi0 = B.phi + (long)ctx->Rg.is * ctx->G.sx + (long)ctx->Rg.js * ctx->G.sy + ctx->Rg.ks;
+    dct_pass<T, 1, true>(ctx, nz, out, B.dct2, phi0);
 }
-#endif
 
 // phisolver_dct after its right-hand side is in dct1 (compact [x][y][z])
 template <typename real>
@@ -417,13 +434,12 @@ void launch_poisson(pllgpu_ctx* ctx)
             launch_poisson_umma(ctx);
             return;
         }
-    } else {
-#if !PLL_FP64_EXACT
-        if (ctx->fft_on) {
-            launch_poisson_fft(ctx);
+    }
+    if constexpr (std::is_same<real, float>::value || !PLL_FP64_EXACT) {
+        if (ctx->dct[0].mode != DctAxis::NONE && ctx->dct[1].mode != DctAxis::NONE) {
+            launch_poisson_lines<real>(ctx);
             return;
         }
-#endif
     }
     Bufs<real>& B = bufs<real>(ctx);
     const int nx = ctx->G.nx, ny = ctx->G.ny, nz = ctx->G.nz;
@@ -915,33 +931,65 @@ bool setup_umma(pllgpu_ctx* c)
     return true;
 }
 
-#if !PLL_FP64_EXACT
 // twiddle tables of the FFT DCT passes, evaluated in long double and
 // rounded once (arguments reduced exactly: m < N, k < N)
-bool setup_fft(pllgpu_ctx* c)
+bool setup_fft(pllgpu_ctx* c, int axis, int N)
 {
-    const int len[2] = {c->P.ny, c->P.nz};
     const long double pi = 3.141592653589793238462643383279502884L;
-    for (int a = 0; a < 2; ++a) {
-        const int N = len[a];
-        std::vector<double2> tw((size_t)N), wq((size_t)N);
-        for (int m = 0; m < N; ++m) {
-            const long double t = 2.0L * pi * (long double)m / (long double)N;
-            tw[m] = make_double2((double)cosl(t), (double)sinl(t));
-            const long double q = pi * (long double)m / (2.0L * (long double)N);
-            wq[m] = make_double2((double)cosl(q), (double)sinl(q));
-        }
-        c->fft_tw[a] = (double2*)dalloc<double>(c, 2L * N);
-        c->fft_wq[a] = (double2*)dalloc<double>(c, 2L * N);
-        if (!c->fft_tw[a] || !c->fft_wq[a]) return false;
-        if (cudaMemcpy(c->fft_tw[a], tw.data(), sizeof(double2) * N, cudaMemcpyHostToDevice) != cudaSuccess ||
-            cudaMemcpy(c->fft_wq[a], wq.data(), sizeof(double2) * N, cudaMemcpyHostToDevice) != cudaSuccess)
-            return false;
+    std::vector<double2> tw((size_t)N), wq((size_t)N);
+    for (int m = 0; m < N; ++m) {
+        const long double t = 2.0L * pi * (long double)m / (long double)N;
+        tw[m] = make_double2((double)cosl(t), (double)sinl(t));
+        const long double q = pi * (long double)m / (2.0L * (long double)N);
+        wq[m] = make_double2((double)cosl(q), (double)sinl(q));
     }
-    c->fft_on = true;
+    DctAxis& A = c->dct[axis];
+    A.tw = (double2*)dalloc<double>(c, 2L * N);
+    A.wq = (double2*)dalloc<double>(c, 2L * N);
+    if (!A.tw || !A.wq ||
+        cudaMemcpy(A.tw, tw.data(), sizeof(double2) * N, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(A.wq, wq.data(), sizeof(double2) * N, cudaMemcpyHostToDevice) != cudaSuccess)
+        return false;
+    A.mode = DctAxis::FFT;
     return true;
 }
-#endif
+
+// the folded matrices of both kinds in fragment order (fold_dct.cuh)
+bool setup_fold(pllgpu_ctx* c, int axis, int n)
+{
+    DctAxis& A = c->dct[axis];
+    const int KB = fold_kb(n), MB = fold_mb(n), half = (n + 1) / 2;
+    std::vector<double> M((size_t)n * n), t((size_t)fold_table(n));
+    for (int kind = 0; kind < 2; ++kind) {
+        dct_matrix<double>(kind, n, M.data());
+        for (int p = 0; p < 2; ++p)
+            for (int mb = 0; mb < MB; ++mb)
+                for (int kb = 0; kb < KB; ++kb)
+                    for (int l = 0; l < 32; ++l) {
+                        const int o = 8 * mb + l / 4, k = 4 * kb + l % 4;   // output, term
+                        // DCT-II: mode 2o+p from point k; DCT-III: point o from mode 2k+p
+                        const int row = kind == 0 ? 2 * o + p : o, col = kind == 0 ? k : 2 * k + p;
+                        const bool in = kind == 0 ? (row < n && k < half) : (o < half && col < n);
+                        t[(((size_t)p * MB + mb) * KB + kb) * 32 + l] = in ? M[(size_t)row * n + col] : 0.0;
+                    }
+        if (!(A.table[kind] = dalloc<double>(c, fold_table(n))) ||
+            cudaMemcpy(A.table[kind], t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess)
+            return false;
+    }
+    A.mode = DctAxis::FOLD;
+    return true;
+}
+
+// each axis by FFT where its length is a power of two up to 256, else by the
+// folded product; both axes longer than that keep the GEMM passes
+bool setup_dct_lines(pllgpu_ctx* c)
+{
+    const int len[2] = {c->P.ny, c->P.nz};
+    if (len[0] > FOLD_MAX || len[1] > FOLD_MAX) return true;
+    for (int a = 0; a < 2; ++a)
+        if (!(fft_len_ok(len[a]) ? setup_fft(c, a, len[a]) : setup_fold(c, a, len[a]))) return false;
+    return true;
+}
 
 // shared-memory opt-in of the marching explicit operator and the blocks of
 // it that the device holds at once
@@ -1001,10 +1049,10 @@ bool alloc_state(pllgpu_ctx* c)
             xt_setup<VW, float>(c);
         }
         const bool shape_ok = (p->ny == 128 || p->ny == 256) && (p->nz == 128 || p->nz == 256);
-        if (shape_ok && !p->exact_dct && p->dct_kernel != 1 && !setup_umma(c)) return false;
+        if (!p->exact_dct && p->dct_kernel != 1 && !(shape_ok ? setup_umma(c) : setup_dct_lines(c))) return false;
     } else {
 #if !PLL_FP64_EXACT
-        if (!p->exact_dct && fft_len_ok(p->ny) && fft_len_ok(p->nz) && !setup_fft(c)) return false;
+        if (!p->exact_dct && !setup_dct_lines(c)) return false;
         if (!p->exact_dct && c->nelem < (1L << 31) && encode_tiled()) {
             xt_setup<VC, double>(c);
             xt_setup<VU, double>(c);

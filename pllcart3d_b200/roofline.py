@@ -31,6 +31,7 @@ KERNEL_WORDS = {
     "dct_gemm": 2,       # one dense pass: in ; out (per launch)
     "dct_umma": 2,
     "dct_fft": 2,        # one FFT pass: in ; out
+    "dct_fold": 2,       # one folded dense pass: in ; out
     "poisson_x": 2,
     "project": 17,       # u v w phi mu(4) pg(3) ; u v w pg(3)
     "cfl": 3,
@@ -49,6 +50,7 @@ FAMILY = {
     "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
     "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_fft": "k_dct_fft",
+    "dct_fold": "k_dct_fold",
     "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl",
 }
 
@@ -73,6 +75,7 @@ FAMILY_FP32 = {
     "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
     "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_umma": "k_dct_umma_p",
+    "dct_fft": "k_dct_fft", "dct_fold": "k_dct_fold",
     "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl2",
 }
 
