@@ -3,10 +3,11 @@
 // and Adam, hand-written for the BF16 tensor cores (mma.sync m16n8k16, BF16
 // operands, FP32 accumulation).
 //
-// The forward convolution (and so the input gradient) runs on the 5th-
-// generation tensor cores where the shapes allow (nn_umma.cuh: tcgen05.mma
-// with a TMEM accumulator, TMA-staged operands whose out-of-bounds fill is
-// the zero padding), else on the mma.sync kernel below.
+// The forward convolution (and so the input gradient) and the weight gradient
+// run on the 5th-generation tensor cores where the shapes allow (nn_umma.cuh:
+// tcgen05.mma with a TMEM accumulator, TMA-staged operands whose out-of-bounds
+// fill is the zero padding; w rows of up to 128 voxels, channels in sixteens),
+// else on the mma.sync kernels below.
 //
 // Layout: activations are channels-last [n][d][h][w][c] (voxel-major, c
 // contiguous), BF16 as operands of the convolutions, FP32 for
@@ -545,38 +546,64 @@ EncodeTiledFn nn_encode()
     return fn;
 }
 
-// the geometry of the tcgen05 path, false when the shapes do not fit it:
-// tiles of 128 voxels made of whole w rows (W divides 128), hb rows of h and
-// db slices of d; Cout a multiple of the column tile; Cin a multiple of 16
+// voxel tiles of the tcgen05 kernels: the whole-row box of at most 128 voxels
+// that needs the fewest tiles, of equal ones the one tallest in h; false
+// where a w row is longer than a tile
+bool cu_boxes(int N, int D, int H, int W, CuGeom& g)
+{
+    if (W > CU_BM || N < 1 || D < 1 || H < 1 || W < 1) return false;
+    g.N = N, g.D = D, g.H = H, g.W = W;
+    long best = -1;
+    for (int hb = CU_BM / W < H ? CU_BM / W : H; hb >= 1; --hb) {
+        const int fit = CU_BM / (W * hb), db = fit < D ? fit : D;
+        const long tiles = (long)((H + hb - 1) / hb) * ((D + db - 1) / db);
+        if (best < 0 || tiles < best) {
+            best = tiles;
+            g.hb = hb;
+            g.db = db;
+        }
+    }
+    g.th = (H + g.hb - 1) / g.hb;
+    g.td = (D + g.db - 1) / g.db;
+    return cu_tiles(g) < (1L << 31);
+}
+
+// the geometry of the tcgen05 forward path, false when the shapes do not fit
+// it: Cout a multiple of the column tile, Cin a multiple of 16
 bool cu_geom(int N, int D, int H, int W, int Cin, int Cout, int ksize, CuGeom& g, int& BN, int& CK)
 {
-    const long V = (long)N * D * H * W;
-    if (V % CU_BM || W > CU_BM || CU_BM % W || Cin % 16 || Cout % 16) return false;
-    const int hb = (CU_BM / W) < H ? (CU_BM / W) : H;
-    if (H % hb || (CU_BM / W) % hb) return false;
-    const int db = CU_BM / (W * hb);
-    if (db > D || D % db) return false;
-    BN = Cout >= 128 ? 128 : Cout >= 64 ? 64 : Cout >= 32 ? 32 : 16;
-    if (Cout % BN) return false;
+    if (Cin % 16 || Cout % 16 || !cu_boxes(N, D, H, W, g)) return false;
+    BN = Cout % 128 == 0 ? 128 : Cout % 96 == 0 ? 96 : Cout % 64 == 0 ? 64 : Cout % 32 == 0 ? 32 : 16;
     CK = Cin % 64 == 0 ? 64 : Cin % 32 == 0 ? 32 : 16;
-    g = CuGeom{N, D, H, W, hb, db, Cin, Cout, ksize};
+    g.Cin = Cin, g.Cout = Cout, g.ksize = ksize;
     return true;
+}
+
+// channels-last [n][d][h][w][C] BF16 array, boxes of CB channels x the tile's
+// voxels, swizzled by the box row's width
+bool cu_act_map(const CuGeom& g, int C, int CB, const void* X, CUtensorMap* m)
+{
+    EncodeTiledFn fn = nn_encode();
+    if (!fn) return false;
+    const CUtensorMapSwizzle sw = CB == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                : CB == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+    const cuuint64_t c2 = (cuuint64_t)C * 2;
+    const cuuint64_t xd[5] = {(cuuint64_t)C, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.D, (cuuint64_t)g.N};
+    const cuuint64_t xs[4] = {c2, c2 * g.W, c2 * g.W * g.H, c2 * g.W * g.H * g.D};
+    const cuuint32_t xb[5] = {(cuuint32_t)CB, (cuuint32_t)g.W, (cuuint32_t)g.hb, (cuuint32_t)g.db, 1};
+    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void*)X, xd, xs, xb, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool cu_maps(const CuGeom& g, int BN, int CK, const void* X, const void* Wt, CUtensorMap* mx, CUtensorMap* mw)
 {
     EncodeTiledFn fn = nn_encode();
-    if (!fn) return false;
+    if (!fn || !cu_act_map(g, g.Cin, CK, X, mx)) return false;
     const CUtensorMapSwizzle sw = CK == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
                                 : CK == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
     const cuuint64_t c2 = (cuuint64_t)g.Cin * 2;
-    const cuuint64_t xd[5] = {(cuuint64_t)g.Cin, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.D, (cuuint64_t)g.N};
-    const cuuint64_t xs[4] = {c2, c2 * g.W, c2 * g.W * g.H, c2 * g.W * g.H * g.D};
-    const cuuint32_t xb[5] = {(cuuint32_t)CK, (cuuint32_t)g.W, (cuuint32_t)g.hb, (cuuint32_t)g.db, 1};
-    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    if (fn(mx, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, (void*)X, xd, xs, xb, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
-           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return false;
+    const cuuint32_t es[3] = {1, 1, 1};
     const int taps = g.ksize * g.ksize * g.ksize;
     const cuuint64_t wd[3] = {(cuuint64_t)g.Cin, (cuuint64_t)taps, (cuuint64_t)g.Cout};
     const cuuint64_t ws[2] = {c2, c2 * taps};
@@ -596,8 +623,7 @@ bool cu_launch(const CUtensorMap& mx, const CUtensorMap& mw, const CuGeom& g, co
             return false;
         attr = true;
     }
-    const long V = (long)g.N * g.D * g.H * g.W;
-    const dim3 grid((unsigned)(V / CU_BM), (unsigned)(g.Cout / BN));
+    const dim3 grid((unsigned)cu_tiles(g), (unsigned)(g.Cout / BN));
     k_conv_umma<BN, CK><<<grid, CU_THREADS, CuSmem<BN, CK>::DYN, st>>>(mx, mw, g, bias, Y32, (__nv_bfloat16*)Y16,
                                                                          act, slope);
     return true;
@@ -626,9 +652,80 @@ bool conv_umma(const void* X, int N, int D, int H, int W, int Cin, const void* W
     std::memset(&mw, 0, sizeof(mw));
     if (!cu_maps(g, BN, CK, X, Wt, &mx, &mw)) return false;
     if (BN == 128) return cu_launch_ck<128>(CK, mx, mw, g, bias, Y32, Y16, act, slope, st);
+    if (BN == 96) return cu_launch_ck<96>(CK, mx, mw, g, bias, Y32, Y16, act, slope, st);
     if (BN == 64) return cu_launch_ck<64>(CK, mx, mw, g, bias, Y32, Y16, act, slope, st);
     if (BN == 32) return cu_launch_ck<32>(CK, mx, mw, g, bias, Y32, Y16, act, slope, st);
     return cu_launch_ck<16>(CK, mx, mw, g, bias, Y32, Y16, act, slope, st);
+}
+
+// partial sums over the voxels that the weight gradient of one weight is
+// split into
+long wgrad_chunks(int taps, int Cin, int Cout)
+{
+    const long n = 4096 / ((long)taps * ((Cout + 63) / 64) * ((Cin + 63) / 64));
+    return n < 1 ? 1 : n;
+}
+
+template <int GA, int GN>
+bool wg_launch(const CuGeom& g, const WgPlan& p, dim3 grid, const CUtensorMap& mx, const CUtensorMap& mg, float* dW,
+               cudaStream_t st)
+{
+    const int smem = (int)WgSmem<GA, GN>::bytes(p.nb);
+    // a per-device attribute, set on every launch: the largest block's need
+    if (cudaFuncSetAttribute(k_wgrad_umma<GA, GN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)WgSmem<GA, GN>::bytes(128)) != cudaSuccess)
+        return false;
+    k_wgrad_umma<GA, GN><<<grid, CU_THREADS, smem, st>>>(mx, mg, g, p, dW);
+    return true;
+}
+
+// the weight gradient on tcgen05; false when the shapes do not fit (the
+// caller then runs the mma.sync kernel)
+bool wgrad_umma(const void* G, const void* X, int N, int D, int H, int W, int Cin, int Cout, int ksize, float* dW,
+                cudaStream_t st)
+{
+    CuGeom g;
+    if (Cin % 16 || Cout % 16 || ((uintptr_t)G & 15) || ((uintptr_t)X & 15) || !cu_boxes(N, D, H, W, g)) return false;
+    g.Cin = Cin, g.Cout = Cout, g.ksize = ksize;
+    const int GA = Cin % 64 == 0 ? 64 : Cin % 32 == 0 ? 32 : 16;
+    WgPlan p;
+    p.nb = Cout % 128 == 0 ? 128 : Cout % 64 == 0 ? 64 : Cout % 32 == 0 ? 32 : 16;
+    const int GN = p.nb >= 64 ? 64 : p.nb;
+    p.taps = ksize * ksize * ksize;
+    p.groups = p.taps * (Cin / GA);
+    const int tiles = (p.groups * GA + 127) / 128, most = 512 / p.nb;   // row tiles in all; a CTA's accumulators
+    p.splits = (tiles + most - 1) / most;
+    p.mt = (tiles + p.splits - 1) / p.splits;
+    p.splits = (tiles + p.mt - 1) / p.mt;
+    p.cols = 32;
+    while (p.cols < p.mt * p.nb) p.cols *= 2;
+    CUtensorMap mx, mg;
+    std::memset(&mx, 0, sizeof(mx));
+    std::memset(&mg, 0, sizeof(mg));
+    if (!cu_act_map(g, Cin, GA, X, &mx) || !cu_act_map(g, Cout, GN, G, &mg)) return false;
+    const long T = cu_tiles(g);
+    const int ny = p.splits * (Cout / p.nb);
+    int dev = 0, sms = 148;
+    if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    // one CTA per SM, the voxel tiles split between the CTAs of a row-tile set
+    const long nx = sms / ny < 1 ? 1 : sms / ny;
+    const dim3 grid((unsigned)(nx < T ? nx : T), (unsigned)ny);
+    // runs a weight's voxels are summed in (wgrad_chunks), in whole runs per CTA
+    const long per = (wgrad_chunks(p.taps, Cin, Cout) + grid.x / 2) / grid.x, most_runs = T / grid.x;
+    p.runs = (int)(per < 1 ? 1 : per > most_runs ? most_runs : per);
+    if (GA == 64) {
+        if (GN == 64) return wg_launch<64, 64>(g, p, grid, mx, mg, dW, st);
+        if (GN == 32) return wg_launch<64, 32>(g, p, grid, mx, mg, dW, st);
+        return wg_launch<64, 16>(g, p, grid, mx, mg, dW, st);
+    }
+    if (GA == 32) {
+        if (GN == 64) return wg_launch<32, 64>(g, p, grid, mx, mg, dW, st);
+        if (GN == 32) return wg_launch<32, 32>(g, p, grid, mx, mg, dW, st);
+        return wg_launch<32, 16>(g, p, grid, mx, mg, dW, st);
+    }
+    if (GN == 64) return wg_launch<16, 64>(g, p, grid, mx, mg, dW, st);
+    if (GN == 32) return wg_launch<16, 32>(g, p, grid, mx, mg, dW, st);
+    return wg_launch<16, 16>(g, p, grid, mx, mg, dW, st);
 }
 
 }  // namespace
@@ -658,9 +755,9 @@ int pllnn_conv_fwd(const void* X, int N, int D, int H, int W, int Cin, const voi
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
-// which kernel the forward convolution uses: 0 the tcgen05 kernel where the
-// shapes allow (default), 1 the mma.sync kernel, 2 the tcgen05 kernel or
-// status 6; returns the previous setting
+// which kernels the convolutions use: 0 the tcgen05 ones where the shapes
+// allow (default), 1 the mma.sync ones, 2 the tcgen05 kernel or status 6
+// (forward); returns the previous setting
 int pllnn_set_conv_path(int path)
 {
     const int old = g_conv_path;
@@ -682,12 +779,13 @@ int pllnn_conv_wgrad(const void* G, const void* X, int N, int D, int H, int W, i
                      float* dW, void* stream)
 {
     if (Cin % 8 || Cout % 8 || (ksize != 1 && ksize != 3)) return 6;
+    if (g_conv_path != 1 && wgrad_umma(G, X, N, D, H, W, Cin, Cout, ksize, dW, (cudaStream_t)stream))
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
     const Vol g{N, D, H, W};
     const long V = (long)N * D * H * W;
     const int ntaps = ksize * ksize * ksize;
     const int tiles = ((Cout + 63) / 64) * ((Cin + 63) / 64);
-    long chunks = 4096 / ((long)ntaps * tiles);
-    if (chunks < 1) chunks = 1;
+    const long chunks = wgrad_chunks(ntaps, Cin, Cout);
     long vchunk = (V + chunks - 1) / chunks;
     vchunk = ((vchunk + 15) / 16) * 16;
     if (vchunk < 256) vchunk = 256;

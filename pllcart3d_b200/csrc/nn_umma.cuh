@@ -14,6 +14,10 @@
 // reads.  The B tile (BN output channels x CK input channels of one tap) is
 // a 3-d TMA load of the weights [cout][tap][cin].  No multicast.
 //
+// A tile's voxels are W x hb x db whole w rows, up to 128 of them; the box may
+// reach past H or D (zero fill in, nothing stored), and rows of a box smaller
+// than 128 voxels are left out, so every volume with W <= 128 has tiles.
+//
 // CTA: 128 voxels x BN channels; four pipeline stages.
 //   warp 0      TMA producer (one thread)
 //   warp 1      TMEM owner and MMA issuer (one thread)
@@ -48,7 +52,7 @@ struct CuSmem {
     static constexpr uint32_t BAR_OFF = CU_STAGES * STAGE;
     static constexpr uint32_t TOTAL = BAR_OFF + 128;
     static constexpr uint32_t DYN = TOTAL + 1024;   // slack for 1024-byte alignment
-    static constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN;
+    static constexpr uint32_t TMEM_COLS = BN < 32 ? 32 : BN == 96 ? 128 : BN;
 };
 
 // shared-memory matrix descriptor (sm_100, version 1), K-major rows of CK
@@ -107,6 +111,11 @@ __device__ __noinline__ bool cu_wait(uint64_t* b, uint32_t parity, volatile int*
     }
 }
 
+__device__ __forceinline__ void cu_expect(uint64_t* bar, uint32_t bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(cu_smem(bar)), "r"(bytes) : "memory");
+}
+
 __device__ __forceinline__ void cu_tma_5d(void* dst, const CUtensorMap* map, uint64_t* bar, int c, int w, int h, int d,
                                           int n)
 {
@@ -151,13 +160,34 @@ __device__ __forceinline__ void cu_ld16(uint32_t taddr, uint32_t* r)
         : "r"(taddr));
 }
 
-// the voxel box of one tile: 128 voxels = W x hb x db (every tile starts a
-// whole w row; hb rows of h; db slices of d)
+// the voxel box of one tile: W x hb x db voxels (whole w rows; hb rows of h;
+// db slices of d), th x td tiles per volume
 struct CuGeom {
     int N, D, H, W;
-    int hb, db;
+    int hb, db, th, td;
     int Cin, Cout, ksize;
 };
+
+__host__ __device__ inline int cu_rows(const CuGeom& g) { return g.W * g.hb * g.db; }
+__host__ __device__ inline long cu_tiles(const CuGeom& g) { return (long)g.N * g.td * g.th; }
+
+__device__ __forceinline__ void cu_tile_at(const CuGeom& g, int t, int& n, int& d0, int& h0)
+{
+    h0 = (t % g.th) * g.hb;
+    t /= g.th;
+    d0 = (t % g.td) * g.db;
+    n = t / g.td;
+}
+
+__device__ __forceinline__ void cu_tap(int ksize, int tap, int& dz, int& dy, int& dx)
+{
+    dz = dy = dx = 0;
+    if (ksize == 3) {
+        dz = tap / 9 - 1;
+        dy = (tap / 3) % 3 - 1;
+        dx = tap % 3 - 1;
+    }
+}
 
 template <int BN, int CK>
 __global__ void __launch_bounds__(CU_THREADS, 1)
@@ -176,11 +206,9 @@ __global__ void __launch_bounds__(CU_THREADS, 1)
     volatile int* abort_flag = (volatile int*)(bars + 2 * CU_STAGES + 2);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const long m0 = (long)blockIdx.x * CU_BM;
     const int n0 = blockIdx.y * BN;
-    // the tile's first voxel (whole w rows): row index r0 = (n D + d) H + h
-    const long r0 = m0 / g.W;
-    const int h0 = (int)(r0 % g.H), d0 = (int)((r0 / g.H) % g.D), nn = (int)(r0 / ((long)g.H * g.D));
+    int h0, d0, nn;   // the tile's first voxel
+    cu_tile_at(g, blockIdx.x, nn, d0, h0);
     const int ntaps = g.ksize * g.ksize * g.ksize;
     const int nch = g.Cin / CK;
     const int nk = ntaps * nch;
@@ -215,16 +243,10 @@ __global__ void __launch_bounds__(CU_THREADS, 1)
                 const int s = kc % CU_STAGES;
                 if (kc >= CU_STAGES && !cu_wait(&empty[s], (kc / CU_STAGES + 1) & 1, abort_flag, true)) break;
                 const int tap = kc / nch, c0 = (kc - tap * nch) * CK;
-                int dz = 0, dy = 0, dx = 0;
-                if (g.ksize == 3) {
-                    dz = tap / 9 - 1;
-                    dy = (tap / 3) % 3 - 1;
-                    dx = tap % 3 - 1;
-                }
+                int dz, dy, dx;
+                cu_tap(g.ksize, tap, dz, dy, dx);
                 uint8_t* st = sm + s * L::STAGE;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(cu_smem(&full[s])),
-                             "r"(L::A_BYTES + L::B_BYTES)
-                             : "memory");
+                cu_expect(&full[s], (uint32_t)(cu_rows(g) * CK * 2) + L::B_BYTES);
                 cu_tma_5d(st, &tmX, &full[s], c0, dx, h0 + dy, d0 + dz, nn);
                 cu_tma_3d(st + L::A_BYTES, &tmW, &full[s], c0, tap, n0);
                 last[s] = kc;
@@ -259,31 +281,36 @@ __global__ void __launch_bounds__(CU_THREADS, 1)
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         const int q = warp & 3;
         const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
-        const long row = m0 + 32 * q + lane;
+        const int r = 32 * q + lane, rh = r / g.W, h = h0 + rh % g.hb, d = d0 + rh / g.hb;
+        const long row = (((long)nn * g.D + d) * g.H + h) * g.W + r % g.W;
+        const bool live = r < cu_rows(g) && h < g.H && d < g.D;
         if (ok) {
 #pragma unroll 1
             for (int c0 = 0; c0 < BN; c0 += 16) {
                 uint32_t v[16];
                 cu_ld16(trow + c0, v);
                 asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-                float y[16];
+                if (live) {
+                    float y[16];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(v[j]) + (bias ? bias[n0 + c0 + j] : 0.f);
-                const long o = row * g.Cout + n0 + c0;
-                if (Y32) {
+                    for (int j = 0; j < 16; ++j) y[j] = __uint_as_float(v[j]) + (bias ? bias[n0 + c0 + j] : 0.f);
+                    const long o = row * g.Cout + n0 + c0;
+                    if (Y32) {
 #pragma unroll
-                    for (int j = 0; j < 16; j += 4) *(float4*)(Y32 + o + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
-                }
-                if (Y16) {
-                    __align__(16) __nv_bfloat16 b[16];
-#pragma unroll
-                    for (int j = 0; j < 16; ++j) {
-                        const float a = act ? (y[j] > 0.f ? y[j] : slope * y[j]) : y[j];
-                        b[j] = __float2bfloat16(a);
+                        for (int j = 0; j < 16; j += 4) *(float4*)(Y32 + o + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
                     }
-                    *(uint4*)(Y16 + o) = *(const uint4*)&b[0];
-                    *(uint4*)(Y16 + o + 8) = *(const uint4*)&b[8];
+                    if (Y16) {
+                        __align__(16) __nv_bfloat16 b[16];
+#pragma unroll
+                        for (int j = 0; j < 16; ++j) {
+                            const float a = act ? (y[j] > 0.f ? y[j] : slope * y[j]) : y[j];
+                            b[j] = __float2bfloat16(a);
+                        }
+                        *(uint4*)(Y16 + o) = *(const uint4*)&b[0];
+                        *(uint4*)(Y16 + o + 8) = *(const uint4*)&b[8];
+                    }
                 }
+                __syncwarp();
             }
         }
     }
@@ -293,6 +320,224 @@ __global__ void __launch_bounds__(CU_THREADS, 1)
     if (warp == 1) {
         asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(L::TMEM_COLS));
+    }
+    if (threadIdx.x == 0 && *abort_flag) atomicOr(&g_nn_status, 0x100);
+}
+
+// ---- weight gradient -------------------------------------------------------------
+// dW[co][tap][ci] += sum over voxels of G[v][co] X[v + o(tap)][ci] as a GEMM
+// whose K axis is the voxels: D (rows: 128 of the (tap, input channel) pairs,
+// columns: output channels) accumulates in tensor memory over all of a CTA's
+// voxel tiles and goes to dW by FP32 atomics once.  Both operands are the
+// channels-last arrays themselves, [voxel][channel] tiles brought in by the
+// same 5-d TMA boxes as the forward pass (zero fill = zero padding): channels
+// are contiguous, so both are MN-major operands.  A row tile is 128 / GA groups
+// of GA channels, each group one tap's box, GA the largest of 64, 32, 16 that
+// divides Cin; with Cin = 96 or 16 and one group per row tile most of the
+// tensor pipe's rows would be empty.
+// Bound: the boxes' L2 -> shared traffic (each X tile is fetched once per tap,
+// 2 GA bytes a voxel for 2 GA N operations).  8 x 128x64x64 voxels, 96 -> 32
+// channels: 21.0 ms on the warp-level kernel, whose every 16 voxels passed two
+// block barriers and a transposing store.
+// The tensor pipe's running sum truncates, so a weight's voxels are summed in
+// as many separate runs as the warp-level kernel has voxel chunks: after each
+// run the accumulators are added to dW, rounded to nearest, and start anew.
+// Roles as k_conv_umma; shared memory: WG_STAGES row tiles of A, two of G.
+constexpr int WG_STAGES = 4;
+
+struct WgPlan {
+    int taps, groups;      // of GA channels: taps * Cin / GA
+    int nb;                // output channels (columns) per CTA
+    int mt;                // row tiles per CTA
+    int splits;            // CTAs that share the row tiles
+    int cols;              // tensor-memory columns
+    int runs;              // of voxel tiles per CTA
+};
+
+template <int GA, int GN>
+struct WgSmem {
+    static constexpr uint32_t A_GROUP = 128 * GA * 2, A_TILE = 128 * 128 * 2, G_GROUP = 128 * GN * 2;
+    static uint32_t bytes(int nb) { return WG_STAGES * A_TILE + 2 * 128 * (uint32_t)nb * 2 + 256 + 1024; }
+};
+
+// MN-major descriptor: K rows of GA (GN) channels, 8-row groups SBO apart,
+// channel groups LBO apart
+template <int GC>
+__device__ __forceinline__ uint64_t wg_desc(uint32_t saddr)
+{
+    constexpr uint64_t layout = GC == 64 ? 2 : GC == 32 ? 4 : 6;   // SWIZZLE_128B / 64B / 32B
+    constexpr uint64_t sbo = 8 * GC * 2, lbo = 128 * GC * 2;
+    return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((lbo >> 4) << 16) | ((sbo >> 4) << 32) | ((uint64_t)1 << 46) |
+           (layout << 61);
+}
+
+template <int GA, int GN>
+__global__ void __launch_bounds__(CU_THREADS, 1)
+    k_wgrad_umma(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmG, CuGeom g, WgPlan p,
+                 float* __restrict__ dW)
+{
+    using L = WgSmem<GA, GN>;
+    constexpr int MG = 128 / GA;   // groups of a row tile
+    extern __shared__ uint8_t cu_raw[];
+    uint8_t* sm = (uint8_t*)(((uintptr_t)cu_raw + 1023) & ~(uintptr_t)1023);
+    const uint32_t g_tile = 128 * (uint32_t)p.nb * 2;
+    uint8_t* smG = sm + WG_STAGES * L::A_TILE;
+    uint64_t* bars = (uint64_t*)(smG + 2 * g_tile);
+    uint64_t *full = bars, *empty = bars + WG_STAGES, *gfull = bars + 2 * WG_STAGES, *gempty = gfull + 2;
+    uint64_t *done = gempty + 2, *drained = done + 1;
+    volatile uint32_t* tmem_slot = (volatile uint32_t*)(done + 2);
+    volatile int* abort_flag = (volatile int*)(done + 3);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int split = blockIdx.y % p.splits, n0 = (blockIdx.y / p.splits) * p.nb;
+    const int mt0 = split * p.mt;
+    const int mts = min(p.mt, (p.groups + MG - 1) / MG - mt0);   // this CTA's row tiles (>= 1)
+    const long T = cu_tiles(g);
+    // run c of this CTA: tiles [run(c), run(c + 1))
+    auto run = [&](int c) { return (int)(T * ((long)blockIdx.x * p.runs + c) / ((long)gridDim.x * p.runs)); };
+    const int t0 = run(0), t1 = run(p.runs);
+    const int rows = cu_rows(g), ksteps = (rows + 15) / 16;
+    const int cgroups = g.Cin / GA;
+
+    // rows past a small box and groups past the last tap stay zero
+    for (uint32_t i = threadIdx.x; i < (WG_STAGES * L::A_TILE + 2 * g_tile) / 16; i += CU_THREADS)
+        ((uint4*)sm)[i] = make_uint4(0, 0, 0, 0);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < WG_STAGES; ++s) {
+            cu_bar_init(&full[s], 1);
+            cu_bar_init(&empty[s], 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            cu_bar_init(&gfull[s], 1);
+            cu_bar_init(&gempty[s], 1);
+        }
+        cu_bar_init(done, 1);
+        cu_bar_init(drained, 4);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+    }
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
+                         cu_smem((const void*)tmem_slot)),
+                     "r"((uint32_t)p.cols));
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int last[WG_STAGES], glast[2] = {-1, -1}, kc = 0;
+#pragma unroll
+            for (int s = 0; s < WG_STAGES; ++s) last[s] = -1;
+            bool ok = true;
+            for (int t = t0; t < t1 && ok; ++t) {
+                const int it = t - t0, gb = it & 1;
+                int n, d0, h0;
+                cu_tile_at(g, t, n, d0, h0);
+                if (it >= 2 && !cu_wait(&gempty[gb], (it / 2 + 1) & 1, abort_flag, true)) break;
+                cu_expect(&gfull[gb], (uint32_t)(rows * p.nb * 2));
+                for (int c = 0; c < p.nb / GN; ++c)
+                    cu_tma_5d(smG + gb * g_tile + c * L::G_GROUP, &tmG, &gfull[gb], n0 + c * GN, 0, h0, d0, n);
+                glast[gb] = it;
+                for (int m = 0; m < mts; ++m, ++kc) {
+                    const int s = kc % WG_STAGES, first = (mt0 + m) * MG, ng = min(MG, p.groups - first);
+                    if (kc >= WG_STAGES && !cu_wait(&empty[s], (kc / WG_STAGES + 1) & 1, abort_flag, true)) {
+                        ok = false;
+                        break;
+                    }
+                    cu_expect(&full[s], (uint32_t)(ng * rows * GA * 2));
+                    for (int q = 0; q < ng; ++q) {
+                        const int tap = (first + q) / cgroups, c0 = ((first + q) % cgroups) * GA;
+                        int dz, dy, dx;
+                        cu_tap(g.ksize, tap, dz, dy, dx);
+                        cu_tma_5d(sm + s * L::A_TILE + q * L::A_GROUP, &tmX, &full[s], c0, dx, h0 + dy, d0 + dz, n);
+                    }
+                    last[s] = kc;
+                }
+            }
+            // drain: no copy may still be landing when the CTA leaves
+            for (int s = 0; s < WG_STAGES; ++s)
+                if (last[s] >= 0) cu_wait(&full[s], (last[s] / WG_STAGES) & 1, abort_flag, false);
+            for (int s = 0; s < 2; ++s)
+                if (glast[s] >= 0) cu_wait(&gfull[s], (glast[s] / 2) & 1, abort_flag, false);
+        }
+        __syncwarp();
+    } else if (warp == 1) {
+        if (lane == 0) {
+            // kind::f16, D = F32, A = B = BF16, both MN-major, M = 128, N = nb
+            const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 15) | (1u << 16) |
+                                   ((uint32_t)(p.nb >> 3) << 17) | (8u << 24);
+            int kc = 0;
+            bool ok = true;
+            for (int c = 0; c < p.runs; ++c) {
+                if (c > 0 && ok) {   // the previous run's sums have been taken
+                    ok = cu_wait(drained, (c - 1) & 1, abort_flag, true);
+                    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                }
+                for (int t = run(c), first = t; t < run(c + 1) && ok; ++t) {
+                    const int it = t - t0, gb = it & 1;
+                    if (!cu_wait(&gfull[gb], (it / 2) & 1, abort_flag, true)) {
+                        ok = false;
+                        break;
+                    }
+                    const uint64_t db = wg_desc<GN>(cu_smem(smG + gb * g_tile));
+                    for (int m = 0; m < mts; ++m, ++kc) {
+                        const int s = kc % WG_STAGES;
+                        if (!cu_wait(&full[s], (kc / WG_STAGES) & 1, abort_flag, true)) {
+                            ok = false;
+                            break;
+                        }
+                        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+                        const uint64_t da = wg_desc<GA>(cu_smem(sm + s * L::A_TILE));
+                        for (int k = 0; k < ksteps; ++k)   // 16 voxels: two 8-row groups
+                            cu_mma(tmem + m * p.nb, da + (uint64_t)(k * 16 * GA * 2 >> 4),
+                                   db + (uint64_t)(k * 16 * GN * 2 >> 4), idesc, (t > first || k) ? 1u : 0u);
+                        cu_commit(&empty[s]);
+                    }
+                    cu_commit(&gempty[gb]);
+                }
+                cu_commit(done);   // tracks every MMA issued above, also after an abort
+            }
+        }
+        __syncwarp();
+    } else {
+        const int q = warp & 3, r = 32 * q + lane;
+        const uint32_t trow = tmem + ((uint32_t)(32 * q) << 16);
+        for (int run_ = 0; run_ < p.runs; ++run_) {
+            const bool ok = cu_wait(done, run_ & 1, abort_flag, false) && !*abort_flag;
+            asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+            for (int m = 0; m < mts && ok; ++m) {
+                const int grp = (mt0 + m) * MG + r / GA;
+                const int tap = grp / cgroups, ci = (grp % cgroups) * GA + r % GA;
+#pragma unroll 1
+                for (int c = 0; c < p.nb; c += 16) {
+                    uint32_t v[16];
+                    cu_ld16(trow + m * p.nb + c, v);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+                    if (grp < p.groups) {
+#pragma unroll
+                        for (int j = 0; j < 16; ++j)
+                            atomicAdd(&dW[((long)(n0 + c + j) * p.taps + tap) * g.Cin + ci], __uint_as_float(v[j]));
+                    }
+                    __syncwarp();
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+            __syncwarp();
+            if (lane == 0)
+                asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(cu_smem(drained)) : "memory");
+        }
+    }
+
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    __syncthreads();
+    if (warp == 1) {
+        asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"((uint32_t)p.cols));
     }
     if (threadIdx.x == 0 && *abort_flag) atomicOr(&g_nn_status, 0x100);
 }
