@@ -66,6 +66,8 @@ def nnlib():
         L.pllnn_up_bwd.argtypes = [P, I, I, I, I, I, P, I, P]
         L.pllnn_cat_fwd.argtypes = [P, I, P, I, Lg, P, P]
         L.pllnn_cat_bwd.argtypes = [P, I, I, Lg, P, I, P, I, P]
+        L.pllnn_upcat_fwd.argtypes = [P, I, I, I, I, I, P, I, P, P]
+        L.pllnn_upcat_bwd.argtypes = [P, I, I, I, I, I, I, P, I, P, P]
         L.pllnn_mse.argtypes = [P, P, Lg, F, P, P, P]
         L.pllnn_adam.argtypes = [P, P, P, P, Lg, F, F, F, F, I, P, P, F, P]
         L.pllnn_sumsq.argtypes = [P, Lg, P, P]
@@ -181,10 +183,8 @@ class UNet:
             return y
 
         def upcat(x, s, C, skip, CS):
-            u = torch.empty((Vs[s - 1], C), dtype=torch.bfloat16, device=dev)
-            _ok(L.pllnn_up_fwd(_p(x), *vols[s], C, _p(u), st), "up")
             y = torch.empty((Vs[s - 1], C + CS), dtype=torch.bfloat16, device=dev)
-            _ok(L.pllnn_cat_fwd(_p(u), C, _p(skip), CS, Vs[s - 1], _p(y), st), "cat")
+            _ok(L.pllnn_upcat_fwd(_p(x), *vols[s], C, _p(skip), CS, _p(y), st), "up and cat")
             return y
 
         e1 = l["e1"].forward(x16, vols[0])
@@ -207,10 +207,8 @@ class UNet:
         def cat_up_bwd(gc, s, C, CS, gskip):
             """gc over (up(x) | skip) at level s-1 -> grad of x (level s);
             the skip's share goes into gskip (overwritten)."""
-            gu = torch.empty((Vs[s - 1], C), dtype=torch.float32, device=dev)
-            _ok(L.pllnn_cat_bwd(_p(gc), C, CS, Vs[s - 1], _p(gu), 0, _p(gskip), 0, st), "cat backward")
             gx = torch.empty((Vs[s], C), dtype=torch.float32, device=dev)
-            _ok(L.pllnn_up_bwd(_p(gu), *vols[s], C, _p(gx), 0, st), "up backward")
+            _ok(L.pllnn_upcat_bwd(_p(gc), *vols[s], C, CS, _p(gx), 0, _p(gskip), st), "up and cat backward")
             return gx
 
         def pool_bwd_acc(g, s, C, into):

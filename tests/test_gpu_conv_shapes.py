@@ -77,3 +77,52 @@ def test_weight_gradient(k, ci, co, vol):
     ref = nn_ref.conv_bwd(xf, wf, gf, k)[1] + start.double().numpy()
     mag = nn_ref.conv_bwd(np.abs(xf), wf, np.abs(gf), k)[1] + np.abs(start.numpy())
     assert np.all(np.abs(dw.cpu().numpy() - ref) <= _bound(int(np.prod(vol)), mag))
+
+
+# channel counts that go in 16-byte pieces and ones that go singly
+@pytest.mark.parametrize("ca,cb", [(16, 8), (64, 32), (12, 4), (5, 3), (8, 0)])
+def test_upsample_concatenate(ca, cb):
+    import torch
+
+    from pllcart3d_b200 import surrogate as S
+
+    L, st = S.nnlib(), S._stream()
+    vol = (2, 3, 2, 5)
+    fine = (2, 6, 4, 10)
+    rng = np.random.default_rng(ca * 10 + cb)
+    a, b = _bf16(rng.standard_normal(vol + (ca,))), _bf16(rng.standard_normal(fine + (cb,)))
+    ad, bd = a.cuda().contiguous(), b.cuda().contiguous()
+    y = torch.zeros(fine + (ca + cb,), dtype=torch.bfloat16, device="cuda")
+    assert L.pllnn_upcat_fwd(S._p(ad), *vol, ca, S._p(bd), cb, S._p(y), st) == 0
+    ref = np.concatenate([nn_ref.up(a.float().numpy()), b.float().numpy()], -1)
+    assert np.array_equal(y.float().cpu().numpy(), ref)
+    g = rng.standard_normal(fine + (ca + cb,)).astype(np.float32)
+    start = rng.standard_normal(vol + (ca,)).astype(np.float32)
+    gd, da = torch.tensor(g, device="cuda"), torch.tensor(start, device="cuda")
+    db = torch.zeros(fine + (cb,), dtype=torch.float32, device="cuda")
+    assert L.pllnn_upcat_bwd(S._p(gd), *vol, ca, cb, S._p(da), 1, S._p(db), st) == 0
+    assert np.array_equal(db.cpu().numpy(), g[..., ca:])
+    ref = start + nn_ref.up_bwd(g[..., :ca].astype(np.float64))
+    # eight FP32 additions of the children and one of the start value
+    assert np.all(np.abs(da.cpu().numpy() - ref) <= 9 * 2.0 ** -24 * (np.abs(start) + nn_ref.up_bwd(np.abs(g[..., :ca]))))
+
+
+@pytest.mark.parametrize("c", [16, 6, 1])
+def test_pooling(c):
+    import torch
+
+    from pllcart3d_b200 import surrogate as S
+
+    L, st = S.nnlib(), S._stream()
+    rng = np.random.default_rng(c)
+    x = _bf16(rng.standard_normal((2, 4, 6, 2, c)))
+    xd = x.cuda().contiguous()
+    y = torch.zeros((2, 2, 3, 1, c), dtype=torch.bfloat16, device="cuda")
+    assert L.pllnn_pool_fwd(S._p(xd), 2, 4, 6, 2, c, S._p(y), st) == 0
+    ref = nn_ref.pool(x.double().numpy())
+    # BF16 rounding of an FP32 mean
+    assert np.all(np.abs(y.double().cpu().numpy() - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-6)
+    g = rng.standard_normal((2, 2, 3, 1, c)).astype(np.float32)
+    gd, dx = torch.tensor(g, device="cuda"), torch.zeros((2, 4, 6, 2, c), dtype=torch.float32, device="cuda")
+    assert L.pllnn_pool_bwd(S._p(gd), 2, 4, 6, 2, c, S._p(dx), 0, st) == 0
+    assert np.array_equal(dx.cpu().numpy(), nn_ref.pool_bwd(g).astype(np.float32))
