@@ -76,6 +76,14 @@ struct Consts {
     double Re;
     double area;                  // (Y2-Y1)*(Z2-Z1)
     double dx2i;                  // 1/(dx*dx) (phisolver_dct)
+    // products of the above for the forms that contract (operands straight
+    // from the parameter bank)
+    double hix, hiy, hiz;         // 0.5 / h
+    double qix, qiy, qiz;         // 0.25 / h
+    double e1x, e1y, e1z;         // 1/(Re h^2)
+    double e2x, e2y, e2z;         // 2/(Re h^2)
+    double iRe;                   // 1/Re
+    double wfx, wfy, wfz;         // 4e-99 h^2: WENO5 weight floor on undivided differences
     double CFLmax;
     double M, Vnorm;
 };

@@ -12,9 +12,10 @@
 // resident while plane i+2 is in flight.  Values read only along x at the
 // thread's own (j, k) -- the x WENO5 window q(i-3 .. i+3), the x-face
 // viscosity and velocity, c, pg, H_old -- stay in registers, one plain
-// coalesced load per plane.  Every formula, closure and the stale-D2 hazard
-// are k_explicit's; only where each operand comes from differs (results agree
-// to rounding with the same arithmetic type and contraction flags).
+// coalesced load per plane.  Closures and the stale-D2 hazard are
+// k_explicit's, and so are the formulas in other words: differences undivided,
+// the stencils read in the upwind direction, WENO5 as the central difference
+// plus one weighted correction (weno_corr), stresses as fluxes.
 // TMA boxes start on 16-byte boundaries: the k tiles start at k0 = 1 + 32 b,
 // so the +-1 box starts at k0-1 (a multiple of 32 elements) and the q box at
 // k0-3 (FP64: a multiple of 2) or k0-5 (FP32: a multiple of 4).  No
@@ -26,6 +27,7 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <type_traits>
 
 #include "step_kernels.cuh"
 
@@ -105,48 +107,98 @@ __device__ __noinline__ bool xt_wait(uint64_t* b, uint32_t parity)
     return true;
 }
 
-// upwind derivative along one axis from the 7 values q(m-3 .. m+3) of the
-// line (v[3] is the point itself), the ENO-2 closure on the first and last
-// two points of the range (stale-D2 values from global memory), WENO5
-// elsewhere -- upwind_deriv's arithmetic
+// the type that evaluates the WENO5 weights of a state in `real`
+template <typename real>
+struct XtWeno {
+    using type = real;
+};
+#if PLL_WENO_F32
+template <>
+struct XtWeno<double> {
+    using type = float;
+};
+#endif
+
+// the ENO-2 closure's correction (the first and last two points of a range):
+// half the smaller of the two second differences, b behind and c ahead of the
+// point in the upwind sense; ties go to the lower line index, b for up
+template <typename real>
+__device__ __forceinline__ real eno_corr(real b, real c, bool up)
+{
+    const bool first = up ? fabs(b) <= fabs(c) : !(fabs(c) <= fabs(b));
+    return (real)0.5 * (first ? b : c);
+}
+
+// b of the closure where it lies outside the range: what an earlier pass of
+// the routine left in its scratch line, in undivided differences of this axis
 template <int AXIS, typename real>
-__device__ __forceinline__ real xt_upwind(const real* v, const real* __restrict__ qg, const Geo& G, const Rng& R,
-                                          const Consts& K, int m, real vv)
+__device__ __forceinline__ real eno_behind(const real* __restrict__ qg, const Geo& G, const Rng& R, const Consts& K,
+                                           int m, bool up, real b)
 {
     const int s = AXIS == 0 ? R.is : AXIS == 1 ? R.js : R.ks;
     const int e = AXIS == 0 ? R.ie : AXIS == 1 ? R.je : R.ke;
     const double h = AXIS == 0 ? K.hx : AXIS == 1 ? K.hy : K.hz;
-    const double ih = AXIS == 0 ? K.ihx : AXIS == 1 ? K.ihy : K.ihz;
-    const double i2h = AXIS == 0 ? K.i2hx : AXIS == 1 ? K.i2hy : K.i2hz;
-    const int sign = (vv >= (real)0) ? 1 : -1;
-    if ((m <= s + 1) | (m >= e - 1)) {
-        const bool up = sign == 1;
-        const int kk = up ? m - 1 : m;
-        // q(kk-1), q(kk), q(kk+1), q(kk+2): v[1..4] upwind from the left,
-        // v[2..5] from the right (selected, so that v stays in registers)
-        const real wm = up ? v[1] : v[2], w0 = up ? v[2] : v[3], w1 = up ? v[3] : v[4], w2 = up ? v[4] : v[5];
-        real d1k = over_h<real>(w1 - w0, h, ih, K.pow2);
-        real d2a, d2b;
-        if (kk >= s) {
-            real d1m = over_h<real>(w0 - wm, h, ih, K.pow2);
-            d2a = over_2h<real>(d1k - d1m, h, i2h, K.pow2);
-        } else {
-            d2a = stale_d2<real>(qg, G, R, K, AXIS, kk);
-        }
-        if (kk + 1 <= e) {
-            real d1p = over_h<real>(w2 - w1, h, ih, K.pow2);
-            d2b = over_2h<real>(d1p - d1k, h, i2h, K.pow2);
-        } else {
-            d2b = stale_d2<real>(qg, G, R, K, AXIS, kk + 1);
-        }
-        real d2v = (fabs(d2a) <= fabs(d2b)) ? d2a : d2b;
-        return d1k + d2v * (real)h * (real)sign;
+    if (up ? m == s : m == e) return stale_d2<real>(qg, G, R, K, AXIS, up ? s - 1 : e + 1) * (real)(2.0 * h * h);
+    return b;
+}
+
+template <int AXIS>
+__device__ __forceinline__ bool eno_band(const Rng& R, int m)
+{
+    const int s = AXIS == 0 ? R.is : AXIS == 1 ? R.js : R.ks;
+    const int e = AXIS == 0 ? R.ie : AXIS == 1 ? R.je : R.ke;
+    return (m <= s + 1) | (m >= e - 1);
+}
+
+// WENO5 correction in the form's weight type
+template <typename real>
+__device__ __forceinline__ real xt_weno(real v0, real v1, real v2, real v3, real v4, real a, real b, real c, real d,
+                                        real floor4)
+{
+    if constexpr (std::is_same<typename XtWeno<real>::type, float>::value) {
+        return (real)weno_corr((float)v2, (float)a, (float)b, (float)c, (float)d);
+    } else {
+        const real vmax = fmax(fmax(fmax(fabs(v0), fabs(v1)), fmax(fabs(v2), fabs(v3))), fabs(v4));
+        return weno_corr(a, b, c, d, vmax, floor4);
     }
-    real d[6];
+}
+
+// h x |upwind derivative| sense along y or z: p is the point in its shared
+// tile, st the tile's step along the axis.  The window is read in the upwind
+// direction (up: increasing), so that neither the differences nor anything
+// made of them is selected by the sign; the derivative times the velocity is
+// |velocity| / h times the result.  c2: the second difference at the point.
+template <int AXIS, typename real>
+__device__ __forceinline__ real xt_upwind(const real* p, int st, const real* __restrict__ qg, const Geo& G,
+                                          const Rng& R, const Consts& K, int m, bool up, real floor4, real& c2)
+{
+    const int s = up ? st : -st;
+    const real* w = p - 3 * s;
+    real d[5];
+    real q0 = w[0];
 #pragma unroll
-    for (int t = 0; t < 6; ++t) d[t] = over_h<real>(v[t + 1] - v[t], h, ih, K.pow2);
-    const bool up = sign == 1;
-    return weno5<real>(up ? d[0] : d[5], up ? d[1] : d[4], up ? d[2] : d[3], up ? d[3] : d[2], up ? d[4] : d[1]);
+    for (int t = 0; t < 5; ++t) {
+        const real q1 = w[(t + 1) * s];
+        d[t] = q1 - q0;
+        q0 = q1;
+    }
+    const real b = d[2] - d[1], c = d[3] - d[2];
+    c2 = c;
+    if (eno_band<AXIS>(R, m)) return d[2] + eno_corr<real>(eno_behind<AXIS, real>(qg, G, R, K, m, up, b), c, up);
+    return d[2] + xt_weno<real>(d[0], d[1], d[2], d[3], d[4], d[1] - d[0], b, c, d[4] - d[3], floor4);
+}
+
+// the same along x from the register window D[t] = q(i-2+t) - q(i-3+t)
+template <typename real>
+__device__ __forceinline__ real xt_upwind_x(const real* D, const real* __restrict__ qg, const Geo& G, const Rng& R,
+                                            const Consts& K, int i, bool up, real floor4, real& c2)
+{
+    const real v2 = up ? D[2] : -D[3], c = D[3] - D[2];
+    const real b = (up ? D[2] : D[4]) - (up ? D[1] : D[3]);
+    c2 = c;
+    if (eno_band<0>(R, i)) return v2 + eno_corr<real>(eno_behind<0, real>(qg, G, R, K, i, up, b), c, up);
+    const real a = (up ? D[1] : D[5]) - (up ? D[0] : D[4]), d = (up ? D[4] : D[2]) - (up ? D[3] : D[1]);
+    return v2 + xt_weno<real>(up ? D[0] : D[5], D[1], D[2], D[3], D[4], a, b, c, d, floor4);
 }
 
 template <int VAR, typename real>
@@ -199,9 +251,16 @@ __global__ void __launch_bounds__(XT_THREADS) k_explicit_tma(const __grid_consta
     // register windows along x at (j, k)
     const long col = (long)j * sy + k;
     const real* __restrict__ q = A.q;
-    real qx[7];
+    real D[6], ql;   // differences of q(i-3 .. i+3), and q(i+3)
+    {
+        real q0 = live ? q[(long)(i0 - 3) * sx + col] : (real)0;
 #pragma unroll
-    for (int t = 0; t < 7; ++t) qx[t] = live ? q[(long)(i0 - 3 + t) * sx + col] : (real)0;
+        for (int t = 0; t < 6; ++t) {
+            ql = live ? q[(long)(i0 - 2 + t) * sx + col] : (real)0;
+            D[t] = ql - q0;
+            q0 = ql;
+        }
+    }
     real xa0 = 0, xa1 = 0, xb0 = 0, xb1 = 0;   // VC: u(i), u(i+1); VU: mu_cell(i-1), (i), c(i-1), c(i);
                                                // VV: mu_xy(i), (i+1); VW: mu_xz(i), (i+1)
     const real* __restrict__ xa = VAR == VC ? A.un : VAR == VU ? A.mu.cell : VAR == VV ? A.mu.xy : A.mu.xz;
@@ -260,136 +319,86 @@ __global__ void __launch_bounds__(XT_THREADS) k_explicit_tma(const __grid_consta
                 return tile1(i + dp, a)[o1 + dj * KB1 + dk];
             };
             auto QT = [&](int dj, int dk) -> real { return Q[o3 + dj * KB3 + dk]; };
-            const real hf = (real)0.5, qr = (real)0.25;
-            // advecting velocities (adv_vel)
+            // advecting velocities (adv_vel), up to their factor of 1/2 or 1/4
+            const real q0 = QT(0, 0);
             real ux, uy, uz;
             if (VAR == VC) {
-                ux = hf * (xa1 + xa0);
-                uy = hf * (T(0, 0, 1, 0) + T(0, 0, 0, 0));
-                uz = hf * (T(1, 0, 0, 1) + T(1, 0, 0, 0));
+                ux = xa1 + xa0;
+                uy = T(0, 0, 1, 0) + T(0, 0, 0, 0);
+                uz = T(1, 0, 0, 1) + T(1, 0, 0, 0);
             } else if (VAR == VU) {
-                ux = qx[3];
-                uy = qr * (T(0, -1, 0, 0) + T(0, 0, 0, 0) + T(0, 0, 1, 0) + T(0, -1, 1, 0));
-                uz = qr * (T(1, -1, 0, 0) + T(1, 0, 0, 0) + T(1, 0, 0, 1) + T(1, -1, 0, 1));
+                ux = q0;
+                uy = T(0, -1, 0, 0) + T(0, 0, 0, 0) + T(0, 0, 1, 0) + T(0, -1, 1, 0);
+                uz = T(1, -1, 0, 0) + T(1, 0, 0, 0) + T(1, 0, 0, 1) + T(1, -1, 0, 1);
             } else if (VAR == VV) {
-                ux = qr * (T(0, 0, -1, 0) + T(0, 1, -1, 0) + T(0, 0, 0, 0) + T(0, 1, 0, 0));
-                uy = qx[3];
-                uz = qr * (T(1, 0, -1, 0) + T(1, 0, -1, 1) + T(1, 0, 0, 0) + T(1, 0, 0, 1));
+                ux = T(0, 0, -1, 0) + T(0, 1, -1, 0) + T(0, 0, 0, 0) + T(0, 1, 0, 0);
+                uy = q0;
+                uz = T(1, 0, -1, 0) + T(1, 0, -1, 1) + T(1, 0, 0, 0) + T(1, 0, 0, 1);
             } else {
-                ux = qr * (T(0, 0, 0, -1) + T(0, 1, 0, -1) + T(0, 0, 0, 0) + T(0, 1, 0, 0));
-                uy = qr * (T(1, 0, 0, -1) + T(1, 0, 0, 0) + T(1, 0, 1, -1) + T(1, 0, 1, 0));
-                uz = qx[3];
+                ux = T(0, 0, 0, -1) + T(0, 1, 0, -1) + T(0, 0, 0, 0) + T(0, 1, 0, 0);
+                uy = T(1, 0, 0, -1) + T(1, 0, 0, 0) + T(1, 0, 1, -1) + T(1, 0, 1, 0);
+                uz = q0;
             }
-            // one stencil window at a time (y, then z) keeps register use low
-            const real cx = ux * xt_upwind<0, real>(qx, q, G, R, K, i, ux);
-            real cy, cz, qym, qyp, qzm, qzp;
-            {
-                real vy[7];
-#pragma unroll
-                for (int t = 0; t < 7; ++t) vy[t] = QT(t - 3, 0);
-                cy = uy * xt_upwind<1, real>(vy, q, G, R, K, j, uy);
-                qym = vy[2];
-                qyp = vy[4];
-            }
-            {
-                real vz[7];
-#pragma unroll
-                for (int t = 0; t < 7; ++t) vz[t] = QT(0, t - 3);
-                cz = uz * xt_upwind<2, real>(vz, q, G, R, K, k, uz);
-                qzm = vz[2];
-                qzp = vz[4];
-            }
-            const real ct = cz + cx + cy;
-            real H;
+            const real fx = (real)(VAR == VC ? K.hix : VAR == VU ? K.ihx : K.qix);
+            const real fy = (real)(VAR == VC ? K.hiy : VAR == VV ? K.ihy : K.qiy);
+            const real fz = (real)(VAR == VC ? K.hiz : VAR == VW ? K.ihz : K.qiz);
+            // velocity x upwind derivative = |velocity| / h x the upwind-sense
+            // difference; one axis at a time keeps register use low
+            real c2x, c2y, c2z;
+            real ct = fabs(ux) * fx * xt_upwind_x<real>(D, q, G, R, K, i, ux >= (real)0, (real)K.wfx, c2x);
+            ct = fma(fabs(uy) * fy, xt_upwind<1, real>(Q + o3, KB3, q, G, R, K, j, uy >= (real)0, (real)K.wfy, c2y), ct);
+            ct = fma(fabs(uz) * fz, xt_upwind<2, real>(Q + o3, 1, q, G, R, K, k, uz >= (real)0, (real)K.wfz, c2z), ct);
+            // cross stress, and the implicit operator on q_old (acoef) as
+            // fluxes: c (q+ - q) - a (q - q-)
+            real H = -ct, diff;
             if (VAR == VC) {
-                H = -(ct);
+                diff = fma((real)K.cdx, c2x, fma((real)K.cdy, c2y, (real)K.cdz * c2z));
             } else {
-                real s1, s2, s3, s4;
+                const real yp = QT(1, 0) - q0, ym = q0 - QT(-1, 0), zp = QT(0, 1) - q0, zm = q0 - QT(0, -1);
                 if (VAR == VU) {   // tiles: 0 v, 1 w, 2 mu_xy, 3 mu_xz
-                    s1 = (real)K.xuv * T(2, 0, 1, 0) * (T(0, 0, 1, 0) - T(0, -1, 1, 0));
-                    s2 = (real)K.xuv * T(2, 0, 0, 0) * (T(0, 0, 0, 0) - T(0, -1, 0, 0));
-                    s3 = (real)K.xuw * T(3, 0, 0, 1) * (T(1, 0, 0, 1) - T(1, -1, 0, 1));
-                    s4 = (real)K.xuw * T(3, 0, 0, 0) * (T(1, 0, 0, 0) - T(1, -1, 0, 0));
+                    const real my = T(2, 0, 0, 0), my1 = T(2, 0, 1, 0), mz = T(3, 0, 0, 0), mz1 = T(3, 0, 0, 1);
+                    H = fma((real)K.xuv, fma(my1, T(0, 0, 1, 0) - T(0, -1, 1, 0), -my * (T(0, 0, 0, 0) - T(0, -1, 0, 0))),
+                            H);
+                    H = fma((real)K.xuw, fma(mz1, T(1, 0, 0, 1) - T(1, -1, 0, 1), -mz * (T(1, 0, 0, 0) - T(1, -1, 0, 0))),
+                            H);
+                    diff = (real)K.e2x * fma(xa1, D[3], -xa0 * D[2]);
+                    diff = fma((real)K.e1y, fma(my1, yp, -my * ym), diff);
+                    diff = fma((real)K.e1z, fma(mz1, zp, -mz * zm), diff);
                 } else if (VAR == VV) {   // tiles: 0 u, 1 w, 2 mu_yz, 3 mu_cell, 4 c
-                    s1 = (real)K.xvu * xa1 * (T(0, 1, 0, 0) - T(0, 1, -1, 0));
-                    s2 = (real)K.xvu * xa0 * (T(0, 0, 0, 0) - T(0, 0, -1, 0));
-                    s3 = (real)K.xvw * T(2, 0, 0, 1) * (T(1, 0, 0, 1) - T(1, 0, -1, 1));
-                    s4 = (real)K.xvw * T(2, 0, 0, 0) * (T(1, 0, 0, 0) - T(1, 0, -1, 0));
+                    const real mz = T(2, 0, 0, 0), mz1 = T(2, 0, 0, 1);
+                    H = fma((real)K.xvu, fma(xa1, T(0, 1, 0, 0) - T(0, 1, -1, 0), -xa0 * (T(0, 0, 0, 0) - T(0, 0, -1, 0))),
+                            H);
+                    H = fma((real)K.xvw, fma(mz1, T(1, 0, 0, 1) - T(1, 0, -1, 1), -mz * (T(1, 0, 0, 0) - T(1, 0, -1, 0))),
+                            H);
+                    diff = (real)K.e1x * fma(xa1, D[3], -xa0 * D[2]);
+                    diff = fma((real)K.e2y, fma(T(3, 0, 0, 0), yp, -T(3, 0, -1, 0) * ym), diff);
+                    diff = fma((real)K.e1z, fma(mz1, zp, -mz * zm), diff);
                 } else {   // tiles: 0 u, 1 v, 2 mu_yz, 3 mu_cell
-                    s1 = (real)K.xwu * xa1 * (T(0, 1, 0, 0) - T(0, 1, 0, -1));
-                    s2 = (real)K.xwu * xa0 * (T(0, 0, 0, 0) - T(0, 0, 0, -1));
-                    s3 = (real)K.xwv * T(2, 0, 1, 0) * (T(1, 0, 1, 0) - T(1, 0, 1, -1));
-                    s4 = (real)K.xwv * T(2, 0, 0, 0) * (T(1, 0, 0, 0) - T(1, 0, 0, -1));
+                    const real my = T(2, 0, 0, 0), my1 = T(2, 0, 1, 0);
+                    H = fma((real)K.xwu, fma(xa1, T(0, 1, 0, 0) - T(0, 1, 0, -1), -xa0 * (T(0, 0, 0, 0) - T(0, 0, 0, -1))),
+                            H);
+                    H = fma((real)K.xwv, fma(my1, T(1, 0, 1, 0) - T(1, 0, 1, -1), -my * (T(1, 0, 0, 0) - T(1, 0, 0, -1))),
+                            H);
+                    diff = (real)K.e1x * fma(xa1, D[3], -xa0 * D[2]);
+                    diff = fma((real)K.e1y, fma(my1, yp, -my * ym), diff);
+                    diff = fma((real)K.e2z, fma(T(3, 0, 0, 0), zp, -T(3, 0, 0, -1) * zm), diff);
                 }
-                H = -ct + s1 - s2 + s3 - s4;
             }
             A.H[id] = H;
 
-            // dt*(gamma H + rho H_old + alpha A q_old + alpha body) (acoef)
-            const real conv = rk_comb<real>((real)A.g, H, (real)A.r, hmv);
-            real a, c;
-            if (VAR == VC) {
-                a = c = (real)K.cdx;
-            } else if (VAR == VU) {
-                a = over_h<real>((real)K.d2x * xa0, K.hx, K.ihx, K.pow2);
-                c = over_h<real>((real)K.d2x * xa1, K.hx, K.ihx, K.pow2);
-            } else {
-                a = over_h<real>((real)K.d1x * xa0, K.hx, K.ihx, K.pow2);
-                c = over_h<real>((real)K.d1x * xa1, K.hx, K.ihx, K.pow2);
+            // dt*(gamma H + rho H_old + alpha (A q_old + body))
+            if (VAR != VC) {
+                diff = fma(-pgv, (real)K.iRe, diff);
+                if (VAR == VU) diff = fma((real)K.FxRe, (real)0.5 * (xb1 + xb0), diff);
+                if (VAR == VV) diff = fma((real)K.FyRe, (real)0.5 * (T(4, 0, 0, 0) + T(4, 0, -1, 0)), diff);
             }
-            real b = -(a + c);
-            const real ax = a * qx[2] + b * qx[3] + c * qx[4];
-            if (VAR == VC) {
-                a = c = (real)K.cdy;
-            } else if (VAR == VU) {
-                a = over_h<real>((real)K.d1y * T(2, 0, 0, 0), K.hy, K.ihy, K.pow2);
-                c = over_h<real>((real)K.d1y * T(2, 0, 1, 0), K.hy, K.ihy, K.pow2);
-            } else if (VAR == VV) {
-                a = over_h<real>((real)K.d2y * T(3, 0, -1, 0), K.hy, K.ihy, K.pow2);
-                c = over_h<real>((real)K.d2y * T(3, 0, 0, 0), K.hy, K.ihy, K.pow2);
-            } else {
-                a = over_h<real>((real)K.d1y * T(2, 0, 0, 0), K.hy, K.ihy, K.pow2);
-                c = over_h<real>((real)K.d1y * T(2, 0, 1, 0), K.hy, K.ihy, K.pow2);
-            }
-            b = -(a + c);
-            const real ay = a * qym + b * qx[3] + c * qyp;
-            if (VAR == VC) {
-                a = c = (real)K.cdz;
-            } else if (VAR == VU) {
-                a = over_h<real>((real)K.d1z * T(3, 0, 0, 0), K.hz, K.ihz, K.pow2);
-                c = over_h<real>((real)K.d1z * T(3, 0, 0, 1), K.hz, K.ihz, K.pow2);
-            } else if (VAR == VV) {
-                a = over_h<real>((real)K.d1z * T(2, 0, 0, 0), K.hz, K.ihz, K.pow2);
-                c = over_h<real>((real)K.d1z * T(2, 0, 0, 1), K.hz, K.ihz, K.pow2);
-            } else {
-                a = over_h<real>((real)K.d2z * T(3, 0, 0, -1), K.hz, K.ihz, K.pow2);
-                c = over_h<real>((real)K.d2z * T(3, 0, 0, 0), K.hz, K.ihz, K.pow2);
-            }
-            b = -(a + c);
-            const real az = a * qzm + b * qx[3] + c * qzp;
-            const real diff = alpha * (ax + ay + az);
-            real S;
-            if (VAR == VC) {
-                S = dt * (conv + diff);
-            } else {
-                real bf;
-                if (VAR == VU) {
-                    const real cval = (real)0.5 * (xb1 + xb0);
-                    bf = alpha * ((real)K.FxRe * cval - over_h<real>(pgv, K.Re, 1.0 / K.Re, 0));
-                } else if (VAR == VV) {
-                    const real cval = (real)0.5 * (T(4, 0, 0, 0) + T(4, 0, -1, 0));
-                    bf = alpha * ((real)K.FyRe * cval - over_h<real>(pgv, K.Re, 1.0 / K.Re, 0));
-                } else {
-                    bf = alpha * (-over_h<real>(pgv, K.Re, 1.0 / K.Re, 0));
-                }
-                S = dt * (conv + diff + bf);
-            }
-            A.S[id] = S;
+            A.S[id] = dt * fma(alpha, diff, rk_comb<real>((real)A.g, H, (real)A.r, hmv));
         }
         // slide the windows one plane along x
 #pragma unroll
-        for (int t = 0; t < 6; ++t) qx[t] = qx[t + 1];
-        qx[6] = qn;
+        for (int t = 0; t < 5; ++t) D[t] = D[t + 1];
+        D[5] = qn - ql;
+        ql = qn;
         xa0 = xa1;
         xa1 = xan;
         if (VAR == VU) {

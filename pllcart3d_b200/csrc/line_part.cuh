@@ -30,26 +30,6 @@ __device__ __forceinline__ void lp_cp16(void* dst, const void* src)
                  : "memory");
 }
 
-// 1/x of the partitioned solves, whose pivots are normal numbers (>= 1 in
-// magnitude in the diagonally dominant ADI systems).  FP32: approximate, <= 2
-// ulp.  FP64: the hardware's seed and one third-order step of Newton's
-// iteration (y (1 + e + e^2), e = 1 - x y), within an ulp of the IEEE quotient
-// in 4 instructions: the solves do a third of their arithmetic in it (IEEE
-// division measured 8 % slower per launch: x 256 rows 30.5 -> 27.8 us at
-// 256x128x128, z 157 -> 137 us at 512x256x256).
-template <typename real>
-__device__ __forceinline__ real rcp_(real x);
-template <>
-__device__ __forceinline__ double rcp_<double>(double x)
-{
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-    const double e = fma(-x, y, 1.0);
-    return fma(y, fma(e, e, e), y);
-}
-template <>
-__device__ __forceinline__ float rcp_<float>(float x) { return __fdividef(1.0f, x); }
-
 // couplings below this are dropped: far below the rounding of anything they
 // could still multiply
 template <typename real>

@@ -224,6 +224,12 @@ pllgpu_ctx* pllgpu_create(const pllgpu_params* p, int device)
     K.Re = Re;
     K.area = (p->Y2 - p->Y1) * (p->Z2 - p->Z1);
     K.dx2i = 1.0 / (G.dx * G.dx);
+    K.hix = 0.5 * K.ihx; K.hiy = 0.5 * K.ihy; K.hiz = 0.5 * K.ihz;
+    K.qix = 0.25 * K.ihx; K.qiy = 0.25 * K.ihy; K.qiz = 0.25 * K.ihz;
+    K.e1x = K.d1x * K.ihx; K.e1y = K.d1y * K.ihy; K.e1z = K.d1z * K.ihz;
+    K.e2x = K.d2x * K.ihx; K.e2y = K.d2y * K.ihy; K.e2z = K.d2z * K.ihz;
+    K.iRe = 1.0 / Re;
+    K.wfx = 4.0e-99 * G.dx * G.dx; K.wfy = 4.0e-99 * G.dy * G.dy; K.wfz = 4.0e-99 * G.dz * G.dz;
     K.CFLmax = p->CFLmax;
     K.M = p->Vratio;
     K.Vnorm = 0.0;

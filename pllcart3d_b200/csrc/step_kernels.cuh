@@ -237,6 +237,78 @@ __device__ __forceinline__ double weno5<double>(double v0, double v1, double v2,
 }
 #endif
 
+// 1/x for a normal number x (the pivots of the partitioned line solves, >= 1 in
+// magnitude in the diagonally dominant ADI systems; the WENO5 weight sums).
+// FP32: approximate, <= 2 ulp.  FP64: the hardware's seed and one third-order
+// step of Newton's iteration (y (1 + e + e^2), e = 1 - x y), within an ulp of
+// the IEEE quotient in 4 instructions: the solves do a third of their
+// arithmetic in it (IEEE division measured 8 % slower per launch: x 256 rows
+// 30.5 -> 27.8 us at 256x128x128, z 157 -> 137 us at 512x256x256).
+template <typename real>
+__device__ __forceinline__ real rcp_(real x);
+template <>
+__device__ __forceinline__ double rcp_<double>(double x)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    const double e = fma(-x, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+template <>
+__device__ __forceinline__ float rcp_<float>(float x) { return __fdividef(1.0f, x); }
+
+// The WENO5 derivative in undivided differences, taken in the upwind sense:
+// v0 .. v4 the five differences (v2 the one behind the point), a, b, c, d
+// their own differences (a = v1 - v0, ...).  The candidates are v2 plus
+// (5b-2a)/6, (b+2c)/6 and (4c-d)/6, the smoothness indicators (times 4)
+// 13/3 (b-a)^2 + (3b-a)^2, 13/3 (c-b)^2 + (b+c)^2 and 13/3 (d-c)^2 + (d-3c)^2
+// (calculate_weno, pllcart3d.c:3455-3507, expanded about v2), so the
+// derivative is v2 plus the weighted correction returned here, over h.  The
+// weights w_i / e_i^2 are multiplied by (e_1 e_2 e_3)^2: one division.  The
+// e_i are first brought to [1.5e-8, 2) by subtracting the largest one's
+// exponent from all three (eps >= 1e-6 max(v^2) and s_i <= 33 max(v^2) bound
+// their ratio), so that no product leaves the range.
+// vmax: max |v_i|; floor4: 4 x the reference's 1e-99 h^2 (FP32: 4e-36).
+__device__ __forceinline__ double weno_corr(double a, double b, double c, double d, double vmax, double floor4)
+{
+    const double eps = fma(4.0e-6 * vmax, vmax, floor4);
+    const double k = 13.0 / 3.0;
+    const double p1 = b - a, q1 = fma(3.0, b, -a), p2 = c - b, q2 = b + c, p3 = d - c, q3 = fma(-3.0, c, d);
+    double e1 = fma(k * p1, p1, fma(q1, q1, eps));
+    double e2 = fma(k * p2, p2, fma(q2, q2, eps));
+    double e3 = fma(k * p3, p3, fma(q3, q3, eps));
+    const int h1 = __double2hiint(e1), h2 = __double2hiint(e2), h3 = __double2hiint(e3);
+    const int sh = 0x3ff00000 - (max(max(h1, h2), h3) & 0x7ff00000);
+    e1 = __hiloint2double(h1 + sh, __double2loint(e1));
+    e2 = __hiloint2double(h2 + sh, __double2loint(e2));
+    e3 = __hiloint2double(h3 + sh, __double2loint(e3));
+    const double r23 = e2 * e3, r13 = e1 * e3, r12 = e1 * e2;
+    const double w1 = r23 * r23, w2 = 6.0 * (r13 * r13), w3 = 3.0 * (r12 * r12);
+    const double num = fma(w3, fma(4.0, c, -d), fma(w2, fma(2.0, c, b), w1 * fma(5.0, b, -2.0 * a)));
+    return num * rcp_<double>(6.0 * (w1 + w2 + w3));
+}
+
+// the same in FP32 from the correction's own differences; the v_i are
+// re-formed from v2 (their rounding only enters eps)
+__device__ __forceinline__ float weno_corr(float v2, float a, float b, float c, float d)
+{
+    const float v1 = v2 - b, v0 = v1 - a, v3 = v2 + c, v4 = v3 + d;
+    const float vmax = fmaxf(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))), fabsf(v4));
+    const float eps = fmaf(4.0e-6f * vmax, vmax, 4.0e-36f);
+    const float k = (float)(13.0 / 3.0);
+    const float p1 = b - a, q1 = fmaf(3.0f, b, -a), p2 = c - b, q2 = b + c, p3 = d - c, q3 = fmaf(-3.0f, c, d);
+    const float e1 = fmaf(k * p1, p1, fmaf(q1, q1, eps));
+    const float e2 = fmaf(k * p2, p2, fmaf(q2, q2, eps));
+    const float e3 = fmaf(k * p3, p3, fmaf(q3, q3, eps));
+    const int h1 = __float_as_int(e1), h2 = __float_as_int(e2), h3 = __float_as_int(e3);
+    const int sh = 0x3f800000 - (max(max(h1, h2), h3) & 0x7f800000);
+    const float s1 = __int_as_float(h1 + sh), s2 = __int_as_float(h2 + sh), s3 = __int_as_float(h3 + sh);
+    const float r23 = s2 * s3, r13 = s1 * s3, r12 = s1 * s2;
+    const float w1 = r23 * r23, w2 = 6.0f * (r13 * r13), w3 = 3.0f * (r12 * r12);
+    const float num = fmaf(w3, fmaf(4.0f, c, -d), fmaf(w2, fmaf(2.0f, c, b), w1 * fmaf(5.0f, b, -2.0f * a)));
+    return __fdividef(num, 6.0f * (w1 + w2 + w3));
+}
+
 // D2 value an earlier directional pass of the same H*_op call left in its
 // scratch line at index m (pllcart3d.c:1545-1546: D1/D2 are allocated once
 // per call, zeroed, and reused by the x, y and z passes; each pass writes
