@@ -40,6 +40,15 @@ constexpr int XT_NS = 4;    // plane slots of the ring
 constexpr int XT_THREADS = XT_TK * XT_TJ;
 constexpr long long XT_WAIT_CYCLES = 2000000000LL;   // ~1 s of SM clock
 
+// blocks per SM asked of the compiler.  With FP32 weights v and w fit three
+// (80 registers, 12-20 bytes spilled): 0.92 -> 0.87 and 0.87 -> 0.81 ms per
+// launch at 512x256x256.  u (0.76 -> 0.87) and the FP64 weights (0.13 -> 0.18
+// at 256x128x128) spill more and lose; c has three by itself (0: no demand).
+template <int VAR, typename real>
+struct XtBlocks {
+    static constexpr int value = PLL_WENO_F32 && sizeof(real) == 8 && VAR >= VV ? 3 : 0;
+};
+
 // fields staged with a +-1 halo, per variable (the ones read at a j or k
 // offset besides q); order fixes the slot layout
 //   VC: v, w            VU: v, w, mu_xy, mu_xz
@@ -202,7 +211,7 @@ __device__ __forceinline__ real xt_upwind_x(const real* D, const real* __restric
 }
 
 template <int VAR, typename real>
-__global__ void __launch_bounds__(XT_THREADS) k_explicit_tma(const __grid_constant__ XtMaps maps, Geo G, Rng R,
+__global__ void __launch_bounds__(XT_THREADS, XtBlocks<VAR, real>::value) k_explicit_tma(const __grid_constant__ XtMaps maps, Geo G, Rng R,
                                                              Consts K, ExplicitArgs<real> A, int ni, int* status)
 {
     using GM = XtGeom<real>;
