@@ -159,6 +159,43 @@ struct k_viscosity2_b {
     static constexpr int maxt = 128, minb = 0;
 };
 
+// Last-block ticket: every block's results are written and fenced before it
+// takes a ticket; the block that takes the last of `total` reads them all and
+// resets the counter for the next launch.
+__device__ __forceinline__ bool last_block(unsigned* ticket, unsigned total)
+{
+    __shared__ bool is_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && threadIdx.y == 0) is_last = atomicAdd(ticket, 1u) == total - 1;
+    __syncthreads();
+    if (is_last) __threadfence();
+    return is_last;
+}
+
+// dt = min(CFLmax / max, Timestep), pllcart3d.c:159-160, 3115, from the
+// finished scan, whose slot it clears for the next step; and the simulated
+// time, tval += (gamma + rho) dt per substep (L166; a0 = a1 = a2 = 0 outside a
+// step).  By one thread of the scan's last block.
+struct StepTime {
+    double a0, a1, a2;
+};
+__device__ __forceinline__ void step_dt(const Consts& K, double* scal, unsigned* ticket, const StepTime& a)
+{
+    const double maxall = __longlong_as_double((long long)__ldcg((unsigned long long*)(scal + S_CFLMAX)));
+    const double cfldt = K.CFLmax / maxall, ts = scal[S_TIMESTEP];
+    const double dt = (cfldt < ts) ? cfldt : ts;
+    scal[S_CFLDT] = cfldt;
+    scal[S_DT] = dt;
+    *(unsigned long long*)(scal + S_CFLMAX) = 0ull;
+    double t = scal[S_TVAL];
+    t = t + a.a0 * dt;
+    t = t + a.a1 * dt;
+    t = t + a.a2 * dt;
+    scal[S_TVAL] = t;
+    *ticket = 0u;
+}
+
 // find_cfl (pllcart3d.c:3095-3118): max over interior cells of
 // |u|/dx+|v|/dy+|w|/dz at cell centres, reduced exactly through the bit
 // pattern of non-negative doubles; a NaN/Inf raises ST_NAN (the reference's
@@ -167,7 +204,7 @@ template <typename real>
 __device__ __forceinline__ void k_cfl_run(const uint3 blockIdx, const dim3 gridDim,
     Geo G, Rng R, Consts K, const real* __restrict__ u,
                                              const real* __restrict__ v, const real* __restrict__ w,
-                                             double* scal, int* status)
+                                             double* scal, int* status, unsigned* ticket, StepTime a)
 {
     const int k = R.ks + blockIdx.x * blockDim.x + threadIdx.x;
     const int j = R.js + blockIdx.y * blockDim.y + threadIdx.y;
@@ -178,12 +215,7 @@ __device__ __forceinline__ void k_cfl_run(const uint3 blockIdx, const dim3 gridD
         double uv = 0.5 * ((double)u[id] + (double)u[id + G.sx]);
         double vv = 0.5 * ((double)v[id] + (double)v[id + G.sy]);
         double wv = 0.5 * ((double)w[id] + (double)w[id + 1]);
-#if PLL_FP64_EXACT
         double cfl = (fabs(uv) / K.hx) + (fabs(vv) / K.hy) + (fabs(wv) / K.hz);
-#else
-        // the FP64 forms: reciprocal spacings, the fusions written out
-        double cfl = fma(fabs(wv), K.ihz, fma(fabs(vv), K.ihy, fabs(uv) * K.ihx));
-#endif
         if (!isfinite(cfl)) atomicOr(status, (int)ST_NAN);
         else m = cfl;
     }
@@ -202,39 +234,20 @@ __device__ __forceinline__ void k_cfl_run(const uint3 blockIdx, const dim3 gridD
         if (lane == 0 && m > 0.0)
             atomicMax((unsigned long long*)(scal + S_CFLMAX), (unsigned long long)__double_as_longlong(m));
     }
+    if (last_block(ticket, gridDim.x * gridDim.y * gridDim.z) && threadIdx.x == 0 && threadIdx.y == 0)
+        step_dt(K, scal, ticket, a);
 }
 template <typename real>
 __global__ void __launch_bounds__(256) k_cfl(Geo G, Rng R, Consts K, const real* __restrict__ u,
                                              const real* __restrict__ v, const real* __restrict__ w,
-                                             double* scal, int* status)
+                                             double* scal, int* status, unsigned* ticket, StepTime a)
 {
-    k_cfl_run<real>(blockIdx, gridDim, G, R, K, u, v, w, scal, status);
+    k_cfl_run<real>(blockIdx, gridDim, G, R, K, u, v, w, scal, status, ticket, a);
 }
 template <typename real>
 struct k_cfl_b {
     static constexpr auto run = &k_cfl_run<real>;
     static constexpr int maxt = 256, minb = 0;
-};
-
-// dt = min(CFLmax / max, Timestep), pllcart3d.c:159-160, 3115; clears the
-// reduction slot for the next step
-static __device__ __forceinline__ void k_dt_run(const uint3 blockIdx, const dim3 gridDim,
-    Consts K, double* scal)
-{
-    double maxall = __longlong_as_double((long long)*(unsigned long long*)(scal + S_CFLMAX));
-    double cfldt = K.CFLmax / maxall;
-    double ts = scal[S_TIMESTEP];
-    scal[S_CFLDT] = cfldt;
-    scal[S_DT] = (cfldt < ts) ? cfldt : ts;
-    *(unsigned long long*)(scal + S_CFLMAX) = 0ull;
-}
-static __global__ void k_dt(Consts K, double* scal)
-{
-    k_dt_run(blockIdx, gridDim, K, scal);
-}
-struct k_dt_b {
-    static constexpr auto run = &k_dt_run;
-    static constexpr int maxt = 0, minb = 0;
 };
 
 // inflow/outflow trapezoid fluxes of velo_correction (pllcart3d.c:2171-2223):
@@ -337,19 +350,21 @@ struct k_div_rhs2_b {
     static constexpr int maxt = 128, minb = 0;
 };
 
-// The precision form's CFL scan: cell pairs (k, k+32), CFL_NI planes per
-// thread, the per-cell speed sum in FP64 (the reciprocal spacings multiply:
-// the precision form's dt may differ from the division's in the last bit)
+// The CFL scan outside the exact form: cell pairs (k, k+32), CFL_NI planes per
+// thread, the per-cell speed sum in FP64 (the reciprocal spacings multiply,
+// the fusions written out: dt may differ from the division's in the last bit)
 // and a thread-local maximum before the warp and block reductions.  The
 // maximum itself does not depend on the order.  A second cell past ke reads
 // the slack past the arrays and is left out.
 constexpr int CFL_NI = 8;
 
-__device__ __forceinline__ void k_cfl2_run(const uint3 blockIdx, const dim3 gridDim,
-    Geo G, Rng R, Consts K, const float* __restrict__ u,
-                                              const float* __restrict__ v, const float* __restrict__ w, double* scal,
-                                              int* status)
+template <typename real>
+__device__ __forceinline__ void k_cfl2_run(const uint3 blockIdx, const dim3 gridDim, Geo G, Rng R, Consts K,
+                                           const real* __restrict__ u, const real* __restrict__ v,
+                                           const real* __restrict__ w, double* scal, int* status, unsigned* ticket,
+                                           StepTime a)
 {
+    using T2 = typename PairOf<real>::type;
     const int k = R.ks + blockIdx.x * (2 * EP_DK) + threadIdx.x;
     const int j = R.js + blockIdx.y * blockDim.y + threadIdx.y;
     const int i0 = R.is + blockIdx.z * CFL_NI;
@@ -359,17 +374,16 @@ __device__ __forceinline__ void k_cfl2_run(const uint3 blockIdx, const dim3 grid
         const bool live_b = k + EP_DK <= R.ke;
         const long sx = G.sx, sy = G.sy;
         long id = (long)i0 * sx + (long)j * sy + k;
-        f2 u0 = ld2(u, id);
+        auto speed = [&](double u0, double u1, double v0, double v1, double w0, double w1) {
+            return fma(fabs(w0 + w1), K.hiz, fma(fabs(v0 + v1), K.hiy, mul_rn_(fabs(u0 + u1), K.hix)));
+        };
+        T2 u0 = ld2(u, id);
 #pragma unroll
         for (int t = 0; t < CFL_NI; ++t, id += sx) {
             if (i0 + t > R.ie) break;
-            const f2 u1 = ld2(u, id + sx), v0 = ld2(v, id), v1 = ld2(v, id + sy), w0 = ld2(w, id), w1 = ld2(w, id + 1);
-            double ca = fabs(0.5 * ((double)u0.v.x + (double)u1.v.x)) * K.ihx +
-                        fabs(0.5 * ((double)v0.v.x + (double)v1.v.x)) * K.ihy +
-                        fabs(0.5 * ((double)w0.v.x + (double)w1.v.x)) * K.ihz;
-            double cb = fabs(0.5 * ((double)u0.v.y + (double)u1.v.y)) * K.ihx +
-                        fabs(0.5 * ((double)v0.v.y + (double)v1.v.y)) * K.ihy +
-                        fabs(0.5 * ((double)w0.v.y + (double)w1.v.y)) * K.ihz;
+            const T2 u1 = ld2(u, id + sx), v0 = ld2(v, id), v1 = ld2(v, id + sy), w0 = ld2(w, id), w1 = ld2(w, id + 1);
+            const double ca = speed(u0.v.x, u1.v.x, v0.v.x, v1.v.x, w0.v.x, w1.v.x);
+            double cb = speed(u0.v.y, u1.v.y, v0.v.y, v1.v.y, w0.v.y, w1.v.y);
             if (!live_b) cb = 0.0;
             if (isfinite(ca)) m = fmax(m, ca);
             else bad = true;
@@ -394,39 +408,30 @@ __device__ __forceinline__ void k_cfl2_run(const uint3 blockIdx, const dim3 grid
         if (lane == 0 && m > 0.0)
             atomicMax((unsigned long long*)(scal + S_CFLMAX), (unsigned long long)__double_as_longlong(m));
     }
+    if (last_block(ticket, gridDim.x * gridDim.y * gridDim.z) && threadIdx.x == 0 && threadIdx.y == 0)
+        step_dt(K, scal, ticket, a);
 }
-__global__ void __launch_bounds__(256) k_cfl2(Geo G, Rng R, Consts K, const float* __restrict__ u,
-                                              const float* __restrict__ v, const float* __restrict__ w, double* scal,
-                                              int* status)
+template <typename real>
+__global__ void __launch_bounds__(256) k_cfl2(Geo G, Rng R, Consts K, const real* __restrict__ u,
+                                              const real* __restrict__ v, const real* __restrict__ w, double* scal,
+                                              int* status, unsigned* ticket, StepTime a)
 {
-    k_cfl2_run(blockIdx, gridDim, G, R, K, u, v, w, scal, status);
+    k_cfl2_run<real>(blockIdx, gridDim, G, R, K, u, v, w, scal, status, ticket, a);
 }
+template <typename real>
 struct k_cfl2_b {
-    static constexpr auto run = &k_cfl2_run;
+    static constexpr auto run = &k_cfl2_run<real>;
     static constexpr int maxt = 256, minb = 0;
 };
 
-// Last-block ticket: every block's results are written and fenced before it
-// takes a ticket; the block that takes the last one reads them all and
-// resets the counter for the next launch.
-__device__ __forceinline__ bool last_block(unsigned* ticket)
-{
-    __shared__ bool is_last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) is_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
-    __syncthreads();
-    if (is_last) __threadfence();
-    return is_last;
-}
-
-// The precision form's inflow/outflow fluxes: the trapezoid sums of k_flux
+// The inflow/outflow fluxes outside the exact form: the trapezoid sums of k_flux
 // in FP64, evaluated in parallel in a fixed order (every run gives the same
 // bits): one warp per row of either plane, lane l summing the terms k =
 // ks+1+l, ks+1+l+32, ... and a fixed shuffle tree; the last block forms the
 // sum over y the same way from the row sums.  Blocks of 1024 threads.
+template <typename real>
 __device__ __forceinline__ void k_flux3_run(const uint3 blockIdx, const dim3 gridDim,
-    Geo G, Rng Ru, Consts K, const float* __restrict__ u, double* red,
+    Geo G, Rng Ru, Consts K, const real* __restrict__ u, double* red,
                                                 unsigned* ticket, double* scal)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -446,7 +451,7 @@ __device__ __forceinline__ void k_flux3_run(const uint3 blockIdx, const dim3 gri
         q = tree(q);
         if (lane == 0) red[plane * G.NY + j] = q;
     }
-    if (!last_block(ticket)) return;
+    if (!last_block(ticket, gridDim.x)) return;
     if (warp == 0) {
         double qin = 0.0, qout = 0.0;
         for (int j = Ru.js + 1 + lane; j <= Ru.je; j += 32) {
@@ -463,13 +468,15 @@ __device__ __forceinline__ void k_flux3_run(const uint3 blockIdx, const dim3 gri
         }
     }
 }
-__global__ void __launch_bounds__(1024) k_flux3(Geo G, Rng Ru, Consts K, const float* __restrict__ u, double* red,
+template <typename real>
+__global__ void __launch_bounds__(1024) k_flux3(Geo G, Rng Ru, Consts K, const real* __restrict__ u, double* red,
                                                 unsigned* ticket, double* scal)
 {
-    k_flux3_run(blockIdx, gridDim, G, Ru, K, u, red, ticket, scal);
+    k_flux3_run<real>(blockIdx, gridDim, G, Ru, K, u, red, ticket, scal);
 }
+template <typename real>
 struct k_flux3_b {
-    static constexpr auto run = &k_flux3_run;
+    static constexpr auto run = &k_flux3_run<real>;
     static constexpr int maxt = 1024, minb = 0;
 };
 
@@ -518,7 +525,7 @@ __device__ __forceinline__ void k_bulk2_run(const uint3 blockIdx, const dim3 gri
         }
         if (lane == 0) { pv[blockIdx.x] = best; pi[blockIdx.x] = (double)bidx; }
     }
-    if (!last_block(ticket)) return;
+    if (!last_block(ticket, gridDim.x)) return;
     if (warp == 0) {
         best = 0.0;
         bidx = 0x7fffffff;
@@ -717,43 +724,43 @@ struct k_poisson_x_b {
 };
 
 // update_phi_ghosts (pllcart3d.c:2758-2807): Neumann copies on the six
-// faces; FACE 0: z faces over (i,j), 1: y faces over (i,k), 2: x faces over
-// (j,k)
-template <int FACE, typename real>
+// faces; blockIdx.z 0: z faces over (i,j), 1: y faces over (i,k), 2: x faces
+// over (j,k).  blockIdx.y runs to the longest of the second extents.
+template <typename real>
 __device__ __forceinline__ void k_phi_ghosts_run(const uint3 blockIdx, const dim3 gridDim,
     Geo G, Rng R, real* __restrict__ p)
 {
     const int a = blockIdx.x * blockDim.x + threadIdx.x;
     const int b = blockIdx.y;
     const long sx = G.sx, sy = G.sy;
-    if (FACE == 0) {
+    if (blockIdx.z == 0) {
         const int j = R.js + a, i = R.is + b;
-        if (j > R.je) return;
+        if (j > R.je || i > R.ie) return;
         const long base = (long)i * sx + (long)j * sy;
         p[base + R.ks - 1] = p[base + R.ks];
         p[base + R.ke + 1] = p[base + R.ke];
-    } else if (FACE == 1) {
+    } else if (blockIdx.z == 1) {
         const int k = R.ks + a, i = R.is + b;
-        if (k > R.ke) return;
+        if (k > R.ke || i > R.ie) return;
         const long base = (long)i * sx + k;
         p[base + (long)(R.js - 1) * sy] = p[base + (long)R.js * sy];
         p[base + (long)(R.je + 1) * sy] = p[base + (long)R.je * sy];
     } else {
         const int k = R.ks + a, j = R.js + b;
-        if (k > R.ke) return;
+        if (k > R.ke || j > R.je) return;
         const long base = (long)j * sy + k;
         p[base + (long)(R.is - 1) * sx] = p[base + (long)R.is * sx];
         p[base + (long)(R.ie + 1) * sx] = p[base + (long)R.ie * sx];
     }
 }
-template <int FACE, typename real>
+template <typename real>
 __global__ void k_phi_ghosts(Geo G, Rng R, real* __restrict__ p)
 {
-    k_phi_ghosts_run<FACE, real>(blockIdx, gridDim, G, R, p);
+    k_phi_ghosts_run<real>(blockIdx, gridDim, G, R, p);
 }
-template <int FACE, typename real>
+template <typename real>
 struct k_phi_ghosts_b {
-    static constexpr auto run = &k_phi_ghosts_run<FACE, real>;
+    static constexpr auto run = &k_phi_ghosts_run<real>;
     static constexpr int maxt = 0, minb = 0;
 };
 

@@ -31,7 +31,8 @@ struct Bufs {
     real* pg[4] = {};       // u, v, w at 1..3
     real* phi = nullptr;
     real* div = nullptr;
-    real* S = nullptr;      // ADI right-hand side / eliminated rhs
+    real* S[4] = {};        // ADI right-hand side / eliminated rhs of each variable
+                            // (the exact form: one array for all)
     real* cc = nullptr;     // Thomas scratch
     real* dct1 = nullptr;   // compact nx*ny*nz Poisson buffers
     real* dct2 = nullptr;
@@ -69,6 +70,11 @@ struct pllgpu_ctx {
     int dev = 0;
     bool mixed = false;
     cudaStream_t st = nullptr;
+    // side branches of a step (kernels that do not depend on one another),
+    // forked from and joined back into st; `at` is where go() launches
+    static constexpr int NSIDE = 3;
+    cudaStream_t side[NSIDE] = {}, at = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join[NSIDE] = {};
     long nelem = 0;             // elements of one padded field
     Bufs<double> b64;           // state of the FP64 form
     Bufs<float> b32;            // state of the mixed form
@@ -83,7 +89,7 @@ struct pllgpu_ctx {
     int* status = nullptr;      // device sticky status bits
     double* work = nullptr;     // slope-parameter scratch
     double* red = nullptr;      // multi-block reduction partials (RED_DOUBLES)
-    unsigned* ticket = nullptr; // last-block tickets of those reductions (2, self-resetting)
+    unsigned* ticket = nullptr; // last-block tickets of those reductions (3, self-resetting)
     double* diag = nullptr;     // per-plane diagnostics + results
     int cur = 0;                // buffer index holding the "old" role
     bool resync_c = false;      // after a restart: copy c's buffers once (resume)

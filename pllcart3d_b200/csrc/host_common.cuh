@@ -41,7 +41,38 @@ void go(pllgpu_ctx* ctx, void (*k)(P...), dim3 grid, dim3 blk, size_t smem, A&&.
         ctx->rec->push_back(r);
         return;
     }
-    k<<<grid, blk, smem, ctx->st>>>(std::forward<A>(a)...);
+    k<<<grid, blk, smem, ctx->at>>>(std::forward<A>(a)...);
+}
+
+// Side branches of the step.  fork(n) lets side streams 0 .. n-1 start after
+// everything enqueued so far, on_side(i) sends the following launches there
+// (on_side(-1): back to the main stream), join(n) makes the main stream wait
+// for them.  A step recorded for an ensemble, or profiled launch by launch, has
+// no branches: its launches stay in order.
+bool branches(const pllgpu_ctx* c) { return !c->rec && !c->profiling; }
+
+void fork(pllgpu_ctx* ctx, int n)
+{
+    if (!branches(ctx)) return;
+    bool ok = cudaEventRecord(ctx->ev_fork, ctx->st) == cudaSuccess;
+    for (int i = 0; i < n && ok; ++i) ok = cudaStreamWaitEvent(ctx->side[i], ctx->ev_fork, 0) == cudaSuccess;
+    if (!ok) fail(ctx, PLLGPU_ECUDA);
+}
+
+void on_side(pllgpu_ctx* ctx, int i)
+{
+    if (branches(ctx)) ctx->at = i < 0 ? ctx->st : ctx->side[i];
+}
+
+void join(pllgpu_ctx* ctx, int n)
+{
+    if (!branches(ctx)) return;
+    ctx->at = ctx->st;
+    bool ok = true;
+    for (int i = 0; i < n && ok; ++i)
+        ok = cudaEventRecord(ctx->ev_join[i], ctx->side[i]) == cudaSuccess &&
+             cudaStreamWaitEvent(ctx->st, ctx->ev_join[i], 0) == cudaSuccess;
+    if (!ok) fail(ctx, PLLGPU_ECUDA);
 }
 
 // every kernel launch of the step goes through mark(): it counts launches

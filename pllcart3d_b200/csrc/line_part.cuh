@@ -251,6 +251,7 @@ __device__ __forceinline__ void k_line_seg_run(const uint3 blockIdx, const dim3 
     const int tid = threadIdx.x;
     const int k0 = blockIdx.x * TL;
     const int o = blockIdx.y;   // j (x lines) or i (y lines) offset
+    if (o > (AXIS == 0 ? R.je - R.js : R.ie - R.is)) return;   // past a component's shorter extent
     const int n = AXIS == 0 ? R.ie - R.is + 1 : R.je - R.js + 1;
     const long st = AXIS == 0 ? G.sx : G.sy;
     const long base0 = AXIS == 0 ? (long)R.is * G.sx + (long)(R.js + o) * G.sy + k0
@@ -352,6 +353,31 @@ struct k_line_seg_b {
     static constexpr int maxt = LinePart<VAR, AXIS, real, E, L, TL>::T, minb = 0;
 };
 
+// the three momentum components' lines in one launch, component VU + blockIdx.z
+template <typename real>
+struct Sweeps3 {
+    Rng R[3];
+    XsweepArgs<real> A[3];
+};
+template <int AXIS, typename real, int E, int L, int TL>
+__device__ __forceinline__ void k_line_seg3_run(const uint3 blockIdx, const dim3 gridDim, Geo G, Consts K,
+                                                Sweeps3<real> S)
+{
+    if (blockIdx.z == 0) k_line_seg_run<VU, AXIS, real, E, L, TL>(blockIdx, gridDim, G, S.R[0], K, S.A[0]);
+    else if (blockIdx.z == 1) k_line_seg_run<VV, AXIS, real, E, L, TL>(blockIdx, gridDim, G, S.R[1], K, S.A[1]);
+    else k_line_seg_run<VW, AXIS, real, E, L, TL>(blockIdx, gridDim, G, S.R[2], K, S.A[2]);
+}
+template <int AXIS, typename real, int E, int L, int TL>
+__global__ void __launch_bounds__(LinePart<VU, AXIS, real, E, L, TL>::T) k_line_seg3(Geo G, Consts K, Sweeps3<real> S)
+{
+    k_line_seg3_run<AXIS, real, E, L, TL>(blockIdx, gridDim, G, K, S);
+}
+template <int AXIS, typename real, int E, int L, int TL>
+struct k_line_seg3_b {
+    static constexpr auto run = &k_line_seg3_run<AXIS, real, E, L, TL>;
+    static constexpr int maxt = LinePart<VU, AXIS, real, E, L, TL>::T, minb = 0;
+};
+
 // ---- z lines ---------------------------------------------------------------------
 // The contiguous axis: a warp moves its own 32 / L lines (consecutive j)
 // through a skewed shared buffer, whole rows at a time, in place.
@@ -361,19 +387,18 @@ __device__ __forceinline__ void k_adi_z_part_run(const uint3 blockIdx, const dim
                                                  const double* __restrict__ scal, double alpha)
 {
     constexpr int LPW = 32 / L, PITCH = L * (E + 1) + 1;
-    __shared__ real bS[4][LPW * PITCH];
-    __shared__ real bM[VAR == VC ? 1 : 4][VAR == VC ? 1 : LPW * PITCH];
+    extern __shared__ __align__(16) unsigned char lp_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int j0 = R.js + (blockIdx.x * 4 + warp) * LPW;
     const int i = R.is + blockIdx.y;
-    if (j0 > R.je) return;   // warp-uniform
+    if (j0 > R.je || i > R.ie) return;   // warp-uniform
     const int nl = min(LPW, R.je - j0 + 1);
     const int n = R.ke - R.ks + 1;
     const real* __restrict__ mz = VAR == VU ? mu.xz : VAR == VV ? mu.yz : mu.cell;
     const int moff = VAR == VW ? -1 : 0;
     const long base = (long)i * G.sx + (long)j0 * G.sy + R.ks;
-    real* sS = bS[warp];
-    real* sM = bM[VAR == VC ? 0 : warp];
+    real* sS = (real*)lp_raw + warp * LPW * PITCH;
+    real* sM = sS + 4 * LPW * PITCH;
     auto skew = [](int m) { return m + m / E; };
 #pragma unroll
     for (int q = 0; q < LPW; ++q) {
@@ -409,6 +434,11 @@ __device__ __forceinline__ void k_adi_z_part_run(const uint3 blockIdx, const dim
     }
 }
 template <int VAR, typename real, int E, int L>
+constexpr size_t z_part_smem()
+{
+    return sizeof(real) * 4 * (32 / L) * (L * (E + 1) + 1) * (VAR == VC ? 1 : 2);
+}
+template <int VAR, typename real, int E, int L>
 __global__ void __launch_bounds__(128) k_adi_z_part(Geo G, Rng R, Consts K, MuPtrs<real> mu, real* __restrict__ S,
                                                     const double* __restrict__ scal, double alpha)
 {
@@ -417,6 +447,30 @@ __global__ void __launch_bounds__(128) k_adi_z_part(Geo G, Rng R, Consts K, MuPt
 template <int VAR, typename real, int E, int L>
 struct k_adi_z_part_b {
     static constexpr auto run = &k_adi_z_part_run<VAR, real, E, L>;
+    static constexpr int maxt = 128, minb = 0;
+};
+
+template <typename real, int E, int L>
+__device__ __forceinline__ void k_adi_z_part3_run(const uint3 blockIdx, const dim3 gridDim, Geo G, Consts K,
+                                                  Sweeps3<real> S)
+{
+    // constant indexes: a batched copy's arguments would go to local memory
+    const XsweepArgs<real>&U = S.A[0], &V = S.A[1], &W = S.A[2];
+    if (blockIdx.z == 0)
+        k_adi_z_part_run<VU, real, E, L>(blockIdx, gridDim, G, S.R[0], K, U.mu, U.S, U.scal, U.alpha);
+    else if (blockIdx.z == 1)
+        k_adi_z_part_run<VV, real, E, L>(blockIdx, gridDim, G, S.R[1], K, V.mu, V.S, V.scal, V.alpha);
+    else
+        k_adi_z_part_run<VW, real, E, L>(blockIdx, gridDim, G, S.R[2], K, W.mu, W.S, W.scal, W.alpha);
+}
+template <typename real, int E, int L>
+__global__ void __launch_bounds__(128) k_adi_z_part3(Geo G, Consts K, Sweeps3<real> S)
+{
+    k_adi_z_part3_run<real, E, L>(blockIdx, gridDim, G, K, S);
+}
+template <typename real, int E, int L>
+struct k_adi_z_part3_b {
+    static constexpr auto run = &k_adi_z_part3_run<real, E, L>;
     static constexpr int maxt = 128, minb = 0;
 };
 

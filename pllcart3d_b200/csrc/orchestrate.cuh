@@ -116,7 +116,7 @@ void launch_explicit(pllgpu_ctx* ctx, const real* un, const real* vn, const real
     A.pg = VAR == VC ? nullptr : bufs<real>(ctx).pg[VAR];
     A.Hm = h_nm1<real>(ctx, VAR);
     A.H = h_n<real>(ctx, VAR);
-    A.S = bufs<real>(ctx).S;
+    A.S = bufs<real>(ctx).S[VAR];
     A.scal = ctx->scal;
     A.g = g;
     A.r = r;
@@ -175,23 +175,59 @@ bool launch_line_part(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X)
 }
 
 template <int VAR, typename real, int L>
-void z_part(pllgpu_ctx* ctx, const Rng& R, const MuPtrs<real>& mu, double alpha)
+void z_part(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X)
 {
     constexpr int LINES = 4 * (32 / L);   // per block
     go<k_adi_z_part_b<VAR, real, 8, L>>(ctx, k_adi_z_part<VAR, real, 8, L>, dim3((nj(R) + LINES - 1) / LINES, ni(R)),
-                                        128, 0, ctx->G, R, ctx->K, mu, bufs<real>(ctx).S, ctx->scal, alpha);
+                                        128, z_part_smem<VAR, real, 8, L>(), ctx->G, R, ctx->K, X.mu, X.S, ctx->scal,
+                                        X.alpha);
 }
 
 template <int VAR, typename real>
-bool launch_z_part(pllgpu_ctx* ctx, const Rng& R, const MuPtrs<real>& mu, double alpha)
+bool launch_z_part(pllgpu_ctx* ctx, const Rng& R, const XsweepArgs<real>& X)
 {
     const int n = nk(R);
     if (ctx->P.exact_dct || n > Z_PART_MAX) return false;
-    if (n <= 32) z_part<VAR, real, 4>(ctx, R, mu, alpha);
-    else if (n <= 64) z_part<VAR, real, 8>(ctx, R, mu, alpha);
-    else if (n <= 128) z_part<VAR, real, 16>(ctx, R, mu, alpha);
-    else z_part<VAR, real, 32>(ctx, R, mu, alpha);
+    if (n <= 32) z_part<VAR, real, 4>(ctx, R, X);
+    else if (n <= 64) z_part<VAR, real, 8>(ctx, R, X);
+    else if (n <= 128) z_part<VAR, real, 16>(ctx, R, X);
+    else z_part<VAR, real, 32>(ctx, R, X);
     return true;
+}
+
+// the same for u, v and w together
+template <int AXIS, typename real, int E, int L, int TL>
+void line_part3(pllgpu_ctx* ctx, const Sweeps3<real>& S)
+{
+    using LP = LinePart<VU, AXIS, real, E, L, TL>;
+    if (LP::SMEM > 48 * 1024)
+        cudaFuncSetAttribute(k_line_seg3<AXIS, real, E, L, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)LP::SMEM);
+    const Rng& R = ctx->Rg;
+    go<k_line_seg3_b<AXIS, real, E, L, TL>>(ctx, k_line_seg3<AXIS, real, E, L, TL>,
+                                            dim3(R.ke / TL + 1, AXIS == 0 ? nj(R) : ni(R), 3), LP::T, LP::SMEM, ctx->G,
+                                            ctx->K, S);
+}
+
+template <int AXIS, typename real>
+void launch_line_part3(pllgpu_ctx* ctx, const Sweeps3<real>& S)
+{
+    const int n = AXIS == 0 ? ctx->G.nx : ctx->G.ny;
+    constexpr int TL = sizeof(real) == 8 ? 8 : 16;
+    if (n <= 32) line_part3<AXIS, real, 8, 4, TL>(ctx, S);
+    else if (n <= 64) line_part3<AXIS, real, 8, 8, TL>(ctx, S);
+    else if (n <= 128) line_part3<AXIS, real, 8, 16, TL>(ctx, S);
+    else if (n <= 256) line_part3<AXIS, real, 8, 32, TL>(ctx, S);
+    else line_part3<AXIS, real, 16, 32, 8>(ctx, S);
+}
+
+template <typename real, int L>
+void z_part3(pllgpu_ctx* ctx, const Sweeps3<real>& S)
+{
+    constexpr int LINES = 4 * (32 / L);
+    go<k_adi_z_part3_b<real, 8, L>>(ctx, k_adi_z_part3<real, 8, L>,
+                                    dim3((ctx->G.ny + LINES - 1) / LINES, ctx->G.nx, 3), 128,
+                                    z_part_smem<VU, real, 8, L>(), ctx->G, ctx->K, S);
 }
 
 template <typename T, int E, int L, int TL>
@@ -223,43 +259,52 @@ void launch_modes(pllgpu_ctx* ctx, T* hat, int kz_major)
 }
 
 template <typename real, int VAR>
-void launch_implicit(pllgpu_ctx* ctx, double g, double r)
+XsweepArgs<real> sweep_args(pllgpu_ctx* ctx, double g, double r)
 {
-    static const char* ly[4] = {"adi_y_c", "adi_y_u", "adi_y_v", "adi_y_w"};
-    static const char* lz[4] = {"adi_z_c", "adi_z_u", "adi_z_v", "adi_z_w"};
-    static const char* lx[4] = {"adi_x_c", "adi_x_u", "adi_x_v", "adi_x_w"};
-    const Rng& R = ctx->Rv[VAR];
-    const double alpha = g + r;
-    Bufs<real>& B = bufs<real>(ctx);
     XsweepArgs<real> X;
     X.mu = mu_new<real>(ctx);
     X.q = q_old<real>(ctx, VAR);
     X.qn = q_new<real>(ctx, VAR);
     X.H = h_n<real>(ctx, VAR);
     X.Hm = h_nm1<real>(ctx, VAR);
-    X.S = B.S;
-    X.cc = B.cc;
+    X.S = bufs<real>(ctx).S[VAR];
+    X.cc = bufs<real>(ctx).cc;
     X.scal = ctx->scal;
     X.g = g;
     X.r = r;
-    X.alpha = alpha;
+    X.alpha = g + r;
+    return X;
+}
+
+// whether the line solves are the partitioned ones: never in the exact form
+// (the reference's sweeps), which in FP64 is a unit of its own
+template <typename real>
+constexpr bool part_form()
+{
+    return sizeof(real) == 4 || !PLL_FP64_EXACT;
+}
+
+template <typename real, int VAR>
+void launch_implicit(pllgpu_ctx* ctx, double g, double r)
+{
+    static const char* ly[4] = {"adi_y_c", "adi_y_u", "adi_y_v", "adi_y_w"};
+    static const char* lz[4] = {"adi_z_c", "adi_z_u", "adi_z_v", "adi_z_w"};
+    static const char* lx[4] = {"adi_x_c", "adi_x_u", "adi_x_v", "adi_x_w"};
+    const Rng& R = ctx->Rv[VAR];
+    const XsweepArgs<real> X = sweep_args<real, VAR>(ctx, g, r);
+    constexpr bool part = part_form<real>();
     const int lb = tune_line_block(ctx->tune_line);
-#if PLL_FP64_EXACT
-    constexpr bool part = sizeof(real) == 4;   // the exact form keeps the reference's sweeps
-#else
-    constexpr bool part = true;
-#endif
     bool ydone = false, zdone = false, xdone = false;
     if constexpr (part) ydone = launch_line_part<VAR, 1, real>(ctx, R, X);
     if (!ydone)
         go<k_line_pf_b<VAR, 1, real>>(ctx, k_line_pf<VAR, 1, real>, dim3((nk(R) + lb - 1) / lb, ni(R)), lb, 0, ctx->G,
                                       R, ctx->K, X);
     mark(ctx, ly[VAR]);
-    if constexpr (part) zdone = launch_z_part<VAR, real>(ctx, R, X.mu, alpha);
+    if constexpr (part) zdone = launch_z_part<VAR, real>(ctx, R, X);
     if (!zdone) {
         constexpr size_t smem = adi_z_smem_bytes<VAR, real>();
         go<k_adi_z_tiled_b<VAR, real>>(ctx, k_adi_z_tiled<VAR, real>, dim3((nj(R) + 127) / 128, ni(R)), 128, smem,
-                                       ctx->G, R, ctx->K, X.mu, B.S, B.cc, ctx->scal, alpha);
+                                       ctx->G, R, ctx->K, X.mu, X.S, X.cc, ctx->scal, X.alpha);
     }
     mark(ctx, lz[VAR]);
     if constexpr (part) xdone = launch_line_part<VAR, 0, real>(ctx, R, X);
@@ -267,6 +312,35 @@ void launch_implicit(pllgpu_ctx* ctx, double g, double r)
         go<k_line_pf_b<VAR, 0, real>>(ctx, k_line_pf<VAR, 0, real>, dim3((nk(R) + lb - 1) / lb, nj(R)), lb, 0, ctx->G,
                                       R, ctx->K, X);
     mark(ctx, lx[VAR]);
+}
+
+// u, v and w, whose right-hand sides stand ready: one launch per axis where
+// the partitioned solves take every line (a third of the launches, and on
+// small grids a third of their time: each fills a fraction of the chip)
+template <typename real>
+void launch_implicit_uvw(pllgpu_ctx* ctx, double g, double r)
+{
+    if constexpr (part_form<real>()) {
+        if (!ctx->P.exact_dct && ctx->G.nx <= LINE_PART_MAX && ctx->G.ny <= LINE_PART_MAX && ctx->G.nz <= Z_PART_MAX) {
+            const Sweeps3<real> S{{ctx->Rv[VU], ctx->Rv[VV], ctx->Rv[VW]},
+                                  {sweep_args<real, VU>(ctx, g, r), sweep_args<real, VV>(ctx, g, r),
+                                   sweep_args<real, VW>(ctx, g, r)}};
+            launch_line_part3<1, real>(ctx, S);
+            mark(ctx, "adi_y_uvw");
+            const int n = ctx->G.nz;
+            if (n <= 32) z_part3<real, 4>(ctx, S);
+            else if (n <= 64) z_part3<real, 8>(ctx, S);
+            else if (n <= 128) z_part3<real, 16>(ctx, S);
+            else z_part3<real, 32>(ctx, S);
+            mark(ctx, "adi_z_uvw");
+            launch_line_part3<0, real>(ctx, S);
+            mark(ctx, "adi_x_uvw");
+            return;
+        }
+    }
+    launch_implicit<real, VU>(ctx, g, r);
+    launch_implicit<real, VV>(ctx, g, r);
+    launch_implicit<real, VW>(ctx, g, r);
 }
 
 template <typename real>
@@ -469,11 +543,9 @@ void launch_phi_ghosts(pllgpu_ctx* ctx)
 {
     const Rng& R = ctx->Rg;
     real* phi = bufs<real>(ctx).phi;
-    go<k_phi_ghosts_b<0, real>>(ctx, k_phi_ghosts<0, real>, dim3((nj(R) + 127) / 128, ni(R)), 128, 0, ctx->G, R, phi);
-    mark(ctx, "phi_ghosts");
-    go<k_phi_ghosts_b<1, real>>(ctx, k_phi_ghosts<1, real>, dim3((nk(R) + 127) / 128, ni(R)), 128, 0, ctx->G, R, phi);
-    mark(ctx, "phi_ghosts");
-    go<k_phi_ghosts_b<2, real>>(ctx, k_phi_ghosts<2, real>, dim3((nk(R) + 127) / 128, nj(R)), 128, 0, ctx->G, R, phi);
+    const int m = std::max(nj(R), nk(R));
+    go<k_phi_ghosts_b<real>>(ctx, k_phi_ghosts<real>, dim3((m + 127) / 128, std::max(ni(R), nj(R)), 3), 128, 0, ctx->G,
+                             R, phi);
     mark(ctx, "phi_ghosts");
 }
 
@@ -524,43 +596,43 @@ void launch_div(pllgpu_ctx* ctx, int mode, double alpha)
 template <typename real>
 void launch_flux(pllgpu_ctx* ctx)
 {
-    if constexpr (std::is_same<real, float>::value) {
+    if constexpr (part_form<real>()) {
         const int rows = 2 * nj(ctx->Rv[VU]);
-        go<k_flux3_b>(ctx, k_flux3, (rows + 31) / 32, 1024, 0, ctx->G, ctx->Rv[VU], ctx->K, q_new<real>(ctx, VU),
-                      ctx->red, ctx->ticket, ctx->scal);
-        mark(ctx, "flux");
-        return;
+        go<k_flux3_b<real>>(ctx, k_flux3<real>, (rows + 31) / 32, 1024, 0, ctx->G, ctx->Rv[VU], ctx->K,
+                            q_new<real>(ctx, VU), ctx->red, ctx->ticket, ctx->scal);
+    } else {
+        go<k_flux_b<real>>(ctx, k_flux<real>, 1, 512, sizeof(double) * 2 * ctx->G.NY, ctx->G, ctx->Rv[VU], ctx->K,
+                           q_new<real>(ctx, VU), ctx->scal);
     }
-    go<k_flux_b<real>>(ctx, k_flux<real>, 1, 512, sizeof(double) * 2 * ctx->G.NY, ctx->G, ctx->Rv[VU], ctx->K,
-                                                                       q_new<real>(ctx, VU), ctx->scal);
     mark(ctx, "flux");
 }
 
 template <typename real>
 void launch_bulk(pllgpu_ctx* ctx)
 {
-    go<k_bulk2_b<real>>(ctx, k_bulk2<real>, BULK_BLOCKS, 1024, 0, ctx->G, ctx->Rg, q_old<real>(ctx, VU), ctx->red,
-                                                      ctx->ticket + 1, ctx->scal);
+    // a value per thread of a block, up to BULK_BLOCKS blocks
+    const int blocks = std::min(BULK_BLOCKS, (nj(ctx->Rg) * nk(ctx->Rg) + 1023) / 1024);
+    go<k_bulk2_b<real>>(ctx, k_bulk2<real>, blocks, 1024, 0, ctx->G, ctx->Rg, q_old<real>(ctx, VU), ctx->red,
+                        ctx->ticket + 1, ctx->scal);
     mark(ctx, "bulk_velo");
 }
 
+// the CFL scan and, by its last block, dt and the simulated time
 template <typename real>
-void launch_cfl(pllgpu_ctx* ctx)
+void launch_cfl(pllgpu_ctx* ctx, StepTime a = {0.0, 0.0, 0.0})
 {
     dim3 blk(32, 8);
-    if constexpr (std::is_same<real, float>::value) {
+    if constexpr (part_form<real>()) {
         const dim3 grid((nk(ctx->Rg) + 2 * EP_DK - 1) / (2 * EP_DK), (nj(ctx->Rg) + blk.y - 1) / blk.y,
                         (ni(ctx->Rg) + CFL_NI - 1) / CFL_NI);
-        go<k_cfl2_b>(ctx, k_cfl2, grid, blk, 0, ctx->G, ctx->Rg, ctx->K, q_old<real>(ctx, VU), q_old<real>(ctx, VV),
-                                          q_old<real>(ctx, VW), ctx->scal, ctx->status);
+        go<k_cfl2_b<real>>(ctx, k_cfl2<real>, grid, blk, 0, ctx->G, ctx->Rg, ctx->K, q_old<real>(ctx, VU),
+                           q_old<real>(ctx, VV), q_old<real>(ctx, VW), ctx->scal, ctx->status, ctx->ticket + 2, a);
     } else {
         go<k_cfl_b<real>>(ctx, k_cfl<real>, box_grid(nk(ctx->Rg), nj(ctx->Rg), ni(ctx->Rg), blk), blk, 0, ctx->G,
                           ctx->Rg, ctx->K, q_old<real>(ctx, VU), q_old<real>(ctx, VV), q_old<real>(ctx, VW), ctx->scal,
-                          ctx->status);
+                          ctx->status, ctx->ticket + 2, a);
     }
     mark(ctx, "cfl");
-    go<k_dt_b>(ctx, k_dt, 1, 1, 0, ctx->K, ctx->scal);
-    mark(ctx, "dt");
 }
 
 // one RK3-CN substep of the fast path, pllcart3d.c:164-194
@@ -569,23 +641,48 @@ void enqueue_substep(pllgpu_ctx* ctx, int rk)
 {
     const double g = kRK1[rk], r = kRK2[rk], alpha = g + r;
     const real *uo = q_old<real>(ctx, VU), *vo = q_old<real>(ctx, VV), *wo = q_old<real>(ctx, VW);
+    // branches: whatever the next main-line kernel does not wait for.  The
+    // exact form keeps one right-hand side array, so its explicit operators
+    // and solves alternate; elsewhere those of u, v and w stand side by side.
+    fork(ctx, 1);
+    on_side(ctx, 0);
     launch_bulk<real>(ctx);
+    on_side(ctx, -1);
     // concentration: advected by u->new == u->old
     launch_explicit<real, VC>(ctx, uo, vo, wo, g, r);
+    join(ctx, 1);   // its outflow closure takes the bulk velocity
     launch_implicit<real, VC>(ctx, g, r);
-    launch_viscosity<real>(ctx, q_new<real>(ctx, VC), mu_new<real>(ctx));
-    launch_explicit<real, VU>(ctx, uo, vo, wo, g, r);
-    launch_implicit<real, VU>(ctx, g, r);
-    launch_explicit<real, VV>(ctx, uo, vo, wo, g, r);
-    launch_implicit<real, VV>(ctx, g, r);
-    launch_explicit<real, VW>(ctx, uo, vo, wo, g, r);
-    launch_implicit<real, VW>(ctx, g, r);
+    if constexpr (part_form<real>()) {
+        fork(ctx, 3);
+        on_side(ctx, 0);
+        launch_explicit<real, VV>(ctx, uo, vo, wo, g, r);
+        on_side(ctx, 1);
+        launch_explicit<real, VW>(ctx, uo, vo, wo, g, r);
+        on_side(ctx, 2);
+        launch_viscosity<real>(ctx, q_new<real>(ctx, VC), mu_new<real>(ctx));
+        on_side(ctx, -1);
+        launch_explicit<real, VU>(ctx, uo, vo, wo, g, r);
+        join(ctx, 3);
+        launch_implicit_uvw<real>(ctx, g, r);
+    } else {
+        launch_viscosity<real>(ctx, q_new<real>(ctx, VC), mu_new<real>(ctx));
+        launch_explicit<real, VU>(ctx, uo, vo, wo, g, r);
+        launch_implicit<real, VU>(ctx, g, r);
+        launch_explicit<real, VV>(ctx, uo, vo, wo, g, r);
+        launch_implicit<real, VV>(ctx, g, r);
+        launch_explicit<real, VW>(ctx, uo, vo, wo, g, r);
+        launch_implicit<real, VW>(ctx, g, r);
+    }
     // update_velo_boundary (L182) writes only ghost entries that nothing
     // reads before update_veloghost_points (L189) rewrites them; skipped
+    fork(ctx, 1);
+    on_side(ctx, 0);
     launch_flux<real>(ctx);
+    on_side(ctx, -1);
     launch_div<real>(ctx, 0, alpha);
     launch_poisson<real>(ctx);
     launch_phi_ghosts<real>(ctx);
+    join(ctx, 1);
     launch_project<real>(ctx, alpha, 1, 1, 1);
     ctx->cur ^= 1;  // update_old_*: roles swap
     if (ctx->resync_c) {
@@ -600,32 +697,11 @@ void enqueue_substep(pllgpu_ctx* ctx, int rk)
     }
 }
 
-__device__ __forceinline__ void k_tval_run(const uint3, const dim3, double* scal, double a0, double a1, double a2)
-{
-    // tval += (gamma+rho) dt per substep, pllcart3d.c:166
-    const double dt = scal[S_DT];
-    double t = scal[S_TVAL];
-    t = t + a0 * dt;
-    t = t + a1 * dt;
-    t = t + a2 * dt;
-    scal[S_TVAL] = t;
-}
-__global__ void k_tval(double* scal, double a0, double a1, double a2)
-{
-    k_tval_run(blockIdx, gridDim, scal, a0, a1, a2);
-}
-struct k_tval_b {
-    static constexpr auto run = &k_tval_run;
-    static constexpr int maxt = 0, minb = 0;
-};
-
 template <typename real>
 void enqueue_step(pllgpu_ctx* ctx)
 {
-    launch_cfl<real>(ctx);
+    launch_cfl<real>(ctx, {kRK1[0] + kRK2[0], kRK1[1] + kRK2[1], kRK1[2] + kRK2[2]});
     for (int rk = 0; rk < 3; ++rk) enqueue_substep<real>(ctx, rk);
-    go<k_tval_b>(ctx, k_tval, 1, 1, 0, ctx->scal, kRK1[0] + kRK2[0], kRK1[1] + kRK2[1], kRK1[2] + kRK2[2]);
-    mark(ctx, "tval");
 }
 
 template <typename real>
@@ -1018,10 +1094,12 @@ bool alloc_state(pllgpu_ctx* c)
     for (int v = 1; v < 4 && ok; ++v) ok = (B.pg[v] = dalloc<real>(c, c->nelem)) != nullptr;
     const long ncell = (long)p->nx * p->ny * p->nz;
     ok = ok && (B.phi = dalloc<real>(c, c->nelem)) && (B.div = dalloc<real>(c, c->nelem)) &&
-         (B.S = dalloc<real>(c, c->nelem)) && (B.cc = dalloc<real>(c, c->nelem)) &&
+         (B.S[VC] = dalloc<real>(c, c->nelem)) && (B.cc = dalloc<real>(c, c->nelem)) &&
          (B.dct1 = dalloc<real>(c, ncell)) && (B.dct2 = dalloc<real>(c, ncell)) &&
          (B.Ty = dalloc<real>(c, (long)p->ny * p->ny)) && (B.Tz = dalloc<real>(c, (long)p->nz * p->nz)) &&
          (B.Tiy = dalloc<real>(c, (long)p->ny * p->ny)) && (B.Tiz = dalloc<real>(c, (long)p->nz * p->nz));
+    B.S[VU] = B.S[VV] = B.S[VW] = B.S[VC];   // u's follows c's
+    if (ok && part_form<real>()) ok = (B.S[VV] = dalloc<real>(c, c->nelem)) && (B.S[VW] = dalloc<real>(c, c->nelem));
     if (!ok) return false;
     std::vector<real> T((size_t)std::max(p->ny, p->nz) * std::max(p->ny, p->nz));
     dct_matrix<real>(0, p->ny, T.data());

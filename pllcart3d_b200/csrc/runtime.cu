@@ -182,6 +182,15 @@ pllgpu_ctx* pllgpu_create(const pllgpu_params* p, int device)
         delete ctx;
         return nullptr;
     }
+    ctx->at = ctx->st;
+    bool sides = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) == cudaSuccess;
+    for (int i = 0; i < pllgpu_ctx::NSIDE && sides; ++i)
+        sides = cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking) == cudaSuccess &&
+                cudaEventCreateWithFlags(&ctx->ev_join[i], cudaEventDisableTiming) == cudaSuccess;
+    if (!sides) {
+        pllgpu_destroy(ctx);
+        return nullptr;
+    }
     Geo& G = ctx->G;
     G.nx = p->nx; G.ny = p->ny; G.nz = p->nz;
     G.NX = p->nx + 6; G.NY = p->ny + 2; G.NZ = p->nz + 2;
@@ -193,8 +202,7 @@ pllgpu_ctx* pllgpu_create(const pllgpu_params* p, int device)
     G.dz = (p->Z2 - p->Z1) / (double)p->nz;
     ctx->nelem = (long)G.NX * G.sx;
     if (ctx->nelem >= (1L << 31)) {   // kernels index a field with 32-bit offsets
-        cudaStreamDestroy(ctx->st);
-        delete ctx;
+        pllgpu_destroy(ctx);
         return nullptr;
     }
     // index ranges, simulation_setup pllcart3d.c:405-431 (one rank)
@@ -241,7 +249,7 @@ pllgpu_ctx* pllgpu_create(const pllgpu_params* p, int device)
          (c->lam_y = dalloc<double>(c, p->ny)) && (c->lam_z = dalloc<double>(c, p->nz)) &&
          (c->scal = dalloc<double>(c, S_COUNT)) && (c->work = dalloc<double>(c, 2L * (p->nx + 8))) &&
          (c->diag = dalloc<double>(c, 3L * p->nx + 8)) && (c->status = dalloc<int>(c, 1)) &&
-         (c->red = dalloc<double>(c, red_doubles(c->G))) && (c->ticket = dalloc<unsigned>(c, 2));
+         (c->red = dalloc<double>(c, red_doubles(c->G))) && (c->ticket = dalloc<unsigned>(c, 3));
     if (ok && ctx->mixed) ok = (c->stage64 = dalloc<double>(c, c->nelem)) != nullptr;
     if (!ok) {
         pllgpu_destroy(ctx);
@@ -282,6 +290,11 @@ void pllgpu_destroy(pllgpu_ctx* ctx)
         if (ctx->gexec[t]) cudaGraphExecDestroy(ctx->gexec[t]);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     for (void* p : ctx->allocs) cudaFree(p);
+    if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
+    for (cudaEvent_t e : ctx->ev_join)
+        if (e) cudaEventDestroy(e);
+    for (cudaStream_t s : ctx->side)
+        if (s) cudaStreamDestroy(s);
     if (ctx->st) cudaStreamDestroy(ctx->st);
     delete ctx;
 }

@@ -26,6 +26,8 @@ KERNEL_WORDS = {
     # x line solve + update: rhs, q_old (+ viscosity) ; q_new
     "adi_x_c": 3,
     "adi_x_u": 4, "adi_x_v": 4, "adi_x_w": 4,
+    # u, v and w in one launch
+    "adi_y_uvw": 9, "adi_z_uvw": 9, "adi_x_uvw": 12,
     "viscosity": 5,      # c ; 4 viscosity families
     "div_rhs": 4,        # u, v, w ; rhs
     "dct_gemm": 2,       # one dense pass: in ; out (per launch)
@@ -45,13 +47,14 @@ FAMILY = {
     "explicit_w": "k_explicit_tma",
     "adi_y_c": "k_line_seg (y)", "adi_y_u": "k_line_seg (y)", "adi_y_v": "k_line_seg (y)",
     "adi_y_w": "k_line_seg (y)",
+    "adi_y_uvw": "k_line_seg (y)", "adi_z_uvw": "k_adi_z_part", "adi_x_uvw": "k_line_seg (x)",
     "adi_z_c": "k_adi_z_part", "adi_z_u": "k_adi_z_part", "adi_z_v": "k_adi_z_part",
     "adi_z_w": "k_adi_z_part",
     "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
     "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_fft": "k_dct_fft",
     "dct_fold": "k_dct_fold",
-    "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl",
+    "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl2",
 }
 
 # the exact FP64 form's kernels where they differ (bit-reproducible order of
@@ -63,7 +66,7 @@ FAMILY_EXACT = dict(FAMILY, **{
     "adi_x_w": "k_line_pf (x)", "poisson_x": "k_poisson_x",
     "adi_z_c": "k_adi_z_tiled", "adi_z_u": "k_adi_z_tiled", "adi_z_v": "k_adi_z_tiled",
     "adi_z_w": "k_adi_z_tiled",
-    "viscosity": "k_viscosity", "div_rhs": "k_div_rhs", "dct_gemm": "k_gemm_dmma", "project": "k_project"})
+    "viscosity": "k_viscosity", "div_rhs": "k_div_rhs", "dct_gemm": "k_gemm_dmma", "project": "k_project", "cfl": "k_cfl"})
 
 # the precision form's kernels where they differ from the FP64 form's
 FAMILY_FP32 = {
@@ -71,6 +74,7 @@ FAMILY_FP32 = {
     "explicit_w": "k_explicit2",
     "adi_y_c": "k_line_seg (y)", "adi_y_u": "k_line_seg (y)", "adi_y_v": "k_line_seg (y)",
     "adi_y_w": "k_line_seg (y)",
+    "adi_y_uvw": "k_line_seg (y)", "adi_z_uvw": "k_adi_z_part", "adi_x_uvw": "k_line_seg (x)",
     "adi_z_c": "k_adi_z_part", "adi_z_u": "k_adi_z_part", "adi_z_v": "k_adi_z_part", "adi_z_w": "k_adi_z_part",
     "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
     "adi_x_w": "k_line_seg (x)",
