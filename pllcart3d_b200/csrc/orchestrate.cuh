@@ -93,11 +93,11 @@ bool launch_explicit_tma(pllgpu_ctx* ctx, const ExplicitArgs<real>& A)
     if (!field_map<real>(&M.q, A.q, ctx->G, GM::KB3, GM::JB3)) return false;
     for (int a = 0; a < XtSet<VAR>::NA; ++a)
         if (!field_map<real>(&M.a[a], staged[a], ctx->G, GM::KB1, GM::JB1)) return false;
-    const dim3 tiles((ctx->G.nz + XT_TK - 1) / XT_TK, (nj(R) + XT_TJ - 1) / XT_TJ);
+    const dim3 tiles((ctx->G.nz + XT_TK - 1) / XT_TK, (nj(R) + GM::TJ - 1) / GM::TJ);
     const int np = xt_planes((long)tiles.x * tiles.y, ni(R), ctx->xt_cap[VAR]);
     const dim3 grid(tiles.x, tiles.y, (ni(R) + np - 1) / np);
-    go<NoBatch>(ctx, k_explicit_tma<VAR, real>, grid, XT_THREADS, XtSmem<real, VAR>::DYN, M, ctx->G, R, ctx->K, A, np,
-                ctx->status);
+    go<k_explicit_tma_b<VAR, real>>(ctx, k_explicit_tma<VAR, real>, grid, XT_THREADS, XtSmem<real, VAR>::DYN, M, ctx->G,
+                                    R, ctx->K, xt_const<real>(VAR, ctx->K, A.g, A.r), A, np, ctx->status);
     return true;
 }
 
@@ -124,7 +124,7 @@ void launch_explicit(pllgpu_ctx* ctx, const real* un, const real* vn, const real
     int bx, by;
     tune_exp_block(ctx->tune_exp, bx, by);
     if constexpr (std::is_same<real, float>::value) {
-        if (ctx->P.explicit_kernel == 2 && !ctx->P.exact_dct && launch_explicit_tma<real, VAR>(ctx, A)) {
+        if (ctx->xt_on && ctx->P.explicit_kernel != 1 && launch_explicit_tma<real, VAR>(ctx, A)) {
             mark(ctx, lab[VAR]);
             return;
         }
@@ -1120,11 +1120,12 @@ bool alloc_state(pllgpu_ctx* c)
     cudaFuncSetAttribute(k_adi_z_tiled<VW, real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)adi_z_smem_bytes<VW, real>());
     if constexpr (std::is_same<real, float>::value) {
-        if (p->explicit_kernel == 2) {
+        if (!p->exact_dct && encode_tiled()) {
             xt_setup<VC, float>(c);
             xt_setup<VU, float>(c);
             xt_setup<VV, float>(c);
             xt_setup<VW, float>(c);
+            c->xt_on = true;
         }
         const bool shape_ok = (p->ny == 128 || p->ny == 256) && (p->nz == 128 || p->nz == 256);
         if (!p->exact_dct && p->dct_kernel != 1 && !(shape_ok ? setup_umma(c) : setup_dct_lines(c))) return false;

@@ -263,13 +263,15 @@ __device__ __forceinline__ float rcp_<float>(float x) { return __fdividef(1.0f, 
 // (5b-2a)/6, (b+2c)/6 and (4c-d)/6, the smoothness indicators (times 4)
 // 13/3 (b-a)^2 + (3b-a)^2, 13/3 (c-b)^2 + (b+c)^2 and 13/3 (d-c)^2 + (d-3c)^2
 // (calculate_weno, pllcart3d.c:3455-3507, expanded about v2), so the
-// derivative is v2 plus the weighted correction returned here, over h.  The
+// derivative is v2 plus the weighted correction (returned so), over h.  The
 // weights w_i / e_i^2 are multiplied by (e_1 e_2 e_3)^2: one division.  The
 // e_i are first brought to [1.5e-8, 2) by subtracting the largest one's
 // exponent from all three (eps >= 1e-6 max(v^2) and s_i <= 33 max(v^2) bound
 // their ratio), so that no product leaves the range.
 // vmax: max |v_i|; floor4: 4 x the reference's 1e-99 h^2 (FP32: 4e-36).
-__device__ __forceinline__ double weno_corr(double a, double b, double c, double d, double vmax, double floor4)
+// Every fusion is written out: batched copies must give the same bits.
+__device__ __forceinline__ double weno_diff(double v2, double a, double b, double c, double d, double vmax,
+                                            double floor4)
 {
     const double eps = fma(4.0e-6 * vmax, vmax, floor4);
     const double k = 13.0 / 3.0;
@@ -283,26 +285,33 @@ __device__ __forceinline__ double weno_corr(double a, double b, double c, double
     e2 = __hiloint2double(h2 + sh, __double2loint(e2));
     e3 = __hiloint2double(h3 + sh, __double2loint(e3));
     const double r23 = e2 * e3, r13 = e1 * e3, r12 = e1 * e2;
-    const double w1 = r23 * r23, w2 = 6.0 * (r13 * r13), w3 = 3.0 * (r12 * r12);
+    const double w1 = mul_rn_(r23, r23), w2 = mul_rn_(6.0 * r13, r13), w3 = mul_rn_(3.0 * r12, r12);
     const double num = fma(w3, fma(4.0, c, -d), fma(w2, fma(2.0, c, b), w1 * fma(5.0, b, -2.0 * a)));
-    return num * rcp_<double>(6.0 * (w1 + w2 + w3));
+    return fma(num, rcp_<double>(6.0 * (w1 + w2 + w3)), v2);
 }
 
-// the same in FP32 from the correction's own differences; the v_i are
-// re-formed from v2 (their rounding only enters eps)
+// The correction alone in FP32, from its own differences; the v_i are
+// re-formed from v2 (their rounding only enters eps).  max |v_i| is taken no
+// lower than 1e-15, which stands for the 1e-99, and its exponent, twice, is
+// what the e_i (4e-6 .. 528 times its square) are brought near 1 with.
+__device__ __forceinline__ int weno_shift(float vmax) { return (0x3f800000 - (__float_as_int(vmax) & 0x7f800000)) * 2; }
+__device__ __forceinline__ float weno_vmax(float v0, float v1, float v2, float v3, float v4)
+{
+    return fmaxf(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))), fmaxf(fabsf(v4), 1.0e-15f));
+}
 __device__ __forceinline__ float weno_corr(float v2, float a, float b, float c, float d)
 {
     const float v1 = v2 - b, v0 = v1 - a, v3 = v2 + c, v4 = v3 + d;
-    const float vmax = fmaxf(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))), fabsf(v4));
-    const float eps = fmaf(4.0e-6f * vmax, vmax, 4.0e-36f);
+    const float vmax = weno_vmax(v0, v1, v2, v3, v4);
+    const float eps = 4.0e-6f * vmax * vmax;
     const float k = (float)(13.0 / 3.0);
     const float p1 = b - a, q1 = fmaf(3.0f, b, -a), p2 = c - b, q2 = b + c, p3 = d - c, q3 = fmaf(-3.0f, c, d);
     const float e1 = fmaf(k * p1, p1, fmaf(q1, q1, eps));
     const float e2 = fmaf(k * p2, p2, fmaf(q2, q2, eps));
     const float e3 = fmaf(k * p3, p3, fmaf(q3, q3, eps));
-    const int h1 = __float_as_int(e1), h2 = __float_as_int(e2), h3 = __float_as_int(e3);
-    const int sh = 0x3f800000 - (max(max(h1, h2), h3) & 0x7f800000);
-    const float s1 = __int_as_float(h1 + sh), s2 = __int_as_float(h2 + sh), s3 = __int_as_float(h3 + sh);
+    const int sh = weno_shift(vmax);
+    const float s1 = __int_as_float(__float_as_int(e1) + sh), s2 = __int_as_float(__float_as_int(e2) + sh);
+    const float s3 = __int_as_float(__float_as_int(e3) + sh);
     const float r23 = s2 * s3, r13 = s1 * s3, r12 = s1 * s2;
     const float w1 = r23 * r23, w2 = 6.0f * (r13 * r13), w3 = 3.0f * (r12 * r12);
     const float num = fmaf(w3, fmaf(4.0f, c, -d), fmaf(w2, fmaf(2.0f, c, b), w1 * fmaf(5.0f, b, -2.0f * a)));
@@ -329,8 +338,13 @@ __device__ real stale_d2(const real* __restrict__ q, const Geo& G, const Rng& R,
             } else {
                 base = (long)R.ie * G.sx + R.ke; st = G.sy; h = K.hy; ih = K.ihy; i2h = K.i2hy;
             }
-            real d1m = over_h<real>(q[base + (long)(m + 1) * st] - q[base + (long)m * st], h, ih, K.pow2);
-            real d1p = over_h<real>(q[base + (long)m * st] - q[base + (long)(m - 1) * st], h, ih, K.pow2);
+            const real qm = q[base + (long)(m - 1) * st], q0 = q[base + (long)m * st], qp = q[base + (long)(m + 1) * st];
+#if !PLL_FP64_EXACT
+            // one product: nothing a compiler could fuse either way
+            if (sizeof(real) == 8) return ((qp - q0) - (q0 - qm)) * (real)(ih * i2h);
+#endif
+            real d1m = over_h<real>(qp - q0, h, ih, K.pow2);
+            real d1p = over_h<real>(q0 - qm, h, ih, K.pow2);
             return over_2h<real>(d1m - d1p, h, i2h, K.pow2);
         }
     }
@@ -631,6 +645,34 @@ template <>
 struct PairOf<double> {
     using type = d2;
 };
+
+// weno_corr of two cells in paired instructions.  A paired operand that is a
+// constant costs a register pair or two moves, so they are few: 5b - 2a =
+// 2 (3b - a) - b, b + 2c = (b + c) + c, 4c - d = c - (d - 3c), weights 1, 6, 3
+// as w1 + 3 (2 w2 + w3).
+__device__ __forceinline__ f2 weno_corr2(f2 v2, f2 a, f2 b, f2 c, f2 d)
+{
+    const f2 v1 = v2 - b, v0 = v1 - a, v3 = v2 + c, v4 = v3 + d;
+    const float mx = weno_vmax(v0.v.x, v1.v.x, v2.v.x, v3.v.x, v4.v.x);
+    const float my = weno_vmax(v0.v.y, v1.v.y, v2.v.y, v3.v.y, v4.v.y);
+    const f2 eps = F2(4.0e-6f * mx * mx, 4.0e-6f * my * my);
+    const f2 k = S2((float)(13.0 / 3.0)), three = S2(3.0f);
+    const f2 p1 = b - a, q1 = p1 + (b + b), p2 = c - b, q2 = b + c, p3 = d - c, q3 = p3 - (c + c);
+    const f2 e1 = fma2(k * p1, p1, fma2(q1, q1, eps));
+    const f2 e2 = fma2(k * p2, p2, fma2(q2, q2, eps));
+    const f2 e3 = fma2(k * p3, p3, fma2(q3, q3, eps));
+    const int sx = weno_shift(mx), sy = weno_shift(my);
+    auto near_one = [&](f2 e) {
+        return F2(__int_as_float(__float_as_int(e.v.x) + sx), __int_as_float(__float_as_int(e.v.y) + sy));
+    };
+    const f2 s1 = near_one(e1), s2 = near_one(e2), s3 = near_one(e3);
+    const f2 r23 = s2 * s3, r13 = s1 * s3, r12 = s1 * s2;
+    const f2 w1 = r23 * r23, h2 = r13 * r13, w2 = h2 + h2, w3 = r12 * r12;
+    const f2 num = fma2(three, fma2(w3, c - q3, w2 * (q2 + c)), w1 * ((q1 + q1) - b));
+    const f2 den = fma2(three, w2 + w3, w1);
+    const float sixth = (float)(1.0 / 6.0);
+    return F2(__fdividef(num.v.x * sixth, den.v.x), __fdividef(num.v.y * sixth, den.v.y));
+}
 
 // packed weno5<float>: the same weights with the approximate divisions per
 // component
