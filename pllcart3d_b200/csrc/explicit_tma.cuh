@@ -535,7 +535,7 @@ __global__ void __launch_bounds__(XT_THREADS, XtBlocks<VAR, real>::value)
 template <int VAR, typename real>
 struct k_explicit_tma_b {
     static constexpr auto run = &k_explicit_tma_run<VAR, real>;
-    static constexpr int maxt = XT_THREADS, minb = 0;
+    static constexpr int maxt = XT_THREADS, minb = 0, bminb = sizeof(real) == 4 ? 2 : 0;
 };
 
 }  // namespace
