@@ -151,12 +151,14 @@ __global__ void __launch_bounds__(128) k_viscosity2(Geo G, Rng R, Consts K, cons
                                                     real* __restrict__ mc, real* __restrict__ mxy,
                                                     real* __restrict__ mxz, real* __restrict__ myz)
 {
+    if (!after_previous()) return;
     k_viscosity2_run<real>(blockIdx, gridDim, G, R, K, cn, mc, mxy, mxz, myz);
 }
 template <typename real>
 struct k_viscosity2_b {
     static constexpr auto run = &k_viscosity2_run<real>;
     static constexpr int maxt = 128, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // Last-block ticket: every block's results are written and fenced before it
@@ -342,12 +344,14 @@ __global__ void __launch_bounds__(128) k_div_rhs2(Geo G, Rng R, Consts K, const 
                                                   real* __restrict__ rhs, const double* __restrict__ scal,
                                                   double alpha)
 {
+    if (!after_previous()) return;
     k_div_rhs2_run<real>(blockIdx, gridDim, G, R, K, u, v, w, rhs, scal, alpha);
 }
 template <typename real>
 struct k_div_rhs2_b {
     static constexpr auto run = &k_div_rhs2_run<real>;
     static constexpr int maxt = 128, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // The CFL scan outside the exact form: cell pairs (k, k+32), CFL_NI planes per
@@ -416,12 +420,14 @@ __global__ void __launch_bounds__(256) k_cfl2(Geo G, Rng R, Consts K, const real
                                               const real* __restrict__ v, const real* __restrict__ w, double* scal,
                                               int* status, unsigned* ticket, StepTime a)
 {
+    if (!after_previous()) return;
     k_cfl2_run<real>(blockIdx, gridDim, G, R, K, u, v, w, scal, status, ticket, a);
 }
 template <typename real>
 struct k_cfl2_b {
     static constexpr auto run = &k_cfl2_run<real>;
     static constexpr int maxt = 256, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // The inflow/outflow fluxes outside the exact form: the trapezoid sums of k_flux
@@ -472,12 +478,14 @@ template <typename real>
 __global__ void __launch_bounds__(1024) k_flux3(Geo G, Rng Ru, Consts K, const real* __restrict__ u, double* red,
                                                 unsigned* ticket, double* scal)
 {
+    if (!after_previous()) return;
     k_flux3_run<real>(blockIdx, gridDim, G, Ru, K, u, red, ticket, scal);
 }
 template <typename real>
 struct k_flux3_b {
     static constexpr auto run = &k_flux3_run<real>;
     static constexpr int maxt = 1024, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // bulk_velo (pllcart3d.c:3381-3398): the signed value of the first (j-major,
@@ -551,12 +559,14 @@ template <typename real>
 __global__ void __launch_bounds__(1024) k_bulk2(Geo G, Rng R, const real* __restrict__ u, double* red,
                                                unsigned* ticket, double* scal)
 {
+    if (!after_previous()) return;
     k_bulk2_run<real>(blockIdx, gridDim, G, R, u, red, ticket, scal);
 }
 template <typename real>
 struct k_bulk2_b {
     static constexpr auto run = &k_bulk2_run<real>;
     static constexpr int maxt = 1024, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // divergence (pllcart3d.c:1983-1999) scaled by Re/(dt alpha)
@@ -756,12 +766,14 @@ __device__ __forceinline__ void k_phi_ghosts_run(const uint3 blockIdx, const dim
 template <typename real>
 __global__ void k_phi_ghosts(Geo G, Rng R, real* __restrict__ p)
 {
+    if (!after_previous()) return;
     k_phi_ghosts_run<real>(blockIdx, gridDim, G, R, p);
 }
 template <typename real>
 struct k_phi_ghosts_b {
     static constexpr auto run = &k_phi_ghosts_run<real>;
     static constexpr int maxt = 0, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // planes of i one k_project thread walks
@@ -1005,6 +1017,7 @@ __global__ void __launch_bounds__(128, sizeof(real) == 4 ? 16 : 8) k_project2(Ge
         const real* __restrict__ phi, MuPtrs<real> mu, const double* __restrict__ scal,
         double alpha, int do_correct, int do_ghosts, int do_pg)
 {
+    if (!after_previous()) return;
     k_project2_run<real>(blockIdx, gridDim, G, Rg, Ru, Rv, Rw, K, u, v, w, pgu, pgv, pgw, phi, mu, scal, alpha,
                          do_correct, do_ghosts, do_pg);
 }
@@ -1012,6 +1025,7 @@ template <typename real>
 struct k_project2_b {
     static constexpr auto run = &k_project2_run<real>;
     static constexpr int maxt = 128, minb = sizeof(real) == 4 ? 16 : 8, bminb = 8;
+    static constexpr bool chained = true;
 };
 
 // slope_parameter (pllcart3d.c:722-840) on one rank: bisection for the

@@ -31,6 +31,24 @@ struct Phys {
     int nmvp;
 };
 
+// A kernel that begins with this may be let onto the chip while the launch
+// before it on its stream drains (programmatic dependent launch): its blocks
+// wait here, in hardware, until that launch has completed and its stores are
+// visible, and let the next one in as soon as they are all placed.  What is
+// hidden is the launch latency between dependent kernels, about 1 us each: on
+// small grids a step is a chain of 45 kernels of 3 to 7 us.  The answer is
+// always true; the branch on it keeps read-only loads from moving above it.
+__device__ __forceinline__ bool after_previous()
+{
+    unsigned sm;
+    asm volatile(
+        "griddepcontrol.wait;\n\t"
+        "griddepcontrol.launch_dependents;\n\t"
+        "mov.u32 %0, %%smid;"
+        : "=r"(sm)::"memory");
+    return sm != 0xffffffffu;
+}
+
 enum Var { VC = 0, VU = 1, VV = 2, VW = 3 };
 
 // device scalar slots (one small array per context)

@@ -75,6 +75,8 @@ struct pllgpu_ctx {
     static constexpr int NSIDE = 3;
     cudaStream_t side[NSIDE] = {}, at = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join[NSIDE] = {};
+    bool follows[1 + NSIDE] = {};   // the last thing enqueued on st, side[i] is a kernel of the step
+    bool chaining = false;          // a whole step is being enqueued
     long nelem = 0;             // elements of one padded field
     Bufs<double> b64;           // state of the FP64 form
     Bufs<float> b32;            // state of the mixed form

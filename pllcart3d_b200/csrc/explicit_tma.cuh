@@ -528,6 +528,7 @@ __global__ void __launch_bounds__(XT_THREADS, XtBlocks<VAR, real>::value)
     k_explicit_tma(const __grid_constant__ XtMaps maps, Geo G, Rng R, Consts K, XtConst<real> C, ExplicitArgs<real> A,
                    int ni, int* status)
 {
+    if (!after_previous()) return;
     k_explicit_tma_run<VAR, real>(blockIdx, gridDim, maps, G, R, K, C, A, ni, status);
 }
 // a batched copy takes its tensor maps where they lie, in the argument table
@@ -536,6 +537,7 @@ template <int VAR, typename real>
 struct k_explicit_tma_b {
     static constexpr auto run = &k_explicit_tma_run<VAR, real>;
     static constexpr int maxt = XT_THREADS, minb = 0, bminb = sizeof(real) == 4 ? 2 : 0;
+    static constexpr bool chained = true;
 };
 
 }  // namespace

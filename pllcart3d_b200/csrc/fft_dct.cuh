@@ -290,12 +290,14 @@ __global__ void __launch_bounds__(FFT_THREADS) k_dct_fft(FftLines d, const T* __
                                                          const double2* __restrict__ tw,
                                                          const double2* __restrict__ wq)
 {
+    if (!after_previous()) return;
     k_dct_fft_run<T, N, KIND, CONTIG, WHOLE>(blockIdx, gridDim, d, in, out, tw, wq);
 }
 template <typename T, int N, int KIND, bool CONTIG, bool WHOLE>
 struct k_dct_fft_b {
     static constexpr auto run = &k_dct_fft_run<T, N, KIND, CONTIG, WHOLE>;
     static constexpr int maxt = FFT_THREADS, minb = 0;
+    static constexpr bool chained = true;
 };
 
 }  // namespace

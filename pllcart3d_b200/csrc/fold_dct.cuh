@@ -154,12 +154,14 @@ template <int KIND, bool CONTIG, typename T>
 __global__ void __launch_bounds__(256) k_dct_fold(FftLines d, int n, const T* __restrict__ in, T* __restrict__ out,
                                                   const double* __restrict__ table)
 {
+    if (!after_previous()) return;
     k_dct_fold_run<KIND, CONTIG, T>(blockIdx, gridDim, d, n, in, out, table);
 }
 template <int KIND, bool CONTIG, typename T>
 struct k_dct_fold_b {
     static constexpr auto run = &k_dct_fold_run<KIND, CONTIG, T>;
     static constexpr int maxt = 256, minb = 0;
+    static constexpr bool chained = true;
 };
 
 }  // namespace

@@ -25,6 +25,19 @@ int fail(pllgpu_ctx* c, int code)
         }                                                                            \
     } while (0)
 
+// Side branches of the step.  fork(n) lets side streams 0 .. n-1 start after
+// everything enqueued so far, on_side(i) sends the following launches there
+// (on_side(-1): back to the main stream), join(n) makes the main stream wait
+// for them.  A step recorded for an ensemble, or profiled launch by launch, has
+// no branches: its launches stay in order.
+bool branches(const pllgpu_ctx* c) { return !c->rec && !c->profiling; }
+
+// whether a spec's own kernel (not its batched copy) begins with after_previous()
+template <typename B, typename = void>
+struct Chained : std::false_type {};
+template <typename B>
+struct Chained<B, std::void_t<decltype(B::chained)>> : std::bool_constant<B::chained> {};
+
 // every kernel launch of the step: launched, or recorded while the context
 // records (B: the kernel's batching spec, NoBatch where it has none)
 template <typename B, typename... P, typename... A>
@@ -41,21 +54,32 @@ void go(pllgpu_ctx* ctx, void (*k)(P...), dim3 grid, dim3 blk, size_t smem, A&&.
         ctx->rec->push_back(r);
         return;
     }
-    k<<<grid, blk, smem, ctx->at>>>(std::forward<A>(a)...);
+    // On the same stream as the launch before it, a kernel that begins with
+    // after_previous() is let in while that one still drains.
+    const int at = ctx->at == ctx->st ? 0 : ctx->at == ctx->side[0] ? 1 : ctx->at == ctx->side[1] ? 2 : 3;
+    const bool early = Chained<B>::value && ctx->chaining && ctx->follows[at] && branches(ctx);
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = blk;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = ctx->at;
+    cfg.attrs = &attr;
+    cfg.numAttrs = early ? 1 : 0;
+    if (cudaLaunchKernelEx(&cfg, k, static_cast<P>(std::forward<A>(a))...) != cudaSuccess) fail(ctx, PLLGPU_ECUDA);
+    ctx->follows[at] = true;
 }
-
-// Side branches of the step.  fork(n) lets side streams 0 .. n-1 start after
-// everything enqueued so far, on_side(i) sends the following launches there
-// (on_side(-1): back to the main stream), join(n) makes the main stream wait
-// for them.  A step recorded for an ensemble, or profiled launch by launch, has
-// no branches: its launches stay in order.
-bool branches(const pllgpu_ctx* c) { return !c->rec && !c->profiling; }
 
 void fork(pllgpu_ctx* ctx, int n)
 {
     if (!branches(ctx)) return;
     bool ok = cudaEventRecord(ctx->ev_fork, ctx->st) == cudaSuccess;
-    for (int i = 0; i < n && ok; ++i) ok = cudaStreamWaitEvent(ctx->side[i], ctx->ev_fork, 0) == cudaSuccess;
+    for (int i = 0; i < n && ok; ++i) {
+        ok = cudaStreamWaitEvent(ctx->side[i], ctx->ev_fork, 0) == cudaSuccess;
+        ctx->follows[1 + i] = false;
+    }
     if (!ok) fail(ctx, PLLGPU_ECUDA);
 }
 
@@ -68,6 +92,7 @@ void join(pllgpu_ctx* ctx, int n)
 {
     if (!branches(ctx)) return;
     ctx->at = ctx->st;
+    ctx->follows[0] = false;
     bool ok = true;
     for (int i = 0; i < n && ok; ++i)
         ok = cudaEventRecord(ctx->ev_join[i], ctx->side[i]) == cudaSuccess &&

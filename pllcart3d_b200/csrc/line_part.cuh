@@ -345,12 +345,14 @@ template <int VAR, int AXIS, typename real, int E, int L, int TL>
 __global__ void __launch_bounds__(LinePart<VAR, AXIS, real, E, L, TL>::T)
     k_line_seg(Geo G, Rng R, Consts K, XsweepArgs<real> A)
 {
+    if (!after_previous()) return;
     k_line_seg_run<VAR, AXIS, real, E, L, TL>(blockIdx, gridDim, G, R, K, A);
 }
 template <int VAR, int AXIS, typename real, int E, int L, int TL>
 struct k_line_seg_b {
     static constexpr auto run = &k_line_seg_run<VAR, AXIS, real, E, L, TL>;
     static constexpr int maxt = LinePart<VAR, AXIS, real, E, L, TL>::T, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // the three momentum components' lines in one launch, component VU + blockIdx.z
@@ -370,12 +372,14 @@ __device__ __forceinline__ void k_line_seg3_run(const uint3 blockIdx, const dim3
 template <int AXIS, typename real, int E, int L, int TL>
 __global__ void __launch_bounds__(LinePart<VU, AXIS, real, E, L, TL>::T) k_line_seg3(Geo G, Consts K, Sweeps3<real> S)
 {
+    if (!after_previous()) return;
     k_line_seg3_run<AXIS, real, E, L, TL>(blockIdx, gridDim, G, K, S);
 }
 template <int AXIS, typename real, int E, int L, int TL>
 struct k_line_seg3_b {
     static constexpr auto run = &k_line_seg3_run<AXIS, real, E, L, TL>;
     static constexpr int maxt = LinePart<VU, AXIS, real, E, L, TL>::T, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // ---- z lines ---------------------------------------------------------------------
@@ -442,12 +446,14 @@ template <int VAR, typename real, int E, int L>
 __global__ void __launch_bounds__(128) k_adi_z_part(Geo G, Rng R, Consts K, MuPtrs<real> mu, real* __restrict__ S,
                                                     const double* __restrict__ scal, double alpha)
 {
+    if (!after_previous()) return;
     k_adi_z_part_run<VAR, real, E, L>(blockIdx, gridDim, G, R, K, mu, S, scal, alpha);
 }
 template <int VAR, typename real, int E, int L>
 struct k_adi_z_part_b {
     static constexpr auto run = &k_adi_z_part_run<VAR, real, E, L>;
     static constexpr int maxt = 128, minb = 0;
+    static constexpr bool chained = true;
 };
 
 template <typename real, int E, int L>
@@ -466,12 +472,14 @@ __device__ __forceinline__ void k_adi_z_part3_run(const uint3 blockIdx, const di
 template <typename real, int E, int L>
 __global__ void __launch_bounds__(128) k_adi_z_part3(Geo G, Consts K, Sweeps3<real> S)
 {
+    if (!after_previous()) return;
     k_adi_z_part3_run<real, E, L>(blockIdx, gridDim, G, K, S);
 }
 template <typename real, int E, int L>
 struct k_adi_z_part3_b {
     static constexpr auto run = &k_adi_z_part3_run<real, E, L>;
     static constexpr int maxt = 128, minb = 0;
+    static constexpr bool chained = true;
 };
 
 // ---- Poisson modes ---------------------------------------------------------------
@@ -641,12 +649,14 @@ __global__ void __launch_bounds__(PoissonPart<T, E, L, TL>::TH)
     k_poisson_part(int nx, int ny, int nz, Consts K, const double* __restrict__ lam_y,
                    const double* __restrict__ lam_z, T* __restrict__ hat, int kz_major)
 {
+    if (!after_previous()) return;
     k_poisson_part_run<T, E, L, TL>(blockIdx, gridDim, nx, ny, nz, K, lam_y, lam_z, hat, kz_major);
 }
 template <typename T, int E, int L, int TL>
 struct k_poisson_part_b {
     static constexpr auto run = &k_poisson_part_run<T, E, L, TL>;
     static constexpr int maxt = PoissonPart<T, E, L, TL>::TH, minb = 0;
+    static constexpr bool chained = true;
 };
 
 }  // namespace
