@@ -223,7 +223,7 @@ __device__ __forceinline__ bool eno_band(const Rng& R, int m)
 }
 
 // The upwind-sense difference of one cell from the window's differences
-// v0 .. v4 (v2 behind the point; only the FP64 weights read the others) and
+// v0 .. v4 (v2 behind the point; with FP32 weights a FP64 cell re-forms the others) and
 // their own a, b, c, d: ENO-2 in the band at the ends of a range, else WENO5
 // in the form's weight type.
 template <int AXIS, typename real>
@@ -250,7 +250,7 @@ __device__ __forceinline__ double xt_diffs(const double* v, double v0, double a,
     return xt_diff<AXIS, double>(v0, v[0], v[1], v[2], v[3], a, b, c, d, qg, G, R, K, m, up.a, floor4);
 }
 template <int AXIS>
-__device__ __forceinline__ f2 xt_diffs(const f2* v, f2, f2 a, f2 b, f2 c, f2 d, const float* __restrict__ qg,
+__device__ __forceinline__ f2 xt_diffs(const f2* v, f2 v0, f2 a, f2 b, f2 c, f2 d, const float* __restrict__ qg,
                                        const Geo& G, const Rng& R, const Consts& K, int m, XtUp up, float)
 {
     const int m2 = AXIS == 1 ? m + XT_WJ : m;
@@ -258,7 +258,9 @@ __device__ __forceinline__ f2 xt_diffs(const f2* v, f2, f2 a, f2 b, f2 c, f2 d, 
         return F2(xt_diff<AXIS, float>(0.f, 0.f, v[1].v.x, 0.f, 0.f, a.v.x, b.v.x, c.v.x, d.v.x, qg, G, R, K, m, up.a, 0.f),
                   xt_diff<AXIS, float>(0.f, 0.f, v[1].v.y, 0.f, 0.f, a.v.y, b.v.y, c.v.y, d.v.y, qg, G, R, K, m2, up.b,
                                        0.f));
-    return v[1] + weno_corr2(v[1], a, b, c, d);
+    const float mx = weno_vmax(v0.v.x, v[0].v.x, v[1].v.x, v[2].v.x, v[3].v.x);
+    const float my = weno_vmax(v0.v.y, v[0].v.y, v[1].v.y, v[2].v.y, v[3].v.y);
+    return v[1] + weno_corr2(mx, my, a, b, c, d);
 }
 
 __device__ __forceinline__ double xt_window(const double* p, int st, XtUp up, int t, long)

@@ -290,15 +290,32 @@ __device__ __forceinline__ double weno_diff(double v2, double a, double b, doubl
     return fma(num, rcp_<double>(6.0 * (w1 + w2 + w3)), v2);
 }
 
-// The correction alone in FP32, from its own differences; the v_i are
-// re-formed from v2 (their rounding only enters eps).  max |v_i| is taken no
-// lower than 1e-15, which stands for the 1e-99, and its exponent, twice, is
-// what the e_i (4e-6 .. 528 times its square) are brought near 1 with.
-__device__ __forceinline__ int weno_shift(float vmax) { return (0x3f800000 - (__float_as_int(vmax) & 0x7f800000)) * 2; }
+// The correction alone in FP32, from its own differences.  max |v_i| is taken
+// no lower than 1e-15, which stands for the 1e-99, and the e_i (4e-6 .. 528
+// times its square) are brought near 1 by the power of two of its exponent,
+// twice.
+__device__ __forceinline__ float weno_scale(float vmax)
+{
+    return __int_as_float(0x3f800000 + (0x3f800000 - (__float_as_int(vmax) & 0x7f800000)) * 2);
+}
+__device__ __forceinline__ float max3_abs(float a, float b, float c)
+{
+    float d;
+    asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
 __device__ __forceinline__ float weno_vmax(float v0, float v1, float v2, float v3, float v4)
 {
-    return fmaxf(fmaxf(fmaxf(fabsf(v0), fabsf(v1)), fmaxf(fabsf(v2), fabsf(v3))), fmaxf(fabsf(v4), 1.0e-15f));
+    return max3_abs(max3_abs(v0, v1, v2), max3_abs(v3, v4, 1.0e-15f), 0.0f);
 }
+// num / den for den in the normal range: the hardware's reciprocal (1 ulp)
+__device__ __forceinline__ float weno_ratio(float num, float den)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(den));
+    return num * r;
+}
+// (the v_i are re-formed from v2: their rounding only enters eps)
 __device__ __forceinline__ float weno_corr(float v2, float a, float b, float c, float d)
 {
     const float v1 = v2 - b, v0 = v1 - a, v3 = v2 + c, v4 = v3 + d;
@@ -309,13 +326,12 @@ __device__ __forceinline__ float weno_corr(float v2, float a, float b, float c, 
     const float e1 = fmaf(k * p1, p1, fmaf(q1, q1, eps));
     const float e2 = fmaf(k * p2, p2, fmaf(q2, q2, eps));
     const float e3 = fmaf(k * p3, p3, fmaf(q3, q3, eps));
-    const int sh = weno_shift(vmax);
-    const float s1 = __int_as_float(__float_as_int(e1) + sh), s2 = __int_as_float(__float_as_int(e2) + sh);
-    const float s3 = __int_as_float(__float_as_int(e3) + sh);
+    const float f = weno_scale(vmax);
+    const float s1 = e1 * f, s2 = e2 * f, s3 = e3 * f;
     const float r23 = s2 * s3, r13 = s1 * s3, r12 = s1 * s2;
     const float w1 = r23 * r23, w2 = 6.0f * (r13 * r13), w3 = 3.0f * (r12 * r12);
     const float num = fmaf(w3, fmaf(4.0f, c, -d), fmaf(w2, fmaf(2.0f, c, b), w1 * fmaf(5.0f, b, -2.0f * a)));
-    return __fdividef(num, 6.0f * (w1 + w2 + w3));
+    return weno_ratio(num, 6.0f * (w1 + w2 + w3));
 }
 
 // D2 value an earlier directional pass of the same H*_op call left in its
@@ -646,32 +662,26 @@ struct PairOf<double> {
     using type = d2;
 };
 
-// weno_corr of two cells in paired instructions.  A paired operand that is a
-// constant costs a register pair or two moves, so they are few: 5b - 2a =
-// 2 (3b - a) - b, b + 2c = (b + c) + c, 4c - d = c - (d - 3c), weights 1, 6, 3
-// as w1 + 3 (2 w2 + w3).
-__device__ __forceinline__ f2 weno_corr2(f2 v2, f2 a, f2 b, f2 c, f2 d)
+// weno_corr of two cells in paired instructions, their max |v_i| given.  A
+// paired operand that is a constant costs a register pair or two moves, so
+// they are few: 5b - 2a = 2 (3b - a) - b, b + 2c = (b + c) + c, 4c - d =
+// c - (d - 3c), weights 1, 6, 3 as w1 + 3 (2 w2 + w3).
+__device__ __forceinline__ f2 weno_corr2(float mx, float my, f2 a, f2 b, f2 c, f2 d)
 {
-    const f2 v1 = v2 - b, v0 = v1 - a, v3 = v2 + c, v4 = v3 + d;
-    const float mx = weno_vmax(v0.v.x, v1.v.x, v2.v.x, v3.v.x, v4.v.x);
-    const float my = weno_vmax(v0.v.y, v1.v.y, v2.v.y, v3.v.y, v4.v.y);
     const f2 eps = F2(4.0e-6f * mx * mx, 4.0e-6f * my * my);
     const f2 k = S2((float)(13.0 / 3.0)), three = S2(3.0f);
     const f2 p1 = b - a, q1 = p1 + (b + b), p2 = c - b, q2 = b + c, p3 = d - c, q3 = p3 - (c + c);
     const f2 e1 = fma2(k * p1, p1, fma2(q1, q1, eps));
     const f2 e2 = fma2(k * p2, p2, fma2(q2, q2, eps));
     const f2 e3 = fma2(k * p3, p3, fma2(q3, q3, eps));
-    const int sx = weno_shift(mx), sy = weno_shift(my);
-    auto near_one = [&](f2 e) {
-        return F2(__int_as_float(__float_as_int(e.v.x) + sx), __int_as_float(__float_as_int(e.v.y) + sy));
-    };
-    const f2 s1 = near_one(e1), s2 = near_one(e2), s3 = near_one(e3);
+    const f2 f = F2(weno_scale(mx), weno_scale(my));
+    const f2 s1 = e1 * f, s2 = e2 * f, s3 = e3 * f;
     const f2 r23 = s2 * s3, r13 = s1 * s3, r12 = s1 * s2;
     const f2 w1 = r23 * r23, h2 = r13 * r13, w2 = h2 + h2, w3 = r12 * r12;
     const f2 num = fma2(three, fma2(w3, c - q3, w2 * (q2 + c)), w1 * ((q1 + q1) - b));
     const f2 den = fma2(three, w2 + w3, w1);
     const float sixth = (float)(1.0 / 6.0);
-    return F2(__fdividef(num.v.x * sixth, den.v.x), __fdividef(num.v.y * sixth, den.v.y));
+    return F2(weno_ratio(num.v.x * sixth, den.v.x), weno_ratio(num.v.y * sixth, den.v.y));
 }
 
 // packed weno5<float>: the same weights with the approximate divisions per
