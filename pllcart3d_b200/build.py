@@ -46,7 +46,7 @@ CU_SOURCES = {"runtime.cu": "--fmad=false", "form_f64.cu": "--fmad=true", "form_
               "wave.cu": "--fmad=false", "ensemble.cu": "--fmad=false"}
 HEADERS = ["common.cuh", "step_kernels.cuh", "aux_kernels.cuh", "dct_kernels.cuh", "host_util.h",
            "ctx.cuh", "host_common.cuh", "orchestrate.cuh", "forms.h", "umma_dct.cuh", "fft_dct.cuh", "explicit_tma.cuh",
-           "line_part.cuh", "fold_dct.cuh",
+           "line_part.cuh", "fold_dct.cuh", "plane_dct.cuh",
            "batch.cuh"]
 
 

@@ -55,6 +55,7 @@ struct UmmaPlan {
 struct DctAxis {
     enum Mode { NONE, FFT, FOLD } mode = NONE;
     double2 *tw = nullptr, *wq = nullptr;
+    int r1 = 0, r2 = 0;   // FFT: the length's two factors
     double* table[2] = {nullptr, nullptr};
 };
 
@@ -84,6 +85,8 @@ struct pllgpu_ctx {
     double* stage64 = nullptr;  // one padded FP64 field (mixed-form transfers)
     double *lam_y = nullptr, *lam_z = nullptr;
     DctAxis dct[2];             // the DCT passes along y and z
+    bool planes = false;        // ... both at once, plane by plane (plane_dct.cuh)
+    double *lam_py = nullptr, *lam_pz = nullptr;   // lam_y, lam_z in the planes' mode order
     bool xt_on = false;         // FP64 form: TMA-staged marching explicit operator
     int xt_cap[4] = {};         // its blocks resident at once, per variable
     UmmaPlan um;                // precision form's tensor-core DCT (when shapes allow)

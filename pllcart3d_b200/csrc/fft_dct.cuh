@@ -24,6 +24,8 @@
 
 #include <cuda_runtime.h>
 
+#include "step_kernels.cuh"
+
 namespace pll {
 namespace {
 
@@ -39,7 +41,11 @@ __device__ __forceinline__ cplx<real> csub(cplx<real> a, cplx<real> b) { return 
 template <typename real>
 __device__ __forceinline__ cplx<real> cmul(cplx<real> a, real c, real s)   // a * (c + i s)
 {
+#if PLL_FP64_EXACT   // units without contraction fuse by hand; the compiler's fuses with the sums around it too
+    return {fma(a.re, c, -(a.im * s)), fma(a.re, s, a.im * c)};
+#else
     return {a.re * c - a.im * s, a.re * s + a.im * c};
+#endif
 }
 
 // cos / sin of 2 pi m / 16, m = 0 .. 4 (the twiddles of DFTs up to 16 points)

@@ -15,6 +15,7 @@
 #include "explicit_tma.cuh"
 #include "fft_dct.cuh"
 #include "fold_dct.cuh"
+#include "plane_dct.cuh"
 #include "forms.h"
 #include "host_common.cuh"
 #include "line_part.cuh"
@@ -231,30 +232,30 @@ void z_part3(pllgpu_ctx* ctx, const Sweeps3<real>& S)
 }
 
 template <typename T, int E, int L, int TL>
-void poisson_part(pllgpu_ctx* ctx, T* hat, int kz_major)
+void poisson_part(pllgpu_ctx* ctx, T* hat, int kz_major, const double* ly, const double* lz)
 {
     using PP = PoissonPart<T, E, L, TL>;
     const int N = ctx->G.ny * ctx->G.nz;
     if (PP::SMEM > 48 * 1024)
         cudaFuncSetAttribute(k_poisson_part<T, E, L, TL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PP::SMEM);
     go<k_poisson_part_b<T, E, L, TL>>(ctx, k_poisson_part<T, E, L, TL>, (N + TL - 1) / TL, PP::TH, PP::SMEM, ctx->G.nx,
-                                      ctx->G.ny, ctx->G.nz, ctx->K, ctx->lam_y, ctx->lam_z, hat, kz_major);
+                                      ctx->G.ny, ctx->G.nz, ctx->K, ly, lz, hat, kz_major);
 }
 
 // the x-tridiagonal of every Poisson mode, in place
 template <typename T>
-void launch_modes(pllgpu_ctx* ctx, T* hat, int kz_major)
+void launch_modes(pllgpu_ctx* ctx, T* hat, int kz_major, const double* ly, const double* lz)
 {
     const int nx = ctx->G.nx, N = ctx->G.ny * ctx->G.nz;
     constexpr int TL = 8;
     if (ctx->P.exact_dct || nx > LINE_PART_MAX)
-        go<k_poisson_x_b<T>>(ctx, k_poisson_x<T>, (N + 127) / 128, 128, 0, nx, ctx->G.ny, ctx->G.nz, ctx->K, ctx->lam_y,
-                             ctx->lam_z, hat, ctx->mode_cc, ctx->mode_rr, kz_major);
-    else if (nx <= 32) poisson_part<T, 8, 4, TL>(ctx, hat, kz_major);
-    else if (nx <= 64) poisson_part<T, 8, 8, TL>(ctx, hat, kz_major);
-    else if (nx <= 128) poisson_part<T, 8, 16, TL>(ctx, hat, kz_major);
-    else if (nx <= 256) poisson_part<T, 8, 32, TL>(ctx, hat, kz_major);
-    else poisson_part<T, 16, 32, TL>(ctx, hat, kz_major);
+        go<k_poisson_x_b<T>>(ctx, k_poisson_x<T>, (N + 127) / 128, 128, 0, nx, ctx->G.ny, ctx->G.nz, ctx->K, ly,
+                             lz, hat, ctx->mode_cc, ctx->mode_rr, kz_major);
+    else if (nx <= 32) poisson_part<T, 8, 4, TL>(ctx, hat, kz_major, ly, lz);
+    else if (nx <= 64) poisson_part<T, 8, 8, TL>(ctx, hat, kz_major, ly, lz);
+    else if (nx <= 128) poisson_part<T, 8, 16, TL>(ctx, hat, kz_major, ly, lz);
+    else if (nx <= 256) poisson_part<T, 8, 32, TL>(ctx, hat, kz_major, ly, lz);
+    else poisson_part<T, 16, 32, TL>(ctx, hat, kz_major, ly, lz);
     mark(ctx, "poisson_x");
 }
 
@@ -424,7 +425,7 @@ void launch_poisson_umma(pllgpu_ctx* ctx)
     launch_umma(ctx, 0, (long)nx * ny, nz, UmmaEpi{ny, N, 1, ny, 1.f, 0, 1}, B.dct2);
     // forward y: dct1[x][kz][ky] = sum_y dct2[x][kz][y] Ty[ky][y]
     launch_umma(ctx, 1, (long)nx * nz, ny, UmmaEpi{nz, N, ny, 1, 1.f, 0, 0}, B.dct1);
-    launch_modes<float>(ctx, B.dct1, 1);
+    launch_modes<float>(ctx, B.dct1, 1, ctx->lam_y, ctx->lam_z);
     // inverse y: dct2[x][y][kz] = sum_ky dct1[x][kz][ky] Tiy[y][ky] (stored transposed)
     launch_umma(ctx, 2, (long)nx * nz, ny, UmmaEpi{nz, N, 1, nz, 1.f, 0, 1}, B.dct2);
     // inverse z into phi's interior, divided by 4*ny*nz
@@ -488,7 +489,7 @@ void launch_poisson_lines(pllgpu_ctx* ctx)
     const FftLines zlines{nx * ny, ny, N, nz, 1, N, nz, 1, 1.0};
     dct_pass<T, 0, false>(ctx, ny, ylines, B.dct1, B.dct2);
     dct_pass<T, 0, true>(ctx, nz, zlines, B.dct2, B.dct1);
-    launch_modes<T>(ctx, B.dct1, 0);
+    launch_modes<T>(ctx, B.dct1, 0, ctx->lam_y, ctx->lam_z);
     dct_pass<T, 1, false>(ctx, ny, ylines, B.dct1, B.dct2);
     // into phi's interior, times 1/(4 ny nz)
     FftLines out = zlines;
@@ -497,6 +498,44 @@ void launch_poisson_lines(pllgpu_ctx* ctx)
     out.scale = 1.0 / (4.0 * (double)N);
     T* phi0 = B.phi + (long)ctx->Rg.is * ctx->G.sx + (long)ctx->Rg.js * ctx->G.sy + ctx->Rg.ks;
     dct_pass<T, 1, true>(ctx, nz, out, B.dct2, phi0);
+}
+
+// planes transformed whole (plane_dct.cuh has the figures on both sides)
+inline bool plane_ok(int ny, int nz)
+{
+    auto side = [](int n) { return n == 32 || n == 64 || n == 128; };
+    return side(ny) && side(nz) && ny * nz <= 4096;
+}
+
+template <typename F>
+void with_plane(int ny, int nz, const F& f)
+{
+    using L32 = std::integral_constant<int, 32>;
+    using L64 = std::integral_constant<int, 64>;
+    using L128 = std::integral_constant<int, 128>;
+    if (ny == 32) nz == 32 ? f(L32{}, L32{}) : nz == 64 ? f(L32{}, L64{}) : f(L32{}, L128{});
+    else if (ny == 64) nz == 32 ? f(L64{}, L32{}) : f(L64{}, L64{});
+    else f(L128{}, L32{});
+}
+
+// divergence, phisolver_dct and update_phi_ghosts on planes transformed whole
+template <typename T>
+void launch_poisson_planes(pllgpu_ctx* ctx, double alpha)
+{
+    Bufs<T>& B = bufs<T>(ctx);
+    const DctAxis &Y = ctx->dct[0], &Z = ctx->dct[1];
+    with_plane(ctx->G.ny, ctx->G.nz, [&](auto NY, auto NZ) {
+        using S = PlaneShape<NY.value, NZ.value>;
+        go<k_dct_plane_fwd_b<T, NY.value, NZ.value>>(
+            ctx, k_dct_plane_fwd<T, NY.value, NZ.value>, ctx->G.nx, S::TH, S::SMEM, ctx->G, ctx->Rg, ctx->K,
+            q_new<T>(ctx, VU), q_new<T>(ctx, VV), q_new<T>(ctx, VW), B.dct1, ctx->scal, alpha, Y.tw, Y.wq, Z.tw, Z.wq);
+        mark(ctx, "div_dct");
+        launch_modes<T>(ctx, B.dct1, 0, ctx->lam_py, ctx->lam_pz);
+        go<k_dct_plane_inv_b<T, NY.value, NZ.value>>(
+            ctx, k_dct_plane_inv<T, NY.value, NZ.value>, ctx->G.nx, S::TH, S::SMEM, ctx->G, ctx->Rg, B.dct1, B.phi,
+            1.0 / (4.0 * (double)S::CELLS), Y.tw, Y.wq, Z.tw, Z.wq);
+        mark(ctx, "dct_phi");
+    });
 }
 
 // phisolver_dct after its right-hand side is in dct1 (compact [x][y][z])
@@ -526,7 +565,7 @@ void launch_poisson(pllgpu_ctx* ctx)
     d = GemmDesc{ny, nz, nz, nx, N, nz, 1, 0, 1, nz, N, nz, 1, 0.0, 0};
     launch_gemm(ctx, d, B.dct2, B.Tz, B.dct1);
     // x-tridiagonal per mode, in place in dct1, FP64 arithmetic
-    launch_modes<real>(ctx, B.dct1, 0);
+    launch_modes<real>(ctx, B.dct1, 0, ctx->lam_y, ctx->lam_z);
     // inverse, y pass: dct2[x][y][kz] = sum_ky Tiy[y][ky] dct1[x][ky][kz]
     d = GemmDesc{ny, nz, ny, nx, 0, ny, 1, N, nz, 1, N, nz, 1, 0.0, 0};
     launch_gemm(ctx, d, B.Tiy, B.dct1, B.dct2);
@@ -679,9 +718,18 @@ void enqueue_substep(pllgpu_ctx* ctx, int rk)
     on_side(ctx, 0);
     launch_flux<real>(ctx);
     on_side(ctx, -1);
-    launch_div<real>(ctx, 0, alpha);
-    launch_poisson<real>(ctx);
-    launch_phi_ghosts<real>(ctx);
+    bool done = false;
+    if constexpr (part_form<real>()) {
+        if (ctx->planes) {
+            launch_poisson_planes<real>(ctx, alpha);
+            done = true;
+        }
+    }
+    if (!done) {
+        launch_div<real>(ctx, 0, alpha);
+        launch_poisson<real>(ctx);
+        launch_phi_ghosts<real>(ctx);
+    }
     join(ctx, 1);
     launch_project<real>(ctx, alpha, 1, 1, 1);
     ctx->cur ^= 1;  // update_old_*: roles swap
@@ -1069,12 +1117,25 @@ bool setup_fold(pllgpu_ctx* c, int axis, int n)
 
 // each axis by FFT where its length is a power of two up to 256, else by the
 // folded product; both axes longer than that keep the GEMM passes
+template <typename T>
 bool setup_dct_lines(pllgpu_ctx* c)
 {
     const int len[2] = {c->P.ny, c->P.nz};
     if (len[0] > FOLD_MAX || len[1] > FOLD_MAX) return true;
     for (int a = 0; a < 2; ++a)
         if (!(fft_len_ok(len[a]) ? setup_fft(c, a, len[a]) : setup_fold(c, a, len[a]))) return false;
+    if (plane_ok(len[0], len[1])) {
+        with_plane(len[0], len[1], [&](auto NY, auto NZ) {
+            using S = PlaneShape<NY.value, NZ.value>;
+            c->planes = cudaFuncSetAttribute(k_dct_plane_fwd<T, NY.value, NZ.value>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM) == cudaSuccess &&
+                        cudaFuncSetAttribute(k_dct_plane_inv<T, NY.value, NZ.value>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::SMEM) == cudaSuccess;
+            c->dct[0].r1 = FftShape<NY.value>::R1, c->dct[0].r2 = FftShape<NY.value>::R2;
+            c->dct[1].r1 = FftShape<NZ.value>::R1, c->dct[1].r2 = FftShape<NZ.value>::R2;
+        });
+        return (c->lam_py = dalloc<double>(c, len[0])) && (c->lam_pz = dalloc<double>(c, len[1]));
+    }
     return true;
 }
 
@@ -1139,10 +1200,10 @@ bool alloc_state(pllgpu_ctx* c)
             c->xt_on = true;
         }
         const bool shape_ok = (p->ny == 128 || p->ny == 256) && (p->nz == 128 || p->nz == 256);
-        if (!p->exact_dct && p->dct_kernel != 1 && !(shape_ok ? setup_umma(c) : setup_dct_lines(c))) return false;
+        if (!p->exact_dct && p->dct_kernel != 1 && !(shape_ok ? setup_umma(c) : setup_dct_lines<float>(c))) return false;
     } else {
 #if !PLL_FP64_EXACT
-        if (!p->exact_dct && !setup_dct_lines(c)) return false;
+        if (!p->exact_dct && !setup_dct_lines<double>(c)) return false;
         if (!p->exact_dct && c->nelem < (1L << 31) && encode_tiled()) {
             xt_setup<VC, double>(c);
             xt_setup<VU, double>(c);

@@ -265,6 +265,15 @@ pllgpu_ctx* pllgpu_create(const pllgpu_params* p, int device)
             lz[k] = 2.0 * (std::cos(PI * (double)k / (double)p->nz) - 1.0) / (G.dz * G.dz);
         cudaMemcpy(c->lam_y, ly.data(), sizeof(double) * p->ny, cudaMemcpyHostToDevice);
         cudaMemcpy(c->lam_z, lz.data(), sizeof(double) * p->nz, cudaMemcpyHostToDevice);
+        if (c->planes) {   // position n2 + r2 k1 of a line holds frequency k1 + r1 n2
+            auto order = [](const std::vector<double>& l, const DctAxis& A, double* d) {
+                std::vector<double> o(l.size());
+                for (size_t t = 0; t < l.size(); ++t) o[t] = l[t / A.r2 + A.r1 * (t % A.r2)];
+                cudaMemcpy(d, o.data(), sizeof(double) * o.size(), cudaMemcpyHostToDevice);
+            };
+            order(ly, c->dct[0], c->lam_py);
+            order(lz, c->dct[1], c->lam_pz);
+        }
     }
     // Timestep with the diffusive cap of pllcart3d.c:150-154
     {

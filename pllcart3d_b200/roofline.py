@@ -34,6 +34,8 @@ KERNEL_WORDS = {
     "dct_umma": 2,
     "dct_fft": 2,        # one FFT pass: in ; out
     "dct_fold": 2,       # one folded dense pass: in ; out
+    "div_dct": 4,        # u, v, w ; modes (whole planes)
+    "dct_phi": 2,        # modes ; phi
     "poisson_x": 2,
     "project": 17,       # u v w phi mu(4) pg(3) ; u v w pg(3)
     "cfl": 3,
@@ -53,7 +55,7 @@ FAMILY = {
     "adi_x_c": "k_line_seg (x)", "adi_x_u": "k_line_seg (x)", "adi_x_v": "k_line_seg (x)",
     "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_fft": "k_dct_fft",
-    "dct_fold": "k_dct_fold",
+    "dct_fold": "k_dct_fold", "div_dct": "k_dct_plane_fwd", "dct_phi": "k_dct_plane_inv",
     "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl2",
 }
 
@@ -80,6 +82,7 @@ FAMILY_FP32 = {
     "adi_x_w": "k_line_seg (x)",
     "viscosity": "k_viscosity2", "div_rhs": "k_div_rhs2", "dct_umma": "k_dct_umma_p",
     "dct_fft": "k_dct_fft", "dct_fold": "k_dct_fold",
+    "div_dct": "k_dct_plane_fwd", "dct_phi": "k_dct_plane_inv",
     "poisson_x": "k_poisson_part", "project": "k_project2", "cfl": "k_cfl2",
 }
 
