@@ -419,7 +419,7 @@ def run_ours(args, ws, rank, local):
         sb = roofline.step_bytes(cells, prec)
         m["value"] = replica_value(cells, args.steps, ws, m["ms"])
         m["roofline"] = roofline_of(m["kernels"], m["profile_steps"], cells, prec, (prm.nx, prm.ny, prm.nz),
-                                    form, args.explicit_kernel)
+                                    form, "tma" if args.explicit_kernel == "auto" else args.explicit_kernel)
         m["step_roofline"] = {"bytes_per_step": sb,
                               "achieved_gbs": sb / (m["ms"] / args.steps / 1e3) / 1e9,
                               "frac_of_hbm": sb / (m["ms"] / args.steps / 1e3) / 1e9 / hbm}

@@ -64,19 +64,19 @@ typedef struct pllgpu_params {
                               the CPU restatement; FP64: the reference's
                               operation order throughout), and in the precision form
                               every line / mode solve the sequential Thomas
-                              sweep; 0: tensor-core DCT, and in the precision
-                              form the partitioned line solves and, with the
-                              tcgen05 DCT, the FP32-scratch mode solve        */
+                              sweep; 0: FFT, folded or tcgen05 DCT passes and
+                              partitioned line and mode solves                */
     int use_graph;         /* 1: replay each step as one CUDA graph            */
     int dct_kernel;        /* precision form, exact_dct 0: 0 = tcgen05 split-TF32
                               GEMMs (persistent, one CTA per SM) where ny, nz
-                              are 128 or 256, else mma.sync; 1 = mma.sync
-                              split-TF32 always; 2 = tcgen05, one tile per CTA */
-    int explicit_kernel;   /* explicit operator, exact_dct 0: 0 = default (FP64
-                              forms: TMA-staged plane-marching kernel; the
-                              precision form: cell pairs in FP32x2), 1 = the
-                              per-cell kernel (FP64) / cell pairs (FP32), 2 =
-                              the TMA-staged kernel in either form           */
+                              are 128 or 256, else the FP64 forms' line passes
+                              on FP32 storage; 1 = mma.sync split-TF32 GEMMs;
+                              2 = tcgen05, one tile per CTA                    */
+    int explicit_kernel;   /* explicit operator, exact_dct 0: 0 = default (the
+                              TMA-staged plane-marching kernel; in the precision
+                              form on pairs of rows in FP32x2), 1 = without
+                              staging: per cell (FP64) / cell pairs (FP32),
+                              2 = as 0                                        */
     int reserved[3];
 } pllgpu_params;
 

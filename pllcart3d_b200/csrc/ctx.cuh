@@ -87,7 +87,7 @@ struct pllgpu_ctx {
     DctAxis dct[2];             // the DCT passes along y and z
     bool planes = false;        // ... both at once, plane by plane (plane_dct.cuh)
     double *lam_py = nullptr, *lam_pz = nullptr;   // lam_y, lam_z in the planes' mode order
-    bool xt_on = false;         // FP64 form: TMA-staged marching explicit operator
+    bool xt_on = false;         // TMA-staged marching explicit operator
     int xt_cap[4] = {};         // its blocks resident at once, per variable
     UmmaPlan um;                // precision form's tensor-core DCT (when shapes allow)
     double* scal = nullptr;     // device scalars (S_*)

@@ -20,8 +20,8 @@
 // Two forms share the orchestration, templated on the storage type:
 // PLLGPU_FP64 keeps every field in FP64 (the reference's arithmetic);
 // PLLGPU_MIXED keeps the state in FP32 (WENO fluxes, stress terms, ADI
-// sweeps in FP32), runs the DCT passes as split-TF32 tensor-core GEMMs with
-// FP32 accumulation, and keeps FP64 for the Poisson mode solve (eigenvalue
+// sweeps in FP32), runs the DCT passes of planes of 128 or 256 points a side as
+// split-TF32 tensor-core GEMMs with FP32 accumulation, and keeps FP64 for the Poisson mode solve (eigenvalue
 // division, zero mode and gauge) and for the CFL, flux, mass and divergence
 // reductions.
 #include <cuda_runtime.h>

@@ -70,7 +70,8 @@ FAMILY_EXACT = dict(FAMILY, **{
     "adi_z_w": "k_adi_z_tiled",
     "viscosity": "k_viscosity", "div_rhs": "k_div_rhs", "dct_gemm": "k_gemm_dmma", "project": "k_project", "cfl": "k_cfl"})
 
-# the precision form's kernels where they differ from the FP64 form's
+# the precision form's kernels where they differ from the FP64 form's (the
+# explicit operator's without staging; explicit="tma", its default, below)
 FAMILY_FP32 = {
     "explicit_c": "k_explicit2", "explicit_u": "k_explicit2", "explicit_v": "k_explicit2",
     "explicit_w": "k_explicit2",
@@ -90,7 +91,8 @@ FAMILY_FP32 = {
 def family(label: str, precision: str = "fp64", form: str = None, explicit: str = "auto"):
     """Kernel (family) that runs `label` in the given form, or None.  `form`
     is "fp64x" for the exact form; `explicit` is the Solver's explicit_kernel
-    ("direct" runs the FP64 forms' explicit operator as k_explicit)."""
+    ("direct" runs the FP64 forms' explicit operator as k_explicit, "tma" the
+    precision form's as k_explicit_tma, which a Solver does by default)."""
     if precision == "fp32" and label in FAMILY_FP32:
         if explicit == "tma" and label.startswith("explicit_"):
             return "k_explicit_tma"

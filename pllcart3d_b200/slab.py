@@ -27,8 +27,8 @@ with MPI_Allreduce (L3113).  Here:
                          own rows.  One collective per sweep instead of
                          pll_tridiag's 2 messages per line per boundary.
 
-The same elimination runs inside one GPU in the precision form's segmented
-line solve (``k_line_seg``).  Nothing in this module is wired into the GPU
+The same elimination runs inside one GPU in the partitioned line solves
+(``k_line_seg``).  Nothing in this module is wired into the GPU
 step: every GPU run available to this project has one device.
 """
 

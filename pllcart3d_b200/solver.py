@@ -35,16 +35,16 @@ class Solver:
     reductions; "mixed64": the FP64 form with the WENO5 weights in FP32.
     dct_kernel="auto" runs the precision form's DCT passes as
     tcgen05 GEMMs where the plane shape allows (ny, nz in {128, 256}; a
-    persistent kernel, one CTA per SM), "umma_tile" the same tcgen05 pass
-    with one tile per CTA, "mma_sync" the warp-level split-TF32 GEMM.
-    explicit_kernel="auto" runs the explicit operator as the TMA-staged
-    plane-marching kernel in the FP64 forms and on FP32x2 cell pairs in the
-    precision form; "direct" the per-cell (FP64) / paired (FP32) kernel,
-    "tma" the TMA-staged kernel in either form.
+    persistent kernel, one CTA per SM; elsewhere as the FP64 forms' line
+    passes), "umma_tile" the same tcgen05 pass with one tile per CTA,
+    "mma_sync" the warp-level split-TF32 GEMM.
+    explicit_kernel="auto" (or "tma") runs the explicit operator as the
+    TMA-staged plane-marching kernel (the precision form's on pairs of rows in
+    FP32x2); "direct" the per-cell (FP64) / paired (FP32) kernel without
+    staging.
     exact_dct=True sums the DCTs in sequential order and, in the precision
     form, runs every line and mode solve as the sequential Thomas sweep (the
-    default: the partitioned line solves and, with the tcgen05 DCT, the
-    FP32-scratch mode solve)."""
+    default: the partitioned solves)."""
 
     def __init__(self, params: Params, device: int = 0, exact_dct: bool = False,
                  use_graph: bool = True, precision: str = "fp64", dct_kernel: str = "auto",
