@@ -11,8 +11,9 @@
 // same body over a grid whose z extent is the class size times the
 // member's, member m = blockIdx.z / gz reading its own arguments from a
 // device table.  Each member so computes exactly what it computes alone.
-// Kernels whose arguments hold a tensor map (passed as __grid_constant__)
-// have no spec and replay one launch per member.
+// A body that takes tensor maps reads them where they lie in that table (a
+// pack starts on 128 bytes, its maps first).  Kernels without a body, the
+// tcgen05 DCT's, replay one launch per member.
 #pragma once
 
 #include <cuda_runtime.h>
