@@ -11,9 +11,12 @@
 // same body over a grid whose z extent is the class size times the
 // member's, member m = blockIdx.z / gz reading its own arguments from a
 // device table.  Each member so computes exactly what it computes alone.
-// A body that takes tensor maps reads them where they lie in that table (a
-// pack starts on 128 bytes, its maps first).  Kernels without a body, the
-// tcgen05 DCT's, replay one launch per member.
+// A body whose first argument is its tensor maps finds them in the launch's
+// parameters instead (MapPack): a map that lies in global memory has to be
+// acquired by every block before it is used, since a later table may lie at an
+// earlier one's address, and with those fences 4 steps of 24 members in FP32
+// took 13.8 ms instead of 12.7.  Kernels without a body, the tcgen05 DCT's, replay one launch
+// per member.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -72,8 +75,12 @@ struct LaunchRec {
     virtual void one(cudaStream_t st) const = 0;
     // before a capture: the batched kernel's shared-memory opt-in
     virtual cudaError_t prepare() const = 0;
-    // n members of a class at once, member m's argument pack at tab + m * stride
-    virtual cudaError_t many(const unsigned char* tab, size_t stride, unsigned n, cudaStream_t st) const = 0;
+    // the most members one launch takes
+    virtual unsigned most() const = 0;
+    // n members of a class at once: their recorded launches, and member m's
+    // argument pack at tab + m * stride
+    virtual cudaError_t many(const LaunchRec* const* members, const unsigned char* tab, size_t stride, unsigned n,
+                             cudaStream_t st) const = 0;
     bool same_launch(const LaunchRec& o) const
     {
         return fn == o.fn && grid.x == o.grid.x && grid.y == o.grid.y && grid.z == o.grid.z && blk.x == o.blk.x &&
@@ -117,6 +124,39 @@ __global__ void __launch_bounds__(MAXT, MINB) k_members_b2(const unsigned char* 
                           dim3(gridDim.x, gridDim.y, gz), std::index_sequence_for<P...>{});
 }
 
+// the same for a body whose first argument M is its tensor maps, member m's
+// in the launch's own parameters
+template <typename M, int N>
+struct MapPack {
+    M m[N];
+};
+template <auto RUN, int MAXT, int MINB, int N, typename M, typename... P, size_t... I>
+__device__ __forceinline__ void member_run_maps(const M& maps, const Tup<M, P...>& t, uint3 b, dim3 g,
+                                                std::index_sequence<I...>)
+{
+    RUN(b, g, maps, TupAt<I + 1>::get(t)...);
+}
+template <auto RUN, int MAXT, int MINB, int N, typename M, typename... P>
+__global__ void __launch_bounds__(MAXT, MINB) k_members_maps(const __grid_constant__ MapPack<M, N> maps,
+                                                             const unsigned char* __restrict__ tab, unsigned stride,
+                                                             unsigned gz)
+{
+    const unsigned m = blockIdx.z / gz;
+    const Tup<M, P...>& t = *reinterpret_cast<const Tup<M, P...>*>(tab + (size_t)m * stride);
+    member_run_maps<RUN, MAXT, MINB, N, M, P...>(maps.m[m], t, make_uint3(blockIdx.x, blockIdx.y, blockIdx.z - m * gz),
+                                                 dim3(gridDim.x, gridDim.y, gz), std::index_sequence_for<P...>{});
+}
+// A large class's launches carry as many maps as a kernel's 32764 bytes of
+// parameters hold, a small one's few: the same time a step, but a graph's nodes
+// keep their parameters, and building it for 24 members on 4 grids and running 4
+// steps took 21 to 24 ms with 40 maps a launch and 19 with 8.
+constexpr int MAPS_FEW = 8, MAPS_MANY = 40;
+
+template <typename B, typename = void>
+struct BatchMaps : std::false_type {};
+template <typename B>
+struct BatchMaps<B, std::void_t<decltype(B::maps)>> : std::bool_constant<B::maps> {};
+
 // minimum blocks per SM of a batched copy: the spec's bminb where it has
 // one (a body that reads its arguments from memory holds more registers
 // than the kernel that finds them in its parameter bank), else its minb
@@ -148,31 +188,58 @@ struct LaunchRecT : LaunchRec {
         k<<<grid, blk, smem, st>>>(TupAt<I>::get(a)...);
     }
     void one(cudaStream_t st) const override { one_(st, std::index_sequence_for<P...>{}); }
-    const void* batched_kernel() const
+    template <int N, typename M, typename... Q>
+    static const void* maps_kernel(const Tup<M, Q...>*)
+    {
+        static_assert(sizeof(MapPack<M, N>) + 16 <= 32764, "a launch's parameters");
+        return (const void*)k_members_maps<B::run, B::maxt, BatchMinb<B>::value, N, M, Q...>;
+    }
+    const void* batched_kernel(unsigned n) const
     {
         if constexpr (std::is_same<B, NoBatch>::value) return nullptr;
+        else if constexpr (BatchMaps<B>::value) return n <= MAPS_FEW ? maps_kernel<MAPS_FEW>(&a) : maps_kernel<MAPS_MANY>(&a);
         else if constexpr (B::maxt == 0) return (const void*)k_members<B::run, P...>;
         else if constexpr (BatchMinb<B>::value == 0) return (const void*)k_members_b1<B::run, B::maxt, P...>;
         else return (const void*)k_members_b2<B::run, B::maxt, BatchMinb<B>::value, P...>;
     }
+    unsigned most() const override { return BatchMaps<B>::value ? (unsigned)MAPS_MANY : 65535u; }
     cudaError_t prepare() const override
     {
         // static and dynamic shared memory together above 48 KB need the
         // opt-in, which is a per-device attribute: set on every build (a
         // host call, once per recorded launch, never per step)
-        const void* kb = batched_kernel();
-        if (kb && smem > 0)
-            return cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        return cudaSuccess;
+        cudaError_t e = cudaSuccess;
+        for (unsigned n : {1u, most()}) {
+            const void* kb = batched_kernel(n);
+            if (kb && smem > 0 && e == cudaSuccess)
+                e = cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        }
+        return e;
     }
-    cudaError_t many(const unsigned char* tab, size_t stride, unsigned n, cudaStream_t st) const override
+    template <int N, typename M, typename... Q>
+    cudaError_t many_maps(const Tup<M, Q...>*, const LaunchRec* const* members, void** rest, dim3 g, unsigned n,
+                          cudaStream_t st) const
     {
-        const void* kb = batched_kernel();
-        if (!kb) return cudaErrorInvalidValue;
+        MapPack<M, N> maps;
+        std::memset(&maps, 0, sizeof(maps));
+        for (unsigned m = 0; m < n; ++m) maps.m[m] = static_cast<const LaunchRecT*>(members[m])->a.h;
+        void* args[4] = {&maps, rest[0], rest[1], rest[2]};
+        return cudaLaunchKernel(batched_kernel(n), g, blk, args, smem, st);
+    }
+    cudaError_t many(const LaunchRec* const* members, const unsigned char* tab, size_t stride, unsigned n,
+                     cudaStream_t st) const override
+    {
+        const void* kb = batched_kernel(n);
+        if (!kb || n > most()) return cudaErrorInvalidValue;
         unsigned st_ = (unsigned)stride, gz = grid.z;
         const dim3 g(grid.x, grid.y, grid.z * n);
         void* args[3] = {(void*)&tab, (void*)&st_, (void*)&gz};
-        return cudaLaunchKernel(kb, g, blk, args, smem, st);
+        if constexpr (BatchMaps<B>::value) {
+            if (n <= MAPS_FEW) return many_maps<MAPS_FEW>(&a, members, args, g, n, st);
+            return many_maps<MAPS_MANY>(&a, members, args, g, n, st);
+        } else {
+            return cudaLaunchKernel(kb, g, blk, args, smem, st);
+        }
     }
 };
 

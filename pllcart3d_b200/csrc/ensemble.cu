@@ -8,9 +8,8 @@
 // whole class: the stage's kernel body runs over a grid whose z extent is
 // the class size times the member's, each member reading its own arguments
 // from a device table (batch.cuh).  64 members on 4 grid classes so issue 4
-// launches per stage, not 64.  Stages whose kernels take a tensor map
-// (none in the precision form at these grid sizes) issue one launch per
-// member in the class's branch.
+// launches per stage, not 64.  The tcgen05 DCT passes (planes of 128 or 256
+// points a side) issue one launch per member in the class's branch.
 //
 // Each member computes exactly what it computes alone (the same kernel body
 // with the same arithmetic on its own buffers); the autotuner picks launch
@@ -202,12 +201,17 @@ int build_batched(pllgpu_ensemble* e)
                     for (int k : c) rec[t][k][p]->one(st);
                     launches += (int)c.size();
                 } else {
-                    // grid.z of one launch stays within 65535: chunks of members
+                    // a launch takes a limited number of members, and its
+                    // grid.z stays within 65535: chunks of members
                     const size_t stride = pack_stride(r);
-                    const size_t chunk = std::max<size_t>(1, 65535 / std::max(1u, r->grid.z));
+                    const size_t chunk = std::max<size_t>(
+                        1, std::min<size_t>(r->most(), 65535 / std::max(1u, r->grid.z)));
+                    std::vector<const LaunchRec*> of;
+                    for (int k : c) of.push_back(rec[t][k][p]);
                     for (size_t k0 = 0; k0 < c.size() && ok; k0 += chunk) {
                         const unsigned cn = (unsigned)std::min(chunk, c.size() - k0);
-                        if (cudaError_t err = r->many(e->tables + off[t][q] + k0 * stride, stride, cn, st)) {
+                        if (cudaError_t err = r->many(of.data() + k0, e->tables + off[t][q] + k0 * stride, stride, cn,
+                                                       st)) {
                             std::fprintf(stderr,
                                          "pllgpu: ensemble: batched launch %zu (grid %u %u %u x %u, block %u %u %u, "
                                          "%zu bytes shared): %s\n", p, r->grid.x, r->grid.y, r->grid.z, cn,

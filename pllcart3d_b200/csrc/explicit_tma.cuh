@@ -533,11 +533,10 @@ __global__ void __launch_bounds__(XT_THREADS, XtBlocks<VAR, real>::value)
     if (!after_previous()) return;
     k_explicit_tma_run<VAR, real>(blockIdx, gridDim, maps, G, R, K, C, A, ni, status);
 }
-// a batched copy takes its tensor maps where they lie, in the argument table
-// (64-byte aligned: the pack's first member)
 template <int VAR, typename real>
 struct k_explicit_tma_b {
     static constexpr auto run = &k_explicit_tma_run<VAR, real>;
+    static constexpr bool maps = true;   // the first argument: tensor maps
     static constexpr int maxt = XT_THREADS, minb = 0, bminb = sizeof(real) == 4 ? 2 : 0;
     static constexpr bool chained = true;
 };
