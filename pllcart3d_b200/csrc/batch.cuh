@@ -15,8 +15,8 @@
 // parameters instead (MapPack): a map that lies in global memory has to be
 // acquired by every block before it is used, since a later table may lie at an
 // earlier one's address, and with those fences 4 steps of 24 members in FP32
-// took 13.8 ms instead of 12.7.  Kernels without a body, the tcgen05 DCT's, replay one launch
-// per member.
+// took 13.8 ms instead of 12.7.  Kernels without a body, the tcgen05 DCT's,
+// replay one launch per member.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -26,6 +26,8 @@
 #include <type_traits>
 #include <utility>
 #include <vector>
+
+#include "host_util.h"
 
 namespace pll {
 
@@ -206,13 +208,12 @@ struct LaunchRecT : LaunchRec {
     cudaError_t prepare() const override
     {
         // static and dynamic shared memory together above 48 KB need the
-        // opt-in, which is a per-device attribute: set on every build (a
-        // host call, once per recorded launch, never per step)
+        // opt-in: asked for on every build (a host call, once per recorded
+        // launch, never per step)
         cudaError_t e = cudaSuccess;
         for (unsigned n : {1u, most()}) {
             const void* kb = batched_kernel(n);
-            if (kb && smem > 0 && e == cudaSuccess)
-                e = cudaFuncSetAttribute(kb, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            if (kb && smem > 0 && e == cudaSuccess) e = allow_smem(kb, smem);
         }
         return e;
     }

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <mutex>
 
 namespace pll {
 
@@ -35,6 +36,20 @@ inline void dct_matrix(int kind, int n, T* out)
             }
             out[(long)k * n + j] = (T)v;
         }
+}
+
+// Dynamic shared memory of a kernel, opted in for up to `bytes`.  The limit
+// belongs to the kernel on the current device, for every context and thread:
+// a kernel launched in several sizes (the folded DCT by its length, the batched
+// copies by their class) must keep the largest, so it is only ever raised.
+inline cudaError_t allow_smem(const void* kernel, size_t bytes)
+{
+    static std::mutex one;
+    std::lock_guard<std::mutex> hold(one);
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, kernel);
+    if (e != cudaSuccess || (long)bytes <= (long)a.maxDynamicSharedSizeBytes) return e;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
 // owning device buffer released on scope exit

@@ -460,11 +460,9 @@ void dct_pass(pllgpu_ctx* ctx, int n, const FftLines& d, const T* in, T* out)
 {
     constexpr int axis = CONTIG ? 1 : 0;
     if (ctx->dct[axis].mode == DctAxis::FOLD) {
-        const size_t smem = fold_smem<CONTIG>(n);
-        if (smem > 48 * 1024)
-            cudaFuncSetAttribute(k_dct_fold<KIND, CONTIG, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         go<k_dct_fold_b<KIND, CONTIG, T>>(ctx, k_dct_fold<KIND, CONTIG, T>, (d.lines + FOLD_LINES - 1) / FOLD_LINES,
-                                          32 * fold_warps(n), smem, d, n, in, out, ctx->dct[axis].table[KIND]);
+                                          32 * fold_warps(n), fold_smem<CONTIG>(n), d, n, in, out,
+                                          ctx->dct[axis].table[KIND]);
         mark(ctx, "dct_fold");
         return;
     }
@@ -1089,10 +1087,16 @@ bool setup_fft(pllgpu_ctx* c, int axis, int N)
     return true;
 }
 
-// the folded matrices of both kinds in fragment order (fold_dct.cuh)
+// the folded matrices of both kinds in fragment order (fold_dct.cuh), and the
+// kernels' shared memory
+template <typename T>
 bool setup_fold(pllgpu_ctx* c, int axis, int n)
 {
     DctAxis& A = c->dct[axis];
+    const void* k[2][2] = {{(const void*)k_dct_fold<0, false, T>, (const void*)k_dct_fold<1, false, T>},
+                           {(const void*)k_dct_fold<0, true, T>, (const void*)k_dct_fold<1, true, T>}};
+    for (const void* f : k[axis])
+        if (allow_smem(f, axis ? fold_smem<true>(n) : fold_smem<false>(n)) != cudaSuccess) return false;
     const int KB = fold_kb(n), MB = fold_mb(n), half = (n + 1) / 2;
     std::vector<double> M((size_t)n * n), t((size_t)fold_table(n));
     for (int kind = 0; kind < 2; ++kind) {
@@ -1123,7 +1127,7 @@ bool setup_dct_lines(pllgpu_ctx* c)
     const int len[2] = {c->P.ny, c->P.nz};
     if (len[0] > FOLD_MAX || len[1] > FOLD_MAX) return true;
     for (int a = 0; a < 2; ++a)
-        if (!(fft_len_ok(len[a]) ? setup_fft(c, a, len[a]) : setup_fold(c, a, len[a]))) return false;
+        if (!(fft_len_ok(len[a]) ? setup_fft(c, a, len[a]) : setup_fold<T>(c, a, len[a]))) return false;
     if (plane_ok(len[0], len[1])) {
         with_plane(len[0], len[1], [&](auto NY, auto NZ) {
             using S = PlaneShape<NY.value, NZ.value>;
