@@ -32,10 +32,11 @@ struct Bufs {
     real* phi = nullptr;
     real* div = nullptr;
     real* S[4] = {};        // ADI right-hand side / eliminated rhs of each variable
-                            // (the exact form: one array for all)
-    real* cc = nullptr;     // Thomas scratch
-    real* dct1 = nullptr;   // compact nx*ny*nz Poisson buffers
-    real* dct2 = nullptr;
+                            // (the exact form: one array for all; else v's and
+                            // w's are dct1 and dct2)
+    real* cc = nullptr;     // Thomas scratch, where a sequential sweep runs
+    real* dct1 = nullptr;   // compact nx*ny*nz Poisson buffers (a field's size
+    real* dct2 = nullptr;   // where they also hold right-hand sides)
     real *Ty = nullptr, *Tz = nullptr, *Tiy = nullptr, *Tiz = nullptr;
 };
 
@@ -81,7 +82,8 @@ struct pllgpu_ctx {
     long nelem = 0;             // elements of one padded field
     Bufs<double> b64;           // state of the FP64 form
     Bufs<float> b32;            // state of the mixed form
-    double *mode_cc = nullptr, *mode_rr = nullptr;  // FP64 Poisson mode scratch
+    // scratch of the sequential Poisson mode solve, where it runs
+    double *mode_cc = nullptr, *mode_rr = nullptr;
     double* stage64 = nullptr;  // one padded FP64 field (mixed-form transfers)
     double *lam_y = nullptr, *lam_z = nullptr;
     DctAxis dct[2];             // the DCT passes along y and z

@@ -1170,12 +1170,26 @@ bool alloc_state(pllgpu_ctx* c)
     for (int v = 1; v < 4 && ok; ++v) ok = (B.pg[v] = dalloc<real>(c, c->nelem)) != nullptr;
     const long ncell = (long)p->nx * p->ny * p->nz;
     ok = ok && (B.phi = dalloc<real>(c, c->nelem)) && (B.div = dalloc<real>(c, c->nelem)) &&
-         (B.S[VC] = dalloc<real>(c, c->nelem)) && (B.cc = dalloc<real>(c, c->nelem)) &&
-         (B.dct1 = dalloc<real>(c, ncell)) && (B.dct2 = dalloc<real>(c, ncell)) &&
+         (B.S[VC] = dalloc<real>(c, c->nelem)) &&
+         (B.dct1 = dalloc<real>(c, part_form<real>() ? c->nelem : ncell)) &&
+         (B.dct2 = dalloc<real>(c, part_form<real>() ? c->nelem : ncell)) &&
          (B.Ty = dalloc<real>(c, (long)p->ny * p->ny)) && (B.Tz = dalloc<real>(c, (long)p->nz * p->nz)) &&
          (B.Tiy = dalloc<real>(c, (long)p->ny * p->ny)) && (B.Tiz = dalloc<real>(c, (long)p->nz * p->nz));
-    B.S[VU] = B.S[VV] = B.S[VW] = B.S[VC];   // u's follows c's
-    if (ok && part_form<real>()) ok = (B.S[VV] = dalloc<real>(c, c->nelem)) && (B.S[VW] = dalloc<real>(c, c->nelem));
+    // right-hand sides: u's follows c's; v's and w's, where they stand beside
+    // it, lie in the Poisson buffers, idle until the line solves are done
+    B.S[VU] = B.S[VC];
+    B.S[VV] = part_form<real>() ? B.dct1 : B.S[VC];
+    B.S[VW] = part_form<real>() ? B.dct2 : B.S[VC];
+    // scratch of the sequential sweeps: for lines that the partitioned solves
+    // do not take; the FP64 mode sweep's c' shares the lines'
+    const bool seq_modes = !part_form<real>() || p->exact_dct || p->nx > LINE_PART_MAX;
+    if (seq_modes || p->ny > LINE_PART_MAX || p->nz > Z_PART_MAX)
+        ok = ok && (B.cc = dalloc<real>(c, c->nelem)) != nullptr;
+    if (seq_modes) {
+        if constexpr (std::is_same<real, double>::value) c->mode_cc = B.cc;
+        else ok = ok && (c->mode_cc = dalloc<double>(c, ncell)) != nullptr;
+        ok = ok && (c->mode_rr = dalloc<double>(c, ncell)) != nullptr;
+    }
     if (!ok) return false;
     std::vector<real> T((size_t)std::max(p->ny, p->nz) * std::max(p->ny, p->nz));
     dct_matrix<real>(0, p->ny, T.data());

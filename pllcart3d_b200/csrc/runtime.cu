@@ -243,10 +243,8 @@ pllgpu_ctx* pllgpu_create(const pllgpu_params* p, int device)
     K.Vnorm = 0.0;
 
     pllgpu_ctx* c = ctx;
-    const long ncell = (long)p->nx * p->ny * p->nz;
     bool ok = FORM_CALL(ctx, form_alloc, c);
-    ok = ok && (c->mode_cc = dalloc<double>(c, ncell)) && (c->mode_rr = dalloc<double>(c, ncell)) &&
-         (c->lam_y = dalloc<double>(c, p->ny)) && (c->lam_z = dalloc<double>(c, p->nz)) &&
+    ok = ok && (c->lam_y = dalloc<double>(c, p->ny)) && (c->lam_z = dalloc<double>(c, p->nz)) &&
          (c->scal = dalloc<double>(c, S_COUNT)) && (c->work = dalloc<double>(c, 2L * (p->nx + 8))) &&
          (c->diag = dalloc<double>(c, 3L * p->nx + 8)) && (c->status = dalloc<int>(c, 1)) &&
          (c->red = dalloc<double>(c, red_doubles(c->G))) && (c->ticket = dalloc<unsigned>(c, 3));
