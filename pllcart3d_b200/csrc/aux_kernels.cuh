@@ -733,6 +733,102 @@ struct k_poisson_x_b {
     static constexpr int maxt = 128, minb = 0;
 };
 
+// The precision form's sequential mode solve (lines longer than the partitioned
+// one takes): the same recurrences and FP64 scratch, but c' is not stored.  It
+// depends on the mode only, so the forward sweep records it every PX_CK rows
+// and the backward sweep recomputes each block of PX_CK values from its
+// checkpoint (the same arithmetic, so the same values): 24.5 bytes per cell
+// instead of 40.  1000x256x256: 374 us
+// (k_poisson_x 472), 2000x32x32: 428 (476).
+constexpr int PX_CK = 16;
+
+__device__ __forceinline__ void k_poisson_x2_run(const uint3 blockIdx, const dim3 gridDim,
+                                                 int nx, int ny, int nz, Consts K, const double* __restrict__ lam_y,
+                                                 const double* __restrict__ lam_z, float* __restrict__ hat,
+                                                 double* __restrict__ rr, double* __restrict__ ck, int kz_major)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    const int N = ny * nz;
+    if (t >= N) return;
+    const int jy = kz_major ? t % ny : t / nz, kz = kz_major ? t / ny : t % nz;
+    const long st = N;
+    const double a = K.dx2i, c = K.dx2i;
+    const double bmid = -2.0 * K.dx2i + lam_y[jy] + lam_z[kz];
+    const bool gauge = (jy == 0) && (kz == 0);
+    auto diag = [&](int m) {
+        double lb = bmid;
+        if (m == 0) lb += a;
+        if (m == nx - 1 && !gauge) lb += c;
+        return lb;
+    };
+    // forward: c'_m = c / (b_m - a c'_{m-1}), r'_m = (r_m - a r'_{m-1}) / (...)
+    constexpr int PF = 8;
+    double cprev = 0.0, rprev = 0.0;
+    float hv[PF];
+#pragma unroll
+    for (int u = 0; u < PF; ++u) hv[u] = u < nx ? hat[t + (long)u * st] : 0.f;
+    for (int m0 = 0; m0 < nx; m0 += PF) {
+        float hn[PF];
+#pragma unroll
+        for (int u = 0; u < PF; ++u) {
+            const int m = m0 + PF + u;
+            hn[u] = m < nx ? hat[t + (long)m * st] : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < PF; ++u) {
+            const int m = m0 + u;
+            if (m < nx) {
+                if (m % PX_CK == 0) ck[(long)(m / PX_CK) * st + t] = cprev;   // c'_{m-1}
+                const double inv = 1.0 / (diag(m) - cprev * a);
+                const double rm = ((double)hv[u] - rprev * a) * inv;
+                cprev = c * inv;   // as the backward sweep recomputes it
+                rprev = rm;
+                rr[t + (long)m * st] = rm;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < PF; ++u) hv[u] = hn[u];
+    }
+    // backward, one checkpoint block at a time from the end: x_{n-1} = r'_{n-1}
+    double xnext = 0.0;
+    for (int b0 = ((nx - 1) / PX_CK) * PX_CK; b0 >= 0; b0 -= PX_CK) {
+        double cb[PX_CK];
+        double rv[PX_CK];
+        double cp = ck[(long)(b0 / PX_CK) * st + t];
+#pragma unroll
+        for (int u = 0; u < PX_CK; ++u) {
+            const int m = b0 + u;
+            rv[u] = m < nx ? rr[t + (long)m * st] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < PX_CK; ++u) {
+            const int m = b0 + u;
+            if (m < nx) cp = c * (1.0 / (diag(m) - cp * a));
+            cb[u] = cp;
+        }
+#pragma unroll
+        for (int u = PX_CK - 1; u >= 0; --u) {
+            const int m = b0 + u;
+            if (m < nx) {
+                const double x = (m == nx - 1) ? rv[u] : rv[u] - cb[u] * xnext;
+                hat[t + (long)m * st] = (float)x;
+                xnext = x;
+            }
+        }
+    }
+}
+__global__ void __launch_bounds__(128) k_poisson_x2(int nx, int ny, int nz, Consts K,
+                                                    const double* __restrict__ lam_y,
+                                                    const double* __restrict__ lam_z, float* __restrict__ hat,
+                                                    double* __restrict__ rr, double* __restrict__ ck, int kz_major)
+{
+    k_poisson_x2_run(blockIdx, gridDim, nx, ny, nz, K, lam_y, lam_z, hat, rr, ck, kz_major);
+}
+struct k_poisson_x2_b {
+    static constexpr auto run = &k_poisson_x2_run;
+    static constexpr int maxt = 128, minb = 0;
+};
+
 // update_phi_ghosts (pllcart3d.c:2758-2807): Neumann copies on the six
 // faces; blockIdx.z 0: z faces over (i,j), 1: y faces over (i,k), 2: x faces
 // over (j,k).  blockIdx.y runs to the longest of the second extents.

@@ -248,9 +248,18 @@ void launch_modes(pllgpu_ctx* ctx, T* hat, int kz_major, const double* ly, const
 {
     const int nx = ctx->G.nx, N = ctx->G.ny * ctx->G.nz;
     constexpr int TL = 8;
-    if (ctx->P.exact_dct || nx > LINE_PART_MAX)
+    if (ctx->P.exact_dct || nx > LINE_PART_MAX) {
+        if constexpr (std::is_same<T, float>::value) {
+            if (!ctx->P.exact_dct) {
+                go<k_poisson_x2_b>(ctx, k_poisson_x2, (N + 127) / 128, 128, 0, nx, ctx->G.ny, ctx->G.nz, ctx->K, ly, lz,
+                                   hat, ctx->mode_rr, ctx->mode_cc, kz_major);
+                mark(ctx, "poisson_x");
+                return;
+            }
+        }
         go<k_poisson_x_b<T>>(ctx, k_poisson_x<T>, (N + 127) / 128, 128, 0, nx, ctx->G.ny, ctx->G.nz, ctx->K, ly,
                              lz, hat, ctx->mode_cc, ctx->mode_rr, kz_major);
+    }
     else if (nx <= 32) poisson_part<T, 8, 4, TL>(ctx, hat, kz_major, ly, lz);
     else if (nx <= 64) poisson_part<T, 8, 8, TL>(ctx, hat, kz_major, ly, lz);
     else if (nx <= 128) poisson_part<T, 8, 16, TL>(ctx, hat, kz_major, ly, lz);
@@ -1187,7 +1196,8 @@ bool alloc_state(pllgpu_ctx* c)
         ok = ok && (B.cc = dalloc<real>(c, c->nelem)) != nullptr;
     if (seq_modes) {
         if constexpr (std::is_same<real, double>::value) c->mode_cc = B.cc;
-        else ok = ok && (c->mode_cc = dalloc<double>(c, ncell)) != nullptr;
+        else if (p->exact_dct) ok = ok && (c->mode_cc = dalloc<double>(c, ncell)) != nullptr;
+        else ok = ok && (c->mode_cc = dalloc<double>(c, (long)((p->nx + PX_CK - 1) / PX_CK) * p->ny * p->nz)) != nullptr;
         ok = ok && (c->mode_rr = dalloc<double>(c, ncell)) != nullptr;
     }
     if (!ok) return false;
