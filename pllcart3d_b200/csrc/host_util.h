@@ -18,24 +18,19 @@ inline bool is_pow2(double h)
 // FFTW REDFT10 (kind 0) / REDFT01 (kind 1) as dense matrices T[k*n+j]
 // (FFTW 3 manual, "1d Real-even DFTs (DCTs)"); the argument is reduced
 // mod 4n exactly
+inline double dct_entry(int kind, int n, int k, int j)
+{
+    const double pi = 3.14159265358979323846;
+    if (kind == 1 && j == 0) return 1.0;
+    const long m = (kind == 0 ? (long)(2 * j + 1) * (long)k : (long)j * (long)(2 * k + 1)) % (4L * n);
+    return 2.0 * std::cos(pi * (double)m / (2.0 * n));
+}
+
 template <typename T>
 inline void dct_matrix(int kind, int n, T* out)
 {
-    const double pi = 3.14159265358979323846;
     for (int k = 0; k < n; ++k)
-        for (int j = 0; j < n; ++j) {
-            double v;
-            if (kind == 0) {
-                const long m = ((long)(2 * j + 1) * (long)k) % (4L * n);
-                v = 2.0 * std::cos(pi * (double)m / (2.0 * n));
-            } else if (j == 0) {
-                v = 1.0;
-            } else {
-                const long m = ((long)j * (long)(2 * k + 1)) % (4L * n);
-                v = 2.0 * std::cos(pi * (double)m / (2.0 * n));
-            }
-            out[(long)k * n + j] = (T)v;
-        }
+        for (int j = 0; j < n; ++j) out[(long)k * n + j] = (T)dct_entry(kind, n, k, j);
 }
 
 // Dynamic shared memory of a kernel, opted in for up to `bytes`.  The limit

@@ -1107,9 +1107,8 @@ bool setup_fold(pllgpu_ctx* c, int axis, int n)
     for (const void* f : k[axis])
         if (allow_smem(f, axis ? fold_smem<true>(n) : fold_smem<false>(n)) != cudaSuccess) return false;
     const int KB = fold_kb(n), MB = fold_mb(n), half = (n + 1) / 2;
-    std::vector<double> M((size_t)n * n), t((size_t)fold_table(n));
+    std::vector<double> t((size_t)fold_table(n));
     for (int kind = 0; kind < 2; ++kind) {
-        dct_matrix<double>(kind, n, M.data());
         for (int p = 0; p < 2; ++p)
             for (int mb = 0; mb < MB; ++mb)
                 for (int kb = 0; kb < KB; ++kb)
@@ -1118,7 +1117,7 @@ bool setup_fold(pllgpu_ctx* c, int axis, int n)
                         // DCT-II: mode 2o+p from point k; DCT-III: point o from mode 2k+p
                         const int row = kind == 0 ? 2 * o + p : o, col = kind == 0 ? k : 2 * k + p;
                         const bool in = kind == 0 ? (row < n && k < half) : (o < half && col < n);
-                        t[(((size_t)p * MB + mb) * KB + kb) * 32 + l] = in ? M[(size_t)row * n + col] : 0.0;
+                        t[(((size_t)p * MB + mb) * KB + kb) * 32 + l] = in ? dct_entry(kind, n, row, col) : 0.0;
                     }
         if (!(A.table[kind] = dalloc<double>(c, fold_table(n))) ||
             cudaMemcpy(A.table[kind], t.data(), sizeof(double) * t.size(), cudaMemcpyHostToDevice) != cudaSuccess)
@@ -1128,13 +1127,29 @@ bool setup_fold(pllgpu_ctx* c, int axis, int n)
     return true;
 }
 
+// the dense cosine matrices of the GEMM and tcgen05 passes
+template <typename real>
+bool setup_dct_dense(pllgpu_ctx* c)
+{
+    Bufs<real>& B = bufs<real>(c);
+    const int ny = c->P.ny, nz = c->P.nz;
+    std::vector<real> T((size_t)std::max(ny, nz) * std::max(ny, nz));
+    auto put = [&](int kind, int n, real*& d) {
+        const size_t n2 = (size_t)n * n;
+        dct_matrix<real>(kind, n, T.data());
+        return (d = dalloc<real>(c, (long)n2)) &&
+               cudaMemcpy(d, T.data(), sizeof(real) * n2, cudaMemcpyHostToDevice) == cudaSuccess;
+    };
+    return put(0, ny, B.Ty) && put(0, nz, B.Tz) && put(1, ny, B.Tiy) && put(1, nz, B.Tiz);
+}
+
 // each axis by FFT where its length is a power of two up to 256, else by the
-// folded product; both axes longer than that keep the GEMM passes
+// folded product; either axis longer than that keeps the GEMM passes on both
 template <typename T>
 bool setup_dct_lines(pllgpu_ctx* c)
 {
     const int len[2] = {c->P.ny, c->P.nz};
-    if (len[0] > FOLD_MAX || len[1] > FOLD_MAX) return true;
+    if (len[0] > FOLD_MAX || len[1] > FOLD_MAX) return setup_dct_dense<T>(c);
     for (int a = 0; a < 2; ++a)
         if (!(fft_len_ok(len[a]) ? setup_fft(c, a, len[a]) : setup_fold<T>(c, a, len[a]))) return false;
     if (plane_ok(len[0], len[1])) {
@@ -1181,9 +1196,7 @@ bool alloc_state(pllgpu_ctx* c)
     ok = ok && (B.phi = dalloc<real>(c, c->nelem)) && (B.div = dalloc<real>(c, c->nelem)) &&
          (B.S[VC] = dalloc<real>(c, c->nelem)) &&
          (B.dct1 = dalloc<real>(c, part_form<real>() ? c->nelem : ncell)) &&
-         (B.dct2 = dalloc<real>(c, part_form<real>() ? c->nelem : ncell)) &&
-         (B.Ty = dalloc<real>(c, (long)p->ny * p->ny)) && (B.Tz = dalloc<real>(c, (long)p->nz * p->nz)) &&
-         (B.Tiy = dalloc<real>(c, (long)p->ny * p->ny)) && (B.Tiz = dalloc<real>(c, (long)p->nz * p->nz));
+         (B.dct2 = dalloc<real>(c, part_form<real>() ? c->nelem : ncell));
     // right-hand sides: u's follows c's; v's and w's, where they stand beside
     // it, lie in the Poisson buffers, idle until the line solves are done
     B.S[VU] = B.S[VC];
@@ -1201,15 +1214,6 @@ bool alloc_state(pllgpu_ctx* c)
         ok = ok && (c->mode_rr = dalloc<double>(c, ncell)) != nullptr;
     }
     if (!ok) return false;
-    std::vector<real> T((size_t)std::max(p->ny, p->nz) * std::max(p->ny, p->nz));
-    dct_matrix<real>(0, p->ny, T.data());
-    cudaMemcpy(B.Ty, T.data(), sizeof(real) * p->ny * p->ny, cudaMemcpyHostToDevice);
-    dct_matrix<real>(0, p->nz, T.data());
-    cudaMemcpy(B.Tz, T.data(), sizeof(real) * p->nz * p->nz, cudaMemcpyHostToDevice);
-    dct_matrix<real>(1, p->ny, T.data());
-    cudaMemcpy(B.Tiy, T.data(), sizeof(real) * p->ny * p->ny, cudaMemcpyHostToDevice);
-    dct_matrix<real>(1, p->nz, T.data());
-    cudaMemcpy(B.Tiz, T.data(), sizeof(real) * p->nz * p->nz, cudaMemcpyHostToDevice);
     // kernels above the 48 KB default of dynamic shared memory
     cudaFuncSetAttribute(k_adi_z_tiled<VC, real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)adi_z_smem_bytes<VC, real>());
@@ -1228,20 +1232,22 @@ bool alloc_state(pllgpu_ctx* c)
             c->xt_on = true;
         }
         const bool shape_ok = (p->ny == 128 || p->ny == 256) && (p->nz == 128 || p->nz == 256);
-        if (!p->exact_dct && p->dct_kernel != 1 && !(shape_ok ? setup_umma(c) : setup_dct_lines<float>(c))) return false;
+        if (p->exact_dct || p->dct_kernel == 1) return setup_dct_dense<float>(c);
+        return shape_ok ? setup_dct_dense<float>(c) && setup_umma(c) : setup_dct_lines<float>(c);
     } else {
-#if !PLL_FP64_EXACT
-        if (!p->exact_dct && !setup_dct_lines<double>(c)) return false;
-        if (!p->exact_dct && c->nelem < (1L << 31) && encode_tiled()) {
+#if PLL_FP64_EXACT
+        return setup_dct_dense<double>(c);
+#else
+        if (c->nelem < (1L << 31) && encode_tiled()) {
             xt_setup<VC, double>(c);
             xt_setup<VU, double>(c);
             xt_setup<VV, double>(c);
             xt_setup<VW, double>(c);
             c->xt_on = true;
         }
+        return setup_dct_lines<double>(c);
 #endif
     }
-    return true;
 }
 
 }  // namespace
