@@ -105,7 +105,7 @@ struct pllgpu_ctx {
     bool rotated = false;       // fast steps ran: "new" roles are stale and
                                 // logically equal to "old" (see materialize)
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};
-    bool graphs_ready = false;
+    int stream_steps = 0;       // steps taken launch by launch
     double timestep = 0;
     int err = PLLGPU_OK;
     int launches_per_step = 0;

@@ -54,22 +54,32 @@ void enqueue_step_any(pllgpu_ctx* ctx) { FORM_CALL(ctx, form_enqueue_step, ctx);
 
 namespace {
 
-int build_graphs(pllgpu_ctx* ctx)
+// the graph of the step that starts from buffers `parity` (its three substeps
+// flip it)
+int build_graph(pllgpu_ctx* ctx, int parity)
 {
-    for (int t = 0; t < 2; ++t) {
-        const int c0 = ctx->cur;
-        cudaGraph_t g = nullptr;
-        CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
-        ctx->counting = 0;
-        enqueue_step_any(ctx);
-        CK(cudaStreamEndCapture(ctx->st, &g));
-        ctx->launches_per_step = ctx->counting;
-        CK(cudaGraphInstantiate(&ctx->gexec[c0], g, 0));
-        cudaGraphDestroy(g);
-        // cur flipped once by the three substeps
-    }
-    ctx->graphs_ready = true;
+    const int c0 = ctx->cur;
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamBeginCapture(ctx->st, cudaStreamCaptureModeThreadLocal));
+    ctx->cur = parity;
+    ctx->counting = 0;
+    enqueue_step_any(ctx);
+    ctx->cur = c0;
+    ctx->launches_per_step = ctx->counting;
+    CK(cudaStreamEndCapture(ctx->st, &g));
+    const cudaError_t e = cudaGraphInstantiate(&ctx->gexec[parity], g, 0);
+    cudaGraphDestroy(g);
+    CK(e);
     return PLLGPU_OK;
+}
+
+void drop_graphs(pllgpu_ctx* ctx)
+{
+    for (cudaGraphExec_t& g : ctx->gexec)
+        if (g) {
+            cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
 }
 
 // ---- field access -------------------------------------------------------------
@@ -293,8 +303,7 @@ void pllgpu_destroy(pllgpu_ctx* ctx)
     if (!ctx) return;
     cudaSetDevice(ctx->dev);
     if (ctx->st) cudaStreamSynchronize(ctx->st);
-    for (int t = 0; t < 2; ++t)
-        if (ctx->gexec[t]) cudaGraphExecDestroy(ctx->gexec[t]);
+    drop_graphs(ctx);
     for (cudaEvent_t e : ctx->ev_pool) cudaEventDestroy(e);
     for (void* p : ctx->allocs) cudaFree(p);
     if (ctx->ev_fork) cudaEventDestroy(ctx->ev_fork);
@@ -406,6 +415,17 @@ int pllgpu_resume(pllgpu_ctx* ctx, double tval)
     return read_status(ctx);
 }
 
+// When a run's two graphs (one per buffer parity) are built: 1 ms each whatever
+// the grid, to save 50 us of a 64x32x32 step.  A run that takes a step or two on
+// each new state paid for graphs that it never replayed (first step on a new
+// 64x32x32 solver: 2.1 ms with them, 0.28 launch by launch), so the first
+// STREAM_STEPS steps go out on the stream and each graph is built when its
+// parity comes next.  Past SHADOW_CELLS a step takes longer than it takes to
+// issue it and build both, which is done while the first one runs (256x128x128:
+// 5.0 ms with the graphs before it, 3.2 so).
+constexpr int STREAM_STEPS = 2;
+constexpr long SHADOW_CELLS = 1L << 21;
+
 int pllgpu_steps(pllgpu_ctx* ctx, int nsteps)
 {
     if (!ctx || nsteps < 0) return PLLGPU_EINVAL;
@@ -418,21 +438,23 @@ int pllgpu_steps(pllgpu_ctx* ctx, int nsteps)
         ctx->rotated = true;
         --nsteps;
     }
-    if (ctx->P.use_graph) {
-        if (!ctx->graphs_ready) {
-            if (int e = build_graphs(ctx)) return e;
-        }
-        for (int s = 0; s < nsteps; ++s) {
+    const bool shadow = (long)ctx->G.nx * ctx->G.ny * ctx->G.nz > SHADOW_CELLS;
+    for (int s = 0; s < nsteps; ++s) {
+        if (ctx->P.use_graph && !ctx->gexec[ctx->cur] && ctx->stream_steps >= STREAM_STEPS)
+            if (int e = build_graph(ctx, ctx->cur)) return e;
+        if (ctx->gexec[ctx->cur]) {
             CK(cudaGraphLaunch(ctx->gexec[ctx->cur], ctx->st));
             ctx->cur ^= 1;
+            continue;
         }
-    } else {
-        for (int s = 0; s < nsteps; ++s) {
-            ctx->counting = 0;
-            enqueue_step_any(ctx);
-            ctx->launches_per_step = ctx->counting;
-            if (int e = check_launch(ctx)) return e;
-        }
+        ctx->counting = 0;
+        enqueue_step_any(ctx);
+        ctx->launches_per_step = ctx->counting;
+        if (int e = check_launch(ctx)) return e;
+        ++ctx->stream_steps;
+        for (int t = 0; t < 2 && ctx->P.use_graph && shadow; ++t)
+            if (!ctx->gexec[t])
+                if (int e = build_graph(ctx, t)) return e;
     }
     if (nsteps > 0) ctx->rotated = true;
     CK(cudaStreamSynchronize(ctx->st));
@@ -480,12 +502,7 @@ int pllgpu_autotune(pllgpu_ctx* ctx, int trial_steps, int* steps_done)
     ctx->tune_exp = best_e;
     ctx->tune_line = best_l;
     // graphs captured with the old shapes are rebuilt on the next steps call
-    for (int t = 0; t < 2; ++t)
-        if (ctx->gexec[t]) {
-            cudaGraphExecDestroy(ctx->gexec[t]);
-            ctx->gexec[t] = nullptr;
-        }
-    ctx->graphs_ready = false;
+    drop_graphs(ctx);
     ctx->rotated = true;
     if (steps_done) *steps_done = done;
     CK(cudaStreamSynchronize(ctx->st));
@@ -507,12 +524,7 @@ int pllgpu_set_tuning(pllgpu_ctx* ctx, int explicit_variant, int line_variant)
         return PLLGPU_EINVAL;
     ctx->tune_exp = explicit_variant;
     ctx->tune_line = line_variant;
-    for (int t = 0; t < 2; ++t)
-        if (ctx->gexec[t]) {
-            cudaGraphExecDestroy(ctx->gexec[t]);
-            ctx->gexec[t] = nullptr;
-        }
-    ctx->graphs_ready = false;
+    drop_graphs(ctx);
     return PLLGPU_OK;
 }
 
