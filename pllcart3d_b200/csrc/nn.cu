@@ -764,6 +764,16 @@ long wgrad_chunks(int taps, int Cin, int Cout)
     return n < 1 ? 1 : n;
 }
 
+// volumes too small for the tcgen05 kernel, whose time hardly depends on the
+// volume until the CTAs are full (it sets up and empties one accumulator per
+// CTA: 13 us for 16 channels, 17 to 24 from 32 on, 11 for a 1x1x1 kernel), where
+// the warp-level kernel takes 7 us and 1 more per 15 voxels: it takes 8 voxels
+// in 7 us (13 to 24), 64 in 11 (13 to 24), 128 in 15 to 17
+bool wgrad_few(long V, int Cin, int ksize)
+{
+    return V < (ksize != 3 ? 64 : Cin < 32 ? 96 : 160);
+}
+
 template <int GA, int GN>
 bool wg_launch(const CuGeom& g, const WgPlan& p, dim3 grid, const CUtensorMap& mx, const CUtensorMap& mg, float* dW,
                cudaStream_t st)
@@ -877,10 +887,11 @@ int pllnn_conv_wgrad(const void* G, const void* X, int N, int D, int H, int W, i
                      float* dW, void* stream)
 {
     if (Cin % 8 || Cout % 8 || (ksize != 1 && ksize != 3)) return 6;
-    if (g_conv_path != 1 && wgrad_umma(G, X, N, D, H, W, Cin, Cout, ksize, dW, (cudaStream_t)stream))
-        return cudaGetLastError() == cudaSuccess ? 0 : 2;
     const Vol g{N, D, H, W};
     const long V = (long)N * D * H * W;
+    if ((g_conv_path == 2 || (g_conv_path == 0 && !wgrad_few(V, Cin, ksize))) &&
+        wgrad_umma(G, X, N, D, H, W, Cin, Cout, ksize, dW, (cudaStream_t)stream))
+        return cudaGetLastError() == cudaSuccess ? 0 : 2;
     const int ntaps = ksize * ksize * ksize;
     const int tiles = ((Cout + 63) / 64) * ((Cin + 63) / 64);
     const long chunks = wgrad_chunks(ntaps, Cin, Cout);
