@@ -985,8 +985,9 @@ int pllnn_cat_bwd(const float* dY, int CA, int CB, long V, float* dA, int accA, 
 
 int pllnn_mse(const float* P, const float* T, long n, float scale, float* grad, float* loss, void* stream)
 {
+    if (n <= 0) return 2;   // no launch of no blocks
     const unsigned blocks = nblk(n, 1024);   // about four terms a thread
-    if (n > 0) k_mse<<<blocks, 256, 0, (cudaStream_t)stream>>>(P, T, n, scale, grad, loss);
+    k_mse<<<blocks, 256, 0, (cudaStream_t)stream>>>(P, T, n, scale, grad, loss);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
