@@ -251,10 +251,12 @@ int pllgpu_find_max(pllgpu_ctx *ctx, const char *dir, double *maxval,
 int pllgpu_shift_conc(pllgpu_ctx *ctx, double ampli, double lamb, int subharm);
 
 /* ---- launch-shape autotuner ----------------------------------------------
- * Times every launch-shape variant of the explicit operators (4) and the x/y
- * line solves (3) on `trial_steps` steps each (plus one warm-up step) and
- * keeps the fastest.  All variants compute bit-identical results, so the
- * trial steps are steps of the run; *steps_done reports how many. */
+ * Times every launch-shape variant of the explicit operators without staging
+ * (4) and of the sequential x/y sweeps (3) on `trial_steps` steps each (plus
+ * one warm-up step) and keeps the fastest.  All variants compute bit-identical
+ * results, so the trial steps are steps of the run; *steps_done reports how
+ * many.  A context that launches neither kernel (by default, with x and y
+ * lines of up to 512 rows) takes the steps and keeps its variants. */
 int pllgpu_autotune(pllgpu_ctx *ctx, int trial_steps, int *steps_done);
 int pllgpu_tuning(pllgpu_ctx *ctx, int *explicit_variant, int *line_variant);
 int pllgpu_set_tuning(pllgpu_ctx *ctx, int explicit_variant, int line_variant);

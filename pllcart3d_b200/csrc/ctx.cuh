@@ -102,6 +102,8 @@ struct pllgpu_ctx {
     bool resync_c = false;      // after a restart: copy c's buffers once (resume)
     int tune_exp = 0;           // launch-shape variants (autotuner): explicit-
     int tune_line = 1;          // operator block, x/y line-solve block
+    bool tunes_exp = false;     // ... and whether this context launches a kernel
+    bool tunes_line = false;    // that takes its shape from them
     bool rotated = false;       // fast steps ran: "new" roles are stale and
                                 // logically equal to "old" (see materialize)
     cudaGraphExec_t gexec[2] = {nullptr, nullptr};

@@ -1214,6 +1214,11 @@ bool alloc_state(pllgpu_ctx* c)
         ok = ok && (c->mode_rr = dalloc<double>(c, ncell)) != nullptr;
     }
     if (!ok) return false;
+    // launch shapes the autotuner has a choice of: the explicit operator
+    // without staging and the sequential x and y sweeps
+    const bool staged = (std::is_same<real, float>::value || !PLL_FP64_EXACT) && !p->exact_dct && encode_tiled();
+    c->tunes_exp = !staged || p->explicit_kernel == 1;
+    c->tunes_line = !part_form<real>() || p->exact_dct || p->nx > LINE_PART_MAX || p->ny > LINE_PART_MAX;
     // kernels above the 48 KB default of dynamic shared memory
     cudaFuncSetAttribute(k_adi_z_tiled<VC, real>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)adi_z_smem_bytes<VC, real>());

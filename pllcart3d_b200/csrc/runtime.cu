@@ -478,10 +478,14 @@ int pllgpu_autotune(pllgpu_ctx* ctx, int trial_steps, int* steps_done)
         enqueue_step_any(ctx);
         ++done;
     }
+    // A choice that no launch of this context takes its shape from (by default
+    // neither, up to 512 rows) stays as it is; the trials advance the run by
+    // the same number of steps.
+    const int e_old = ctx->tune_exp, l_old = ctx->tune_line;
     for (int ve = 0; ve < NTUNE_EXP; ++ve)
         for (int vl = 0; vl < NTUNE_LINE; ++vl) {
-            ctx->tune_exp = ve;
-            ctx->tune_line = vl;
+            if (ctx->tunes_exp) ctx->tune_exp = ve;
+            if (ctx->tunes_line) ctx->tune_line = vl;
             enqueue_step_any(ctx);   // warm-up of this variant
             CK(cudaEventRecord(e0, ctx->st));
             for (int s = 0; s < trial_steps; ++s) enqueue_step_any(ctx);
@@ -493,16 +497,16 @@ int pllgpu_autotune(pllgpu_ctx* ctx, int trial_steps, int* steps_done)
             done += trial_steps + 1;
             if (ms < best) {
                 best = ms;
-                best_e = ve;
-                best_l = vl;
+                best_e = ctx->tune_exp;
+                best_l = ctx->tune_line;
             }
         }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     ctx->tune_exp = best_e;
     ctx->tune_line = best_l;
-    // graphs captured with the old shapes are rebuilt on the next steps call
-    drop_graphs(ctx);
+    // graphs captured with other shapes are rebuilt
+    if (best_e != e_old || best_l != l_old) drop_graphs(ctx);
     ctx->rotated = true;
     if (steps_done) *steps_done = done;
     CK(cudaStreamSynchronize(ctx->st));

@@ -242,8 +242,9 @@ class Solver:
         self._routine("rotate")
 
     def autotune(self, trial_steps: int = 2) -> int:
-        """pllgpu_autotune: picks the fastest launch shapes on steps of this
-        run (bit-identical variants); returns the steps it advanced."""
+        """pllgpu_autotune: picks the fastest launch shapes (of the kernels that
+        have variants: explicit_kernel="direct", exact_dct, x or y lines beyond
+        512 rows) on steps of this run; returns the steps it advanced."""
         done = ctypes.c_int()
         self._check(self._L.pllgpu_autotune(self._h, int(trial_steps), ctypes.byref(done)), "autotune")
         return done.value
