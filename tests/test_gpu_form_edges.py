@@ -1,4 +1,5 @@
-"""One step of mixed64 against the FP64 form at the line lengths and on the planes where the solves and transforms change form."""
+"""One step of mixed64 against the FP64 form at the line lengths and on the planes
+where the solves and transforms change form."""
 
 import pytest
 
