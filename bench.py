@@ -215,7 +215,11 @@ def run_reference(args, ws, rank):
     wl = workload(args.workload)
     ranks = ref_ranks(wl.params.nx)
     budget = 150.0
-    r = ref_mpi(args.workload, ranks, 1, args.steps, budget)
+    try:
+        r = ref_mpi(args.workload, ranks, 1, args.steps, budget)
+    except RuntimeError as e:   # not built on this machine
+        print(json.dumps({"impl": "reference", "unavailable": str(e)}), flush=True)
+        return
     value = r["cell_steps_per_s"]
     sample = (f"{r['steps']} of {args.steps} requested step(s) of {wl.name} after 1 untimed step (a {budget:.0f} s "
               f"budget caps the timed steps): pllcart3d.c on {ranks} x-slab ranks over a shared-memory MPI "
