@@ -295,7 +295,8 @@ def tensor_peak():
 # DRAM traffic over algorithmic bytes of a launch, from the ncu captures of
 # the 256x128x128 case (profiles/); traffic grows with the cells processed,
 # so a full launch's traffic is this ratio times its algorithmic bytes
-TRAFFIC_RATIO = {("k_explicit2", "fp32"): 1.05, ("k_explicit", "fp64"): 1.04, ("k_explicit_tma", "fp64"): 1.04}
+TRAFFIC_RATIO = {("k_explicit2", "fp32"): 1.05, ("k_explicit", "fp64"): 1.04, ("k_explicit_tma", "fp64"): 1.11,
+                 ("k_explicit_tma", "fp32"): 1.05}
 
 
 def l2_note(prm, form):

@@ -66,7 +66,8 @@ typedef struct pllgpu_params {
                               every line / mode solve the sequential Thomas
                               sweep; 0: FFT, folded or tcgen05 DCT passes and
                               partitioned line and mode solves                */
-    int use_graph;         /* 1: replay each step as one CUDA graph            */
+    int use_graph;         /* 1: replay each step as one CUDA graph (the first two
+                              go out launch by launch)                         */
     int dct_kernel;        /* precision form, exact_dct 0: 0 = tcgen05 split-TF32
                               GEMMs (persistent, one CTA per SM) where ny, nz
                               are 128 or 256, else the FP64 forms' line passes

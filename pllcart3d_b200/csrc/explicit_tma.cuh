@@ -6,8 +6,9 @@
 // A block owns a tile of TJ rows (j) x XT_TK cells (k) and walks ni planes
 // along x (chosen per launch, launch_explicit_tma).  An FP64 thread computes one
 // cell of a plane (TJ = 8); an FP32 thread two, rows j and j + 8 (TJ = 16), in
-// sm_100's paired instructions (one for two FP32 operations).  Every plane's tiles arrive by cp.async.bulk.tensor (one
-// thread issues them; an mbarrier per ring slot counts the bytes): q with a
+// sm_100's paired instructions (one for two FP32 operations).  Every plane's
+// tiles arrive by cp.async.bulk.tensor (one thread issues them; an mbarrier per
+// ring slot counts the bytes): q with a
 // +-3 halo in j and k (the WENO5 stencils along y and z), and, with a +-1
 // halo, each field the variable reads at a j or k offset (velocities,
 // viscosity edges, c).  A ring of XT_NS plane slots keeps planes i-1, i, i+1
@@ -357,8 +358,8 @@ __device__ __forceinline__ void k_explicit_tma_run(const uint3 blockIdx, const d
     __syncthreads();
 
     // register windows along x at (j, k).  A pair's second cell, XT_WJ rows on,
-    // may lie past the last row: it reads the rows beyond (inside the padded
-    // box or the slack past the array) and stores nothing
+    // may lie past the last row: it then reads the first one's column (and in
+    // the shared tiles its own row, zero-filled past the box) and stores nothing
     const long col = (long)j * sy + k, r2 = XT_WJ * sy;
     const bool live2 = XtLane<real>::NC == 2 && j + XT_WJ <= R.je;
     const real* __restrict__ q = A.q;

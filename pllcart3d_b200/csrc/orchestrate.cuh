@@ -1,8 +1,8 @@
 // Orchestration of the step (pllcart3d.c:156-196), templated on the storage
 // type: stage launchers, the substep/step sequences, start-up and the
-// per-routine entry points.  form_f64.cu (compiled without multiply-add
-// contraction) and form_f32.cu (with) each instantiate one precision form
-// and export it through the functions declared in forms.h.
+// per-routine entry points.  form_f64.cu and form_f64m.cu (compiled with
+// multiply-add contraction), form_f64x.cu and form_f32.cu (without) each
+// instantiate one form and export it through the functions declared in forms.h.
 #pragma once
 
 #include <algorithm>
